@@ -204,12 +204,14 @@ typedef struct {
  * FP32 (hi, lo) pairs of linv_arena, g_cols and w_hat (spi_split_f64),
  * read by the precision-1 cell kernel only. */
 typedef struct {
-    double *l_arena;     /* Cholesky factor L; for routed systems the
-                            inverse of the reference's saddle matrix */
-    double *linv_arena;  /* Linv = L^-1; NULL when no OK variance is wanted:
-                            spi_krige_factor then forms no inverse and
-                            estimates cond from triangular solves, and
-                            spi_krige_duals solves with L */
+    double *l_arena;     /* Cholesky factor L (without linv_arena: Linv in
+                            its lower triangle, the rest scratch); for
+                            routed systems the inverse of the reference's
+                            saddle matrix */
+    double *linv_arena;  /* Linv = L^-1, zeros above the diagonal; NULL when
+                            no OK variance is wanted: spi_krige_factor then
+                            inverts L in place and estimates cond from
+                            products with fixed vectors */
     int32_t *status;     /* Cholesky: 0, or the 1-based failing pivot */
     int32_t *route;      /* 0 Cholesky path, 1 exact-inverse path,
                             2 singular (nearest-station fallback) */
@@ -248,7 +250,8 @@ typedef struct {
     float *l32;          /* optional arena of the same layout as l_arena
                             (floats): with it, and without linv_arena,
                             spi_krige_factor factors every system in FP32
-                            first; systems whose FP32 factor succeeds with
+                            first (left holding the factor's inverse);
+                            systems whose FP32 factor succeeds with
                             cond <= cond_ir keep it, and spi_krige_duals
                             solves with it by FP64 iterative refinement
                             (residuals b - A x in FP64 with the full

@@ -14,6 +14,7 @@
 // staged in shared memory, and every operand read from L2 at most once per
 // 32-wide block of FMAs.
 #include "spi_common.cuh"
+#include "spi_factor.cuh"
 #include "spi_gj.cuh"
 #include "spi_saddle.cuh"
 
@@ -26,26 +27,6 @@ int launch_gj_multi(const spi_domain_t& dom, const spi_systems_t& sys, const spi
 // Resolves routes 3 / 4 left by k_gj (spi_pinv.cu).
 int launch_pinv(const spi_domain_t& dom, const spi_systems_t& sys, const spi_krige_ws_t& ws,
                 cudaStream_t st);
-
-constexpr int NB = 32;        // panel width of the blocked factorisations
-constexpr int FT = 256;       // threads per factor CTA
-constexpr int GA = SPI_MAX_DRIFT + 1;
-
-struct SysView {
-  int64_t off;
-  int n;
-  const int32_t* idx;
-  int64_t moff;
-};
-
-__device__ __forceinline__ SysView sys_view(const spi_systems_t& sys, int s) {
-  SysView v;
-  v.off = sys.stn_off[s];
-  v.n = (int)(sys.stn_off[s + 1] - v.off);
-  v.idx = sys.stn_idx + v.off;
-  v.moff = sys.mat_off[s];
-  return v;
-}
 
 // Sum of one value per thread over the block (all threads call it).
 __device__ double block_sum(double t, double* red) {
@@ -112,216 +93,6 @@ __global__ void k_build_sys(spi_domain_t dom, spi_systems_t sys, double* __restr
   }
 }
 
-// Right-looking blocked Cholesky, in place on the lower triangle, in T
-// (FP64; FP32 for the refinement path's factor). gate (optional): only
-// systems with gate[s] == want are factored.
-template <typename T>
-__global__ __launch_bounds__(FT) void k_chol(spi_systems_t sys, T* __restrict__ l_arena,
-                                            int32_t* __restrict__ status,
-                                            const int32_t* __restrict__ gate, int want) {
-  const int s = blockIdx.x;
-  if (gate && gate[s] != want) return;
-  SysView v = sys_view(sys, s);
-  const int n = v.n;
-  T* A = l_arena + v.moff;
-  __shared__ T D[NB][NB + 1];
-  __shared__ T Pi[64][NB + 1];
-  __shared__ T Pj[64][NB + 1];
-  __shared__ int fail;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) fail = 0;
-  __syncthreads();
-  for (int k0 = 0; k0 < n; k0 += NB) {
-    const int nb = min(NB, n - k0);
-    for (int e = tid; e < NB * NB; e += FT) {
-      int r = e / NB, c = e % NB;
-      D[r][c] = (r < nb && c <= r) ? A[(int64_t)(k0 + r) * n + k0 + c] : 0.0;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      for (int j = 0; j < nb; ++j) {
-        T djj = D[j][j];
-        if (!(djj > 0.0)) {  // not positive, or NaN
-          if (lane == 0) fail = k0 + j + 1;
-          break;
-        }
-        T ljj = sqrt(djj);
-        __syncwarp();
-        if (lane == j) D[j][j] = ljj;
-        if (lane > j && lane < nb) D[lane][j] = D[lane][j] / ljj;
-        __syncwarp();
-        if (lane > j && lane < nb) {
-          T lij = D[lane][j];
-          for (int c = j + 1; c <= lane; ++c) D[lane][c] -= lij * D[c][j];
-        }
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    if (fail) break;
-    for (int e = tid; e < nb * nb; e += FT) {
-      int r = e / nb, c = e % nb;
-      if (c <= r) A[(int64_t)(k0 + r) * n + k0 + c] = D[r][c];
-    }
-    // panel: rows below the diagonal block, A21 <- A21 L11^-T
-    for (int r = k0 + nb + tid; r < n; r += FT) {
-      T x[NB];
-      T* row = A + (int64_t)r * n + k0;
-#pragma unroll
-      for (int j = 0; j < NB; ++j) x[j] = (j < nb) ? row[j] : 0.0;
-#pragma unroll
-      for (int j = 0; j < NB; ++j) {
-        if (j < nb) {
-          T t = x[j];
-#pragma unroll
-          for (int c = 0; c < NB; ++c)
-            if (c < j) t -= x[c] * D[j][c];
-          x[j] = t / D[j][j];
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < NB; ++j)
-        if (j < nb) row[j] = x[j];
-    }
-    __syncthreads();
-    // trailing update of the lower triangle: A22 -= L21 L21'
-    const int r0 = k0 + nb;
-    const int m = n - r0;
-    if (m <= 0) continue;
-    const int nt = (m + 63) / 64;
-    for (int ti = 0; ti < nt; ++ti) {
-      for (int tj = 0; tj <= ti; ++tj) {
-        for (int e = tid; e < 64 * NB; e += FT) {
-          int r = e / NB, c = e % NB;
-          int gi = r0 + ti * 64 + r, gj = r0 + tj * 64 + r;
-          Pi[r][c] = (gi < n && c < nb) ? A[(int64_t)gi * n + k0 + c] : 0.0;
-          Pj[r][c] = (gj < n && c < nb) ? A[(int64_t)gj * n + k0 + c] : 0.0;
-        }
-        __syncthreads();
-        const int rr = (tid / 16) * 4, cc = (tid % 16) * 4;
-        T acc[4][4] = {};
-#pragma unroll 4
-        for (int c = 0; c < NB; ++c) {
-          T a[4], b[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            a[q] = Pi[rr + q][c];
-            b[q] = Pj[cc + q][c];
-          }
-#pragma unroll
-          for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[p][q] += a[p] * b[q];
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          int gi = r0 + ti * 64 + rr + p;
-          if (gi >= n) continue;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            int gj = r0 + tj * 64 + cc + q;
-            if (gj <= gi) A[(int64_t)gi * n + gj] -= acc[p][q];
-          }
-        }
-        __syncthreads();
-      }
-    }
-  }
-  __syncthreads();
-  if (tid == 0) status[s] = fail;
-}
-
-// Linv = L^-1 by block rows: X_II = inv(L_II), X_IJ = -X_II sum_K L_IK X_KJ.
-__global__ __launch_bounds__(FT) void k_trinv(spi_systems_t sys, const double* __restrict__ l_arena,
-                                             double* __restrict__ x_arena,
-                                             const int32_t* __restrict__ status,
-                                             double* __restrict__ cond) {
-  const int s = blockIdx.x;
-  SysView v = sys_view(sys, s);
-  const int n = v.n;
-  const double* L = l_arena + v.moff;
-  double* X = x_arena + v.moff;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (status[s] != 0) {
-    if (tid == 0) cond[s] = __longlong_as_double(0x7ff0000000000000LL);
-    return;
-  }
-  __shared__ double Ld[NB][NB + 1];
-  __shared__ double Xd[NB][NB + 1];
-  __shared__ double T[3][NB][NB + 1];
-  __shared__ double red[FT / 32];
-  double frob = 0.0;
-  const int nblk = (n + NB - 1) / NB;
-  for (int I = 0; I < nblk; ++I) {
-    const int i0 = I * NB, nb = min(NB, n - i0);
-    for (int e = tid; e < NB * NB; e += FT) {
-      int r = e / NB, c = e % NB;
-      Ld[r][c] = (r < nb && c <= r) ? L[(int64_t)(i0 + r) * n + i0 + c] : 0.0;
-    }
-    __syncthreads();
-    if (warp == 0 && lane < nb) {
-      const int j = lane;
-      for (int i = 0; i < nb; ++i) {
-        double val = 0.0;
-        if (i >= j) {
-          double t = (i == j) ? 1.0 : 0.0;
-          for (int c = j; c < i; ++c) t -= Ld[i][c] * Xd[c][j];
-          val = t / Ld[i][i];
-        }
-        Xd[i][j] = val;
-      }
-    }
-    __syncthreads();
-    for (int e = tid; e < nb * nb; e += FT) {
-      int r = e / nb, c = e % nb;
-      double xv = (c <= r) ? Xd[r][c] : 0.0;
-      X[(int64_t)(i0 + r) * n + i0 + c] = xv;
-      frob += xv * xv;
-    }
-    // off-diagonal blocks, 3 column blocks at a time
-    for (int J0 = 0; J0 < I; J0 += 3) {
-      const int nj = min(3, I - J0);
-      for (int e = tid; e < nj * NB * NB; e += FT) {
-        int jj = e / (NB * NB), rem = e % (NB * NB), r = rem / NB, c = rem % NB;
-        double t = 0.0;
-        if (r < nb) {
-          const int J = J0 + jj;
-          const double* lrow = L + (int64_t)(i0 + r) * n;
-          for (int k = J * NB; k < i0; ++k) t += lrow[k] * X[(int64_t)k * n + J * NB + c];
-        }
-        T[jj][r][c] = t;
-      }
-      __syncthreads();
-      for (int e = tid; e < nj * NB * NB; e += FT) {
-        int jj = e / (NB * NB), rem = e % (NB * NB), r = rem / NB, c = rem % NB;
-        if (r < nb) {
-          double t = 0.0;
-          for (int q = 0; q <= r; ++q) t += Xd[r][q] * T[jj][q][c];
-          double xv = -t;
-          X[(int64_t)(i0 + r) * n + (J0 + jj) * NB + c] = xv;
-          frob += xv * xv;
-        }
-      }
-      __syncthreads();
-    }
-    // zero the upper part of this block row (kept clean for contractions)
-    for (int e = tid; e < nb * (n - i0 - nb); e += FT) {
-      int r = e / (n - i0 - nb), c = e % (n - i0 - nb);
-      X[(int64_t)(i0 + r) * n + i0 + nb + c] = 0.0;
-    }
-    __syncthreads();
-  }
-  for (int o = 16; o > 0; o >>= 1) frob += __shfl_xor_sync(0xffffffffu, frob, o);
-  if (lane == 0) red[warp] = frob;
-  __syncthreads();
-  if (tid == 0) {
-    double f = 0.0;
-    for (int w = 0; w < FT / 32; ++w) f += red[w];
-    double a00 = L[0] * L[0];
-    cond[s] = (double)n * a00 * f;
-  }
-}
-
 // Exact-inverse path. Systems whose Cholesky failed, or whose condition
 // estimate exceeds cond_max, get the reference's own saddle matrix
 // [[Gamma, F], [F', 0]] (interp/steps.py:170-243; SK: the covariance
@@ -381,290 +152,6 @@ __global__ __launch_bounds__(FT) void k_gj(spi_domain_t dom, spi_systems_t sys,
       route[s] = fail ? 4 : 3;
     else
       route[s] = fail ? 2 : 1;
-  }
-}
-
-// y = X x (X lower, row-major n x n): warp per row, lanes along the row.
-__device__ void matvec_lower(const double* __restrict__ X, int n, const double* __restrict__ x,
-                             double* __restrict__ y) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int i = warp; i < n; i += nw) {
-    const double* row = X + (int64_t)i * n;
-    double t = 0.0;
-    for (int j = lane; j <= i; j += 32) t += row[j] * x[j];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) y[i] = t;
-  }
-}
-
-// y = X' q: thread per column, coalesced along rows.
-__device__ void matvec_lower_t(const double* __restrict__ X, int n, const double* __restrict__ q,
-                               double* __restrict__ y) {
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    double t = 0.0;
-    for (int i = j; i < n; ++i) t += X[(int64_t)i * n + j] * q[i];
-    y[j] = t;
-  }
-}
-
-__device__ double block_dot(const double* __restrict__ a, const double* __restrict__ b, int n,
-                            double* red) {
-  double t = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) t += a[i] * b[i];
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) red[warp] = t;
-  __syncthreads();
-  double r = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r += red[w];
-  __syncthreads();
-  return r;
-}
-
-// y = P[:, :n] x for the m x m row-major P (warp per row).
-__device__ void matvec_rows(const double* __restrict__ P, int m, int n,
-                            const double* __restrict__ x, double* __restrict__ y) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int i = warp; i < m; i += nw) {
-    const double* row = P + (int64_t)i * m;
-    double t = 0.0;
-    for (int j = lane; j < n; j += 32) t += row[j] * x[j];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) y[i] = t;
-  }
-}
-
-// S^-1 of the small a x a Schur complement by Gauss-Jordan with partial
-// pivoting (one thread), into Si and out [GA * GA], zero-padded.
-__device__ void schur_inverse(const double (*S)[GA], int a, double (*Si)[GA],
-                              double* __restrict__ out) {
-  double M[GA][2 * GA];
-  for (int i = 0; i < a; ++i)
-    for (int j = 0; j < 2 * a; ++j) M[i][j] = (j < a) ? S[i][j] : (j - a == i ? 1.0 : 0.0);
-  for (int c = 0; c < a; ++c) {
-    int p = c;
-    for (int r = c + 1; r < a; ++r)
-      if (fabs(M[r][c]) > fabs(M[p][c])) p = r;
-    if (p != c)
-      for (int j = 0; j < 2 * a; ++j) {
-        double t = M[c][j];
-        M[c][j] = M[p][j];
-        M[p][j] = t;
-      }
-    double piv = M[c][c];
-    for (int j = 0; j < 2 * a; ++j) M[c][j] /= piv;
-    for (int r = 0; r < a; ++r)
-      if (r != c) {
-        double f = M[r][c];
-        for (int j = 0; j < 2 * a; ++j) M[r][j] -= f * M[c][j];
-      }
-  }
-  for (int i = 0; i < GA; ++i)
-    for (int j = 0; j < GA; ++j) {
-      double val = (i < a && j < a) ? M[i][a + j] : 0.0;
-      Si[i][j] = val;
-      out[i * GA + j] = val;
-    }
-}
-
-// ---- triangular solves with the Cholesky factor (no inverse formed) ----
-// Systems that need no OK variance never form Linv (n^3/3 FP64 per
-// system); their dual vectors come from L by forward and backward
-// substitution, nk <= KS right-hand sides at once, held in shared memory
-// as Y[k * ldy + i]. L: row-major n x n, lower triangle (the upper one
-// still holds the matrix and is never read).
-constexpr int KS = 4;
-
-// Y_k <- L^-1 Y_k. Blocks of 32 rows: the rows' dot products with the
-// solved part (a warp per row, lanes along the row), then the 32 x 32
-// diagonal block by one warp (a lane per row).
-template <typename TL>
-__device__ void trsv_lower_multi(const TL* __restrict__ L, int n, double* Y, int ldy,
-                                 int nk) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i0 = 0; i0 < n; i0 += 32) {
-    const int nb = min(32, n - i0);
-    if (i0 > 0) {
-      for (int r = warp; r < nb; r += FT / 32) {
-        const TL* row = L + (int64_t)(i0 + r) * n;
-        double acc[KS];
-#pragma unroll
-        for (int k = 0; k < KS; ++k) acc[k] = 0.0;
-        for (int j = lane; j < i0; j += 32) {
-          const double l = row[j];
-#pragma unroll
-          for (int k = 0; k < KS; ++k)
-            if (k < nk) acc[k] = fma(l, Y[k * ldy + j], acc[k]);
-        }
-#pragma unroll
-        for (int k = 0; k < KS; ++k)
-          for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-        if (lane == 0)
-          for (int k = 0; k < nk; ++k) Y[k * ldy + i0 + r] -= acc[k];
-      }
-      __syncthreads();
-    }
-    if (warp == 0) {
-      double t[KS];
-      const TL* Lb = L + (int64_t)(i0 + min(lane, nb - 1)) * n + i0;  // this lane's row
-      // one reciprocal per row (divisions run on the 1/64-rate FP64 pipe)
-      const double rd = 1.0 / (double)Lb[min(lane, nb - 1)];
-#pragma unroll
-      for (int k = 0; k < KS; ++k) t[k] = (lane < nb && k < nk) ? Y[k * ldy + i0 + lane] : 0.0;
-      for (int c = 0; c < nb; ++c) {
-        const double rcc = __shfl_sync(0xffffffffu, rd, c);
-        const double lrc = (lane > c && lane < nb) ? (double)Lb[c] : 0.0;
-#pragma unroll
-        for (int k = 0; k < KS; ++k) {
-          const double y = __shfl_sync(0xffffffffu, t[k], c) * rcc;
-          if (lane == c) t[k] = y;
-          else t[k] -= lrc * y;
-        }
-      }
-      if (lane < nb)
-        for (int k = 0; k < nk; ++k) Y[k * ldy + i0 + lane] = t[k];
-    }
-    __syncthreads();
-  }
-}
-
-// Y_k <- L^-T Y_k. Blocks of 32 rows from the bottom: the diagonal block
-// by one warp, then every earlier entry updated by the block's solved
-// values (a thread per entry, reading the block's rows of L along them).
-template <typename TL>
-__device__ void trsv_lower_t_multi(const TL* __restrict__ L, int n, double* Y, int ldy,
-                                   int nk) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nblk = (n + 31) / 32;
-  for (int I = nblk - 1; I >= 0; --I) {
-    const int i0 = I * 32, nb = min(32, n - i0);
-    if (warp == 0) {
-      double t[KS];
-      const double rd =
-          1.0 / (double)L[(int64_t)(i0 + min(lane, nb - 1)) * n + i0 + min(lane, nb - 1)];
-#pragma unroll
-      for (int k = 0; k < KS; ++k) t[k] = (lane < nb && k < nk) ? Y[k * ldy + i0 + lane] : 0.0;
-      for (int c = nb - 1; c >= 0; --c) {
-        const TL* Lc = L + (int64_t)(i0 + c) * n + i0;  // row c of the block
-        const double rcc = __shfl_sync(0xffffffffu, rd, c);
-        const double lcr = (lane < c) ? (double)Lc[lane] : 0.0;
-#pragma unroll
-        for (int k = 0; k < KS; ++k) {
-          const double y = __shfl_sync(0xffffffffu, t[k], c) * rcc;
-          if (lane == c) t[k] = y;
-          else t[k] -= lcr * y;
-        }
-      }
-      if (lane < nb)
-        for (int k = 0; k < nk; ++k) Y[k * ldy + i0 + lane] = t[k];
-    }
-    __syncthreads();
-    for (int r = tid; r < i0; r += FT) {
-      double acc[KS];
-#pragma unroll
-      for (int k = 0; k < KS; ++k) acc[k] = 0.0;
-      for (int c = 0; c < nb; ++c) {
-        const double l = L[(int64_t)(i0 + c) * n + r];
-#pragma unroll
-        for (int k = 0; k < KS; ++k)
-          if (k < nk) acc[k] = fma(l, Y[k * ldy + i0 + c], acc[k]);
-      }
-      for (int k = 0; k < nk; ++k) Y[k * ldy + r] -= acc[k];
-    }
-    __syncthreads();
-  }
-}
-
-// A^-1 applied to the kk vectors Y[k * n + i]: two triangular solves with
-// the system's FP64 factor, or, where the system kept its FP32 factor
-// (ws.ir[s] == 1), FP64 iterative refinement over it: x = L32^-T L32^-1 b,
-// then, with the residual r = b - A x of the full FP64 matrix (kept in
-// l_arena), x += L32^-T L32^-1 r until the componentwise backward error
-// max_i |r_i| / (sum_j |A_ij| |x_j| + |b_i|) is under sqrt(n) eps (the
-// FP64 solve's own level), at most SPI_IR_MAX_ITERS corrections. bval(k, i):
-// entry i of right-hand side k (the Y held on entry); D: scratch of kk * n
-// doubles. ws.ir_iters[s] records the corrections (their maximum over the
-// calls); kIrFailed is or-ed in when they did not converge, and
-// spi_krige_duals then refactors the system in FP64 and solves again.
-constexpr int kIrFailed = 0x40000000;
-template <typename BF>
-__device__ void ainv_apply(const spi_krige_ws_t& ws, int s, int n, int64_t moff, double* Y,
-                           double* D, int kk, BF bval) {
-  if (!(ws.l32 && ws.ir && ws.ir[s] == 1)) {
-    const double* L = ws.l_arena + moff;
-    trsv_lower_multi(L, n, Y, n, kk);
-    trsv_lower_t_multi(L, n, Y, n, kk);
-    return;
-  }
-  const float* L = ws.l32 + moff;
-  const double* A = ws.l_arena + moff;
-  __shared__ double rmax[FT / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const double tol = sqrt((double)n) * 2.220446049250313e-16;
-  trsv_lower_multi(L, n, Y, n, kk);
-  trsv_lower_t_multi(L, n, Y, n, kk);
-  int it = 0;
-  bool conv = false;
-  double prev = __longlong_as_double(0x7ff0000000000000LL);
-  for (;; ++it) {
-    // D = b - A x and the componentwise backward error, a warp per row
-    double be = 0.0;
-    __syncthreads();
-    for (int i = warp; i < n; i += FT / 32) {
-      const double* row = A + (int64_t)i * n;
-      double t[KS], ta[KS];
-#pragma unroll
-      for (int k = 0; k < KS; ++k) t[k] = ta[k] = 0.0;
-      for (int j = lane; j < n; j += 32) {
-        const double a = row[j];
-#pragma unroll
-        for (int k = 0; k < KS; ++k)
-          if (k < kk) {
-            const double x = Y[k * n + j];
-            t[k] = fma(a, x, t[k]);
-            ta[k] = fma(fabs(a), fabs(x), ta[k]);
-          }
-      }
-#pragma unroll
-      for (int k = 0; k < KS; ++k)
-        for (int o = 16; o > 0; o >>= 1) {
-          t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
-          ta[k] += __shfl_xor_sync(0xffffffffu, ta[k], o);
-        }
-      if (lane == 0)
-        for (int k = 0; k < kk; ++k) {
-          const double b = bval(k, i), r = b - t[k];
-          D[k * n + i] = r;
-          const double den = ta[k] + fabs(b);
-          if (den > 0.0) be = fmax(be, fabs(r) / den);
-          else if (r != 0.0) be = __longlong_as_double(0x7ff0000000000000LL);
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) be = fmax(be, __shfl_xor_sync(0xffffffffu, be, o));
-    __syncthreads();
-    if (lane == 0) rmax[warp] = be;
-    __syncthreads();
-    be = 0.0;
-    for (int w = 0; w < FT / 32; ++w) be = fmax(be, rmax[w]);
-    if (be <= tol) {
-      conv = true;
-      break;
-    }
-    // a factor too far from A (cond x the FP32 rounding near 1 or above)
-    // makes no progress: stop once a correction fails to halve the
-    // backward error (a converging refinement shrinks it by orders of
-    // magnitude per step)
-    if (it == SPI_IR_MAX_ITERS || !(be < 0.5 * prev)) break;
-    prev = be;
-    trsv_lower_multi(L, n, D, n, kk);
-    trsv_lower_t_multi(L, n, D, n, kk);
-    for (int e = threadIdx.x; e < kk * n; e += FT) Y[e] += D[e];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && ws.ir_iters) {
-    atomicMax(ws.ir_iters + s, it);
-    if (!conv) atomicOr(ws.ir_iters + s, kIrFailed);
   }
 }
 
@@ -730,14 +217,6 @@ __global__ void k_to_f32(spi_systems_t sys, const double* __restrict__ l_arena,
     l32[v.moff + e] = (float)l_arena[v.moff + e];
 }
 
-// Systems whose refinement did not converge fall back to the FP64 factor
-// (ir = 2): spi_krige_duals then factors and solves them again.
-__global__ void k_ir_fail_gate(spi_systems_t sys, spi_krige_ws_t ws) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= sys.n_sys) return;
-  if (ws.ir[s] == 1 && (ws.ir_iters[s] & kIrFailed)) ws.ir[s] = 2;
-}
-
 // Which systems keep the FP32 factor: it succeeded with cond <= cond_ir;
 // the others' status is reset for the FP64 factorisation.
 __global__ void k_ir_gate(spi_systems_t sys, spi_krige_ws_t ws, double cond_ir) {
@@ -747,340 +226,6 @@ __global__ void k_ir_gate(spi_systems_t sys, spi_krige_ws_t ws, double cond_ir) 
   ws.ir[s] = keep;
   ws.ir_iters[s] = 0;
   if (!keep) ws.status[s] = 0;
-}
-
-// A deterministic Rademacher sign for entry i of probe k of system s.
-__device__ __forceinline__ double probe_sign(int s, int k, int i) {
-  uint32_t h = (uint32_t)i * 0x9E3779B1u ^ ((uint32_t)k * 0x85EBCA77u + (uint32_t)s * 0xC2B2AE3Du);
-  h ^= h >> 16;
-  h *= 0x7FEB352Du;
-  h ^= h >> 15;
-  h *= 0x846CA68Bu;
-  h ^= h >> 16;
-  return (h & 1u) ? 1.0 : -1.0;
-}
-
-// cond = n A_00 ||Linv||_F^2 without Linv: ||Linv||_F^2 = trace(A^-1) =
-// E |L^-1 g|^2 over Rademacher g (Hutchinson), the mean of KP fixed
-// probes (relative spread ~ sqrt(2 / KP) at worst, far inside the orders
-// of magnitude the routing thresholds work in). Dynamic shared memory:
-// nk x n doubles.
-constexpr int KP = 8;
-template <typename TL>
-__global__ __launch_bounds__(FT) void k_cond_est(spi_systems_t sys,
-                                                const TL* __restrict__ l_arena,
-                                                const int32_t* __restrict__ status,
-                                                double* __restrict__ cond, int nk,
-                                                const int32_t* __restrict__ gate, int want) {
-  const int s = blockIdx.x;
-  if (gate && gate[s] != want) return;
-  SysView v = sys_view(sys, s);
-  const int n = v.n;
-  if (status[s] != 0) {
-    if (threadIdx.x == 0) cond[s] = __longlong_as_double(0x7ff0000000000000LL);
-    return;
-  }
-  const TL* L = l_arena + v.moff;
-  extern __shared__ double ysm[];
-  __shared__ double red[FT / 32];
-  double tot = 0.0;
-  for (int k0 = 0; k0 < KP; k0 += nk) {
-    const int kk = min(nk, KP - k0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < kk * n; e += FT) {
-      const int k = e / n, i = e - k * n;
-      ysm[k * n + i] = probe_sign(s, k0 + k, i);
-    }
-    __syncthreads();
-    trsv_lower_multi(L, n, ysm, n, kk);
-    for (int e = threadIdx.x; e < kk * n; e += FT) tot = fma(ysm[e], ysm[e], tot);
-  }
-  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = tot;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < FT / 32; ++w) t += red[w];
-    const double l0 = (double)L[0];
-    cond[s] = (double)n * (l0 * l0) * (t / KP);
-  }
-}
-
-// Route-0 duals without Linv (spi_krige_duals when ws.linv_arena is NULL):
-// the same quantities as k_duals, A^-1 applied by two triangular solves.
-// This kernel: G, S^-1, 1'G per system; k_duals_solve_steps: the steps.
-// Dynamic shared memory: nk x n doubles.
-__global__ __launch_bounds__(FT) void k_duals_solve(spi_domain_t dom, spi_systems_t sys,
-                                                   spi_krige_ws_t ws,
-                                                   const double* __restrict__ vals, int nk,
-                                                   int only_fallback) {
-  const int s = blockIdx.x;
-  if (ws.route[s] != 0) return;
-  if (only_fallback && ws.ir[s] != 2) return;
-  SysView v = sys_view(sys, s);
-  const int n = v.n;
-  extern __shared__ double ysm[];
-  __shared__ double red[FT / 32];
-  __shared__ double S[GA][GA];
-  __shared__ double Si[GA][GA];
-  const int sk = sys.kind == SPI_KIND_SK;
-  const int a = sk ? 1 : extra_rows(sys.kind, dom.n_drift);
-  double* G = ws.g_cols + v.off * GA;  // column k at G + k * n
-  auto fcol = [&](int k, int i) {
-    return (k == 0) ? 1.0 : dom.stn_drift[(int64_t)v.idx[i] * dom.n_drift + (k - 1)];
-  };
-  // G_k = A^-1 F_k
-  for (int k0 = 0; k0 < a; k0 += nk) {
-    const int kk = min(nk, a - k0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < kk * n; e += FT) {
-      const int k = e / n, i = e - k * n;
-      ysm[k * n + i] = fcol(k0 + k, i);
-    }
-    __syncthreads();
-    ainv_apply(ws, s, n, v.moff, ysm, ysm + nk * n, kk,
-               [&](int k, int i) { return fcol(k0 + k, i); });
-    for (int e = threadIdx.x; e < kk * n; e += FT) G[(int64_t)k0 * n + e] = ysm[e];
-  }
-  __syncthreads();
-  // SK: |u| (u = A^-1 1) as a second column (as k_duals)
-  if (sk)
-    for (int i = threadIdx.x; i < n; i += FT) G[n + i] = fabs(G[i]);
-  // S = F'G, its inverse, 1'G
-  for (int k = 0; k < a; ++k)
-    for (int l = 0; l < a; ++l) {
-      double t = 0.0;
-      for (int i = threadIdx.x; i < n; i += FT) t = fma(fcol(k, i), G[(int64_t)l * n + i], t);
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      __syncthreads();
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double u = 0.0;
-        for (int w = 0; w < FT / 32; ++w) u += red[w];
-        S[k][l] = u;
-      }
-    }
-  __syncthreads();
-  if (threadIdx.x == 0) schur_inverse(S, a, Si, ws.s_inv + (int64_t)s * GA * GA);
-  for (int k = 0; k < GA; ++k) {
-    double t = 0.0;
-    if (k < a)
-      for (int i = threadIdx.x; i < n; i += FT) t += G[(int64_t)k * n + i];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double u = 0.0;
-      for (int w = 0; w < FT / 32; ++w) u += red[w];
-      ws.g_colsum[(int64_t)s * GA + k] = (k < a) ? u : 0.0;
-    }
-  }
-}
-
-// The per-step part of the route-0 duals without Linv: CTA (g, s) takes
-// steps g * nk .. of system s (w_hat = A^-1 z - G beta with beta =
-// S^-1 G'z; SK: w_hat = A^-1 z), reading G and S^-1 from k_duals_solve.
-// Dynamic shared memory: nk x n doubles.
-__global__ __launch_bounds__(FT) void k_duals_solve_steps(spi_domain_t dom, spi_systems_t sys,
-                                                         spi_krige_ws_t ws,
-                                                         const double* __restrict__ vals,
-                                                         int nk, int only_fallback) {
-  const int s = blockIdx.y;
-  if (ws.route[s] != 0) return;
-  if (only_fallback && ws.ir[s] != 2) return;
-  const int64_t sb = sys.step_off[s], se = sys.step_off[s + 1];
-  if (sb + (int64_t)blockIdx.x * nk >= se) return;
-  SysView v = sys_view(sys, s);
-  const int n = v.n;
-  extern __shared__ double ysm[];
-  __shared__ double red[FT / 32];
-  __shared__ double Si[GA][GA];
-  __shared__ double hb[KS][GA];
-  const int sk = sys.kind == SPI_KIND_SK;
-  const int a = sk ? 1 : extra_rows(sys.kind, dom.n_drift);
-  const double* G = ws.g_cols + v.off * GA;
-  for (int e = threadIdx.x; e < GA * GA; e += FT)
-    Si[e / GA][e % GA] = ws.s_inv[(int64_t)s * GA * GA + e];
-  for (int64_t q0 = sb + (int64_t)blockIdx.x * nk; q0 < se; q0 += (int64_t)gridDim.x * nk) {
-    const int kk = (int)min((int64_t)nk, se - q0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < kk * n; e += FT) {
-      const int k = e / n, i = e - k * n;
-      ysm[k * n + i] = vals[sys.val_off[sys.steps[q0 + k]] + i];
-    }
-    __syncthreads();
-    if (!sk) {
-      // h = G'z per vector, before the solves overwrite z
-      for (int k = 0; k < kk; ++k)
-        for (int l = 0; l < a; ++l) {
-          double t = 0.0;
-          for (int i = threadIdx.x; i < n; i += FT) t = fma(G[(int64_t)l * n + i], ysm[k * n + i], t);
-          for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-          __syncthreads();
-          if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
-          __syncthreads();
-          if (threadIdx.x == 0) {
-            double u = 0.0;
-            for (int w = 0; w < FT / 32; ++w) u += red[w];
-            hb[k][l] = u;
-          }
-        }
-      __syncthreads();
-    }
-    ainv_apply(ws, s, n, v.moff, ysm, ysm + nk * n, kk, [&](int k, int i) {
-      return vals[sys.val_off[sys.steps[q0 + k]] + i];
-    });
-    for (int k = 0; k < kk; ++k) {
-      const int j = sys.steps[q0 + k];
-      const int64_t vo = sys.val_off[j];
-      double bt[GA];
-      for (int m = 0; m < GA; ++m) {
-        double t = 0.0;
-        if (!sk)
-          for (int l = 0; l < a; ++l) t += Si[m][l] * hb[k][l];
-        bt[m] = (m < a && !sk) ? t : 0.0;
-      }
-      for (int i = threadIdx.x; i < n; i += FT) {
-        double w = ysm[k * n + i];
-        if (!sk)
-          for (int m = 0; m < a; ++m) w -= G[(int64_t)m * n + i] * bt[m];
-        ws.w_hat[vo + i] = w;
-      }
-      if (threadIdx.x < GA) ws.beta[(int64_t)j * GA + threadIdx.x] = bt[threadIdx.x];
-    }
-  }
-}
-
-// Per-system G, S^-1, 1'G and per-step dual weights (route 0), or the
-// split dual vectors of the inverse saddle matrix (route 1). Dynamic shared
-// memory: 3 vectors of n + GA doubles.
-__global__ __launch_bounds__(FT) void k_duals(spi_domain_t dom, spi_systems_t sys,
-                                             spi_krige_ws_t ws,
-                                             const double* __restrict__ vals) {
-  const int s = blockIdx.x;
-  const int route = ws.route[s];
-  if (route == 2) return;
-  if (route == 0 && ws.linv_arena == nullptr) return;  // k_duals_solve
-  SysView v = sys_view(sys, s);
-  const int n = v.n;
-  const double* X = ws.linv_arena + v.moff;
-  extern __shared__ double sm[];
-  double* va = sm;
-  double* vb = sm + (n + GA);
-  double* vz = sm + 2 * (n + GA);
-  __shared__ double red[FT / 32];
-  __shared__ double S[GA][GA];
-  __shared__ double Si[GA][GA];
-  __shared__ double hb[GA];
-  const int sk = sys.kind == SPI_KIND_SK;
-  const int a = sk ? 1 : extra_rows(sys.kind, dom.n_drift);
-  double* G = ws.g_cols + v.off * GA;  // column k at G + k * n
-  if (route == 1) {
-    const int ar = sk ? 0 : a;
-    const int m = n + ar;
-    const double* P = ws.l_arena + v.moff;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) va[i] = 1.0;
-    __syncthreads();
-    matvec_rows(P, m, n, va, vb);
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) G[i] = vb[i];
-    // SK: |u| as a second column, as on the Cholesky path (the FP32 tier's
-    // bound of its sum check's rounding)
-    if (sk)
-      for (int i = threadIdx.x; i < n; i += blockDim.x) G[n + i] = fabs(vb[i]);
-    if (threadIdx.x < GA)
-      ws.g_colsum[(int64_t)s * GA + threadIdx.x] = (threadIdx.x < ar) ? vb[n + threadIdx.x] : 0.0;
-    for (int64_t si = sys.step_off[s]; si < sys.step_off[s + 1]; ++si) {
-      const int j = sys.steps[si];
-      const int64_t vo = sys.val_off[j];
-      __syncthreads();
-      for (int i = threadIdx.x; i < n; i += blockDim.x) vz[i] = vals[vo + i];
-      __syncthreads();
-      matvec_rows(P, m, n, vz, vb);
-      __syncthreads();
-      for (int i = threadIdx.x; i < n; i += blockDim.x) ws.w_hat[vo + i] = vb[i];
-      if (threadIdx.x < GA)
-        ws.beta[(int64_t)j * GA + threadIdx.x] = (threadIdx.x < ar) ? vb[n + threadIdx.x] : 0.0;
-    }
-    return;
-  }
-  // G_k = Linv' (Linv F_k)
-  for (int k = 0; k < a; ++k) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-      va[i] = (k == 0) ? 1.0 : dom.stn_drift[(int64_t)v.idx[i] * dom.n_drift + (k - 1)];
-    __syncthreads();
-    matvec_lower(X, n, va, vb);
-    __syncthreads();
-    matvec_lower_t(X, n, vb, G + (int64_t)k * n);
-    __syncthreads();
-  }
-  // SK: |u| (u = A^-1 1) as a second column. The FP32 cell kernels
-  // contract it to bound the rounding of sum(lambda) = u'c per cell
-  // (covariances are >= 0, so sum |u_i| c_i bounds sum |u_i c_i|).
-  if (sk) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) G[n + i] = fabs(G[i]);
-  }
-  // S = F'G
-  for (int k = 0; k < a; ++k) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-      va[i] = (k == 0) ? 1.0 : dom.stn_drift[(int64_t)v.idx[i] * dom.n_drift + (k - 1)];
-    __syncthreads();
-    for (int l = 0; l < a; ++l) {
-      double d = block_dot(va, G + (int64_t)l * n, n, red);
-      if (threadIdx.x == 0) S[k][l] = d;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) schur_inverse(S, a, Si, ws.s_inv + (int64_t)s * GA * GA);
-  __syncthreads();
-  for (int k = 0; k < GA; ++k) {
-    double cs = 0.0;
-    if (k < a) {
-      for (int i = threadIdx.x; i < n; i += blockDim.x) va[i] = 1.0;
-      __syncthreads();
-      cs = block_dot(va, G + (int64_t)k * n, n, red);
-    }
-    if (threadIdx.x == 0) ws.g_colsum[(int64_t)s * GA + k] = cs;
-  }
-  // per step
-  for (int64_t si = sys.step_off[s]; si < sys.step_off[s + 1]; ++si) {
-    const int j = sys.steps[si];
-    const int64_t vo = sys.val_off[j];
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) vz[i] = vals[vo + i];
-    __syncthreads();
-    if (!sk) {
-      for (int k = 0; k < a; ++k) {
-        double d = block_dot(G + (int64_t)k * n, vz, n, red);
-        if (threadIdx.x == 0) hb[k] = d;
-      }
-      __syncthreads();
-    }
-    matvec_lower(X, n, vz, va);
-    __syncthreads();
-    matvec_lower_t(X, n, va, vb);
-    __syncthreads();
-    if (!sk) {
-      double bt[GA];
-      for (int k = 0; k < GA; ++k) {
-        double t = 0.0;
-        for (int l = 0; l < a; ++l) t += Si[k][l] * hb[l];
-        bt[k] = (k < a) ? t : 0.0;
-      }
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double w = vb[i];
-        for (int k = 0; k < a; ++k) w -= G[(int64_t)k * n + i] * bt[k];
-        ws.w_hat[vo + i] = w;
-      }
-      if (threadIdx.x < GA) ws.beta[(int64_t)j * GA + threadIdx.x] = bt[threadIdx.x];
-    } else {
-      for (int i = threadIdx.x; i < n; i += blockDim.x) ws.w_hat[vo + i] = vb[i];
-      if (threadIdx.x < GA) ws.beta[(int64_t)j * GA + threadIdx.x] = 0.0;
-    }
-  }
 }
 
 // Leave-one-out cross-validation residuals of every station of every step
@@ -1146,21 +291,6 @@ static int check_ws(const spi_krige_ws_t* ws) {
   return SPI_OK;
 }
 
-// Right-hand sides per triangular-solve pass and the shared memory they
-// take (KS at most, within 200 KB).
-// Right-hand sides per pass of the triangular-solve kernels and their
-// dynamic shared memory: nk x n doubles, twice that with the refinement's
-// correction vectors (ir).
-static int solve_smem(int max_n, int* nk, size_t* bytes, int ir = 0) {
-  const size_t per = (size_t)max_n * sizeof(double) * (ir ? 2 : 1);
-  int k = (int)((200 * 1024) / per);
-  if (k > KS) k = KS;
-  if (k < 1) return SPI_ERR_TOO_LARGE;
-  *nk = k;
-  *bytes = (size_t)k * per;
-  return SPI_OK;
-}
-
 static bool ir_mode(const spi_krige_ws_t* ws) {
   return ws->l32 && !ws->linv_arena && ws->ir && ws->ir_iters;
 }
@@ -1182,33 +312,25 @@ extern "C" int spi_krige_factor(const spi_domain_t* dom, const spi_systems_t* sy
   const bool ir = ir_mode(ws);
   k_build_sys<<<dim3(gx, sys->n_sys), 256, 0, st>>>(d, sy, ws->l_arena, ws->shift, ir ? 1 : 0);
   SPI_LAUNCH_CHECK();
-  int nk = 0;
-  size_t ysm = 0;
-  if (!ws->linv_arena) {
-    if ((rc = solve_smem(sys->max_n, &nk, &ysm))) return rc;
-    if (!smem_opt_in(k_cond_est<double>, ysm) || !smem_opt_in(k_cond_est<float>, ysm))
-      return SPI_ERR_CUDA;
-  }
+  const Gate every{nullptr, 0}, not_kept{ws->ir, 0};
   if (ir) {
     // FP32 factor first; systems that keep it skip the FP64 one
     k_to_f32<<<dim3(gx, sys->n_sys), 256, 0, st>>>(sy, ws->l_arena, ws->l32);
-    k_chol<float><<<sys->n_sys, FT, 0, st>>>(sy, ws->l32, ws->status, nullptr, 0);
-    k_cond_est<float><<<sys->n_sys, FT, ysm, st>>>(sy, ws->l32, ws->status, ws->cond, nk,
-                                                    nullptr, 0);
+    if ((rc = launch_chol<float>(sy, ws->l32, ws->status, every, st))) return rc;
+    if ((rc = launch_trinv<float>(sy, ws->l32, ws->l32, ws->status, ws->cond, 1, every, st)))
+      return rc;
     k_ir_gate<<<(sys->n_sys + 255) / 256, 256, 0, st>>>(sy, *ws,
                                                        ws->cond_ir > 0 ? ws->cond_ir : 1e10);
     SPI_LAUNCH_CHECK();
   }
-  k_chol<double><<<sys->n_sys, FT, 0, st>>>(sy, ws->l_arena, ws->status, ir ? ws->ir : nullptr,
-                                            0);
-  SPI_LAUNCH_CHECK();
-  if (ws->linv_arena) {
-    k_trinv<<<sys->n_sys, FT, 0, st>>>(sy, ws->l_arena, ws->linv_arena, ws->status, ws->cond);
-  } else {
-    k_cond_est<double><<<sys->n_sys, FT, ysm, st>>>(sy, ws->l_arena, ws->status, ws->cond, nk,
-                                                     ir ? ws->ir : nullptr, 0);
-  }
-  SPI_LAUNCH_CHECK();
+  const Gate g = ir ? not_kept : every;
+  if ((rc = launch_chol<double>(sy, ws->l_arena, ws->status, g, st))) return rc;
+  // the inverse factor: an arena of its own where the OK variance reads it
+  // (zeros above the diagonal), else over the factor
+  double* x = ws->linv_arena ? ws->linv_arena : ws->l_arena;
+  if ((rc = launch_trinv<double>(sy, ws->l_arena, x, ws->status, ws->cond,
+                                 ws->linv_arena ? 0 : 1, g, st)))
+    return rc;
   size_t gsm = (size_t)(sys->max_n + GA) * (2 * sizeof(double) + sizeof(int));
   if (gsm > 200 * 1024) return SPI_ERR_TOO_LARGE;
   if (!smem_opt_in(k_gj, gsm)) return SPI_ERR_CUDA;
@@ -1241,46 +363,7 @@ extern "C" int spi_krige_duals(const spi_domain_t* dom, const spi_systems_t* sys
   if (sys->n_sys == 0) return SPI_OK;
   if ((rc = check_ws(ws))) return rc;
   if (!vals) return SPI_ERR_ARG;
-  size_t smem = (size_t)3 * (sys->max_n + GA) * sizeof(double);
-  if (smem > 200 * 1024) return SPI_ERR_TOO_LARGE;
-  if (!smem_opt_in(k_duals, smem)) return SPI_ERR_CUDA;
-  k_duals<<<sys->n_sys, FT, smem, (cudaStream_t)stream>>>(*dom, *sys, *ws, vals);
-  SPI_LAUNCH_CHECK();
-  if (!ws->linv_arena) {
-    // route-0 systems without Linv: triangular solves with L (or FP64
-    // refinement over the FP32 factor)
-    int nk;
-    size_t ysm;
-    if ((rc = solve_smem(sys->max_n, &nk, &ysm, ir_mode(ws) ? 1 : 0))) return rc;
-    if (!smem_opt_in(k_duals_solve, ysm) || !smem_opt_in(k_duals_solve_steps, ysm))
-      return SPI_ERR_CUDA;
-    cudaStream_t st = (cudaStream_t)stream;
-    // the steps: groups of nk spread over gx CTAs per system
-    int gx = (304 + sys->n_sys - 1) / sys->n_sys;
-    gx = gx < 1 ? 1 : (gx > 64 ? 64 : gx);
-    const int passes = ir_mode(ws) ? 2 : 1;
-    for (int pass = 0; pass < passes; ++pass) {
-      if (pass == 1) {
-        // systems whose refinement did not converge: FP64 factor, then
-        // their duals again
-        k_ir_fail_gate<<<(sys->n_sys + 255) / 256, 256, 0, st>>>(*sys, *ws);
-        k_chol<double><<<sys->n_sys, FT, 0, st>>>(*sys, ws->l_arena, ws->status, ws->ir, 2);
-        int nk1;
-        size_t ysm1;
-        if ((rc = solve_smem(sys->max_n, &nk1, &ysm1))) return rc;
-        if (!smem_opt_in(k_cond_est<double>, ysm1)) return SPI_ERR_CUDA;
-        k_cond_est<double><<<sys->n_sys, FT, ysm1, st>>>(*sys, ws->l_arena, ws->status,
-                                                         ws->cond, nk1, ws->ir, 2);
-        SPI_LAUNCH_CHECK();
-      }
-      k_duals_solve<<<sys->n_sys, FT, ysm, st>>>(*dom, *sys, *ws, vals, nk, pass);
-      SPI_LAUNCH_CHECK();
-      k_duals_solve_steps<<<dim3(gx, sys->n_sys), FT, ysm, st>>>(*dom, *sys, *ws, vals, nk,
-                                                                 pass);
-      SPI_LAUNCH_CHECK();
-    }
-  }
-  return SPI_OK;
+  return launch_duals(*dom, *sys, *ws, vals, (cudaStream_t)stream);
 }
 
 extern "C" int spi_krige_loo(const spi_domain_t* dom, const spi_systems_t* sys,

@@ -505,6 +505,18 @@ class _KrigeBatch:
         pend = self.n[route != 0]
         return 2 + (2 * int(pend.max() + self.a_rows) if pend.size else 0)
 
+    def factor_launches(self):
+        """Kernels of the Cholesky factors and their inverses beyond one each
+        (csrc/spi_chol.cu): two per panel of 32 rows after the first, two per
+        level of the inverse and its condition pass; three factors (FP32,
+        FP64, FP64 again) on the refinement path."""
+        n = int(self.n.max())
+        if n <= 32:
+            return 0
+        panels = (n + 31) // 32 - 1
+        levels = panels.bit_length()
+        return (2 * panels + 2 * levels + 1) * (3 if self.l32 is not None else 1)
+
     def passes(self):
         """The cell-kernel passes of run(): (precision, route filter)."""
         return [(1, 1), (0, 2)] if self.precision == 1 else [(0, 0)]
@@ -886,7 +898,7 @@ class InterpPlan:
                 # build, Cholesky, inverse or condition estimate, the
                 # exact-inverse elimination (one kernel, or set-up + 2 per
                 # row + finish), the pinv check
-                n += 3 + b.gj_launches() + (b.pinv is not None)
+                n += 3 + b.gj_launches() + (b.pinv is not None) + b.factor_launches()
                 n += 1 if kind == "EDK" else 0  # the drift-dependence check
                 # the FP32 factor of the refinement path: copy, Cholesky,
                 # condition estimate, gate
