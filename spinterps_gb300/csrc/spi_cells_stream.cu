@@ -115,6 +115,7 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
 
   __shared__ double red[SNW][SSV][STC];
   __shared__ double vres[SSV][STC];
+  __shared__ double qsh[GA][STC];  // dual columns (more than a pass holds: EDK, 4 drifts on)
   __shared__ int okf[STC], nnb[STC];
   __shared__ double cvar[STC];
   __shared__ const double* vp64[SSV];
@@ -340,15 +341,18 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
       s_nf[warp * STC + lane] = nf;  // red is free again
       nf_ready = true;
     }
-    if (v0 == 0) {
-      // the sum check of every cell, from the dual columns (all in pass 0)
+    for (int e = tid; e < nv * STC; e += STC * SNW)
+      if (v0 + e / STC < ndual) qsh[v0 + e / STC][e % STC] = vres[e / STC][e % STC];
+    __syncthreads();
+    if (v0 < ndual && v0 + nv >= ndual) {
+      // the sum check of every cell, once its dual columns are complete
       if (tid == 0) any_bad = any_chk = 0;
       __syncthreads();
       if (tid < STC) {
         const int cell = tid;
         const int64_t g = c0 + cell;
         double q[GA], f[GA], nu[GA];
-        for (int k = 0; k < GA; ++k) q[k] = k < ndual ? vres[k][cell] : 0.0;
+        for (int k = 0; k < GA; ++k) q[k] = k < ndual ? qsh[k][cell] : 0.0;
         f[0] = 1.0;
         for (int k = 1; k < GA; ++k)
           f[k] = (k < a && g < C && !sk) ? A.dom.cell_drift[(int64_t)(k - 1) * C + g] : 0.0;

@@ -65,3 +65,13 @@ def test_loo_of_uneven_systems():
     for t in range(4):
         one, r = steps.krige_loo(sx, sy, z[t:t + 1], vgs[:1])
         assert np.array_equal(res[t], one[0]) and rmse[t] == r[0], t
+
+
+@pytest.mark.parametrize("drifts", [4, 5, 7])
+def test_many_drifts_in_the_streamed_kernel(drifts):
+    """More dual columns than the streamed kernel contracts in a pass of its
+    four vectors: the sum check needs them all (with the columns of the
+    later passes missing, cells fell back to their nearest station, by what
+    shared memory held)."""
+    for seed in range(4):
+        _check(90, 3, ["EDK"], False, 400 + seed, drifts, "mixed", 1e-5)
