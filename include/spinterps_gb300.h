@@ -444,6 +444,35 @@ int spi_krige_var_tc_pack(const spi_domain_t *dom, const spi_systems_t *sys,
 int spi_krige_var_df(const spi_domain_t *dom, const spi_systems_t *sys,
                      const spi_krige_ws_t *ws, double cond_cap, spi_stream_t stream);
 
+/* The precision-0 pass of spi_krige_cells_tiled (route_filter 0 or 2) with
+ * the contractions (the OK variance, the dual columns, every step's
+ * estimates) on the tensor cores as exact products of 8-bit slices: operands
+ * of 55 bits, exact sums, FP64 results. Systems it covers: the Cholesky path
+ * (SK also on the exact-inverse path) with Exp, Gau, Sph, Lin and Nug
+ * structures; the others run as in spi_krige_cells_tiled. max_steps: the
+ * most steps of a system of the batch. scratch: device memory of
+ * spi_slices_scratch_bytes (want_var 0 for SK; systems beyond it go in
+ * groups). err_flag (device): set to 1 when a tensor-core wait ran out, whose
+ * cells are then incomplete. */
+int spi_krige_cells_sliced(const spi_domain_t *dom, const spi_systems_t *sys,
+                           const double *vals, const spi_krige_ws_t *ws, int32_t want_var,
+                           int32_t route_filter, double cond_split, const spi_out_t *out,
+                           int32_t tile, int32_t max_steps, void *scratch,
+                           int64_t scratch_bytes, int32_t *err_flag, spi_stream_t stream);
+
+/* spi_krige_var_df's systems by the same sliced contraction (FP64 accuracy),
+ * the double-float kernel for those it does not cover. Requires linv_arena
+ * besides what spi_krige_var_df requires; scratch of spi_slices_scratch_bytes
+ * with want_fields 0. */
+int spi_krige_var_sliced(const spi_domain_t *dom, const spi_systems_t *sys,
+                         const spi_krige_ws_t *ws, double cond_cap, void *scratch,
+                         int64_t scratch_bytes, int32_t *err_flag, spi_stream_t stream);
+
+/* Device scratch of spi_krige_cells_sliced (want_fields 1) or
+ * spi_krige_var_sliced (want_fields 0) on the current device. */
+int64_t spi_slices_scratch_bytes(int32_t max_n, int32_t n_sys, int32_t max_steps,
+                                 int32_t n_drift, int32_t want_var, int32_t want_fields);
+
 /* IDW (interp/steps.py:293-313, cyth/interpmthds.pyx:784-808) for every
  * cell of the listed steps. data [n_steps_total, n_stns] holds every
  * station's value, NaN where missing (the reference's data_df row). For

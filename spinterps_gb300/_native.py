@@ -118,6 +118,11 @@ _SIGS = {
     "spi_krige_cells_tiled": [ctypes.POINTER(DomainT), ctypes.POINTER(SystemsT), c_ptr,
                               ctypes.POINTER(KrigeWsT), c_i32, c_i32, c_i32, c_dbl,
                               ctypes.POINTER(OutT), c_i32, c_ptr],
+    "spi_krige_cells_sliced": [ctypes.POINTER(DomainT), ctypes.POINTER(SystemsT), c_ptr,
+                               ctypes.POINTER(KrigeWsT), c_i32, c_i32, c_dbl,
+                               ctypes.POINTER(OutT), c_i32, c_i32, c_ptr, c_i64, c_ptr, c_ptr],
+    "spi_krige_var_sliced": [ctypes.POINTER(DomainT), ctypes.POINTER(SystemsT),
+                             ctypes.POINTER(KrigeWsT), c_dbl, c_ptr, c_i64, c_ptr, c_ptr],
     "spi_krige_tier": [ctypes.POINTER(SystemsT), ctypes.POINTER(KrigeWsT), c_i64, c_ptr, c_ptr,
                        c_ptr, c_ptr, c_ptr, c_dbl, c_dbl, c_dbl, c_dbl, c_ptr, c_ptr, c_ptr,
                        c_ptr],
@@ -169,7 +174,7 @@ _SIGS = {
 
 # every entry point the header declares (checked by the CPU tests)
 EXPORTS = sorted(list(_SIGS) + ["spi_version", "spi_cuda_error", "spi_mlp_n_params",
-                                 "spi_local_groups_scratch_bytes"])
+                                 "spi_local_groups_scratch_bytes", "spi_slices_scratch_bytes"])
 
 _lib = None
 _lock = threading.Lock()
@@ -198,6 +203,8 @@ def load(path=LIB_PATH):
         lib.spi_mlp_n_params.argtypes = [c_i32, c_i32, c_i32, c_i32]
         lib.spi_local_groups_scratch_bytes.restype = c_i64
         lib.spi_local_groups_scratch_bytes.argtypes = [c_i32, c_i32, c_i32, c_i32, c_i32]
+        lib.spi_slices_scratch_bytes.restype = c_i64
+        lib.spi_slices_scratch_bytes.argtypes = [c_i32] * 6
         _lib = lib
         return lib
 

@@ -23,6 +23,7 @@
 #include "spi_contract.cuh"
 #include "spi_rhs.cuh"
 #include "spi_cells.cuh"
+#include "spi_slices.cuh"
 
 namespace spi {
 
@@ -39,20 +40,14 @@ __device__ __forceinline__ void contract(const T* cvT, T* Bs, const double* cons
 }
 
 template <typename T, int TC, typename OutT>
-__global__ __launch_bounds__(CT) void k_krige_cells(CellsArgs A, int npad) {
+__device__ __forceinline__ void cells_tile(const CellsArgs& A, int npad, int64_t tile) {
   using WL = Layout<TC, true>;
   using NL = Layout<TC, false>;
   constexpr int CPT = WL::CPT;
   const int s = blockIdx.y;
   const int64_t C = A.dom.n_cells;
-  const int64_t c0 = (int64_t)blockIdx.x * TC;
-  if (c0 >= C) return;
+  const int64_t c0 = tile * TC;
   const int route = A.ws.route[s];
-  {
-    // filter 1: well-conditioned Cholesky systems; filter 2: all others
-    const bool fast = fp32_tier(A.ws, s, A.cond_split, A.sys.kind == SPI_KIND_SK);
-    if ((A.route_filter == 1 && !fast) || (A.route_filter == 2 && fast)) return;
-  }
   const bool prim = route == 1;   // exact-inverse path: primal formulas
   const bool failed = route == 2;
   const int64_t soff = A.sys.stn_off[s];
@@ -474,6 +469,22 @@ __global__ __launch_bounds__(CT) void k_krige_cells(CellsArgs A, int npad) {
   }
 }
 
+// A CTA walks over tiles of one system: a pass launched over every system of
+// a batch costs little for those that another kernel computes.
+template <typename T, int TC, typename OutT>
+__global__ __launch_bounds__(CT) void k_krige_cells(CellsArgs A, int npad) {
+  const int s = blockIdx.y;
+  if (A.skip && A.skip[(int64_t)s * A.skip_stride]) return;
+  // filter 1: well-conditioned Cholesky systems; filter 2: all others
+  const bool fast = fp32_tier(A.ws, s, A.cond_split, A.sys.kind == SPI_KIND_SK);
+  if ((A.route_filter == 1 && !fast) || (A.route_filter == 2 && fast)) return;
+  const int64_t tiles = (A.dom.n_cells + TC - 1) / TC;
+  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    cells_tile<T, TC, OutT>(A, npad, t);
+    __syncthreads();
+  }
+}
+
 template <typename T, int TC>
 static size_t cells_smem(int npad) {
   return (size_t)npad * TC * sizeof(T) + (size_t)KC * BSTR * 8 +
@@ -482,7 +493,7 @@ static size_t cells_smem(int npad) {
 }
 
 template <typename T, int TC, typename OutT>
-static int launch_cells(const CellsArgs& A, cudaStream_t st) {
+static int launch_tile(const CellsArgs& A, cudaStream_t st) {
   int npad = (A.sys.max_n + GA + KC - 1) / KC * KC;
   size_t smem = cells_smem<T, TC>(npad);
   auto kern = k_krige_cells<T, TC, OutT>;
@@ -491,7 +502,10 @@ static int launch_cells(const CellsArgs& A, cudaStream_t st) {
     return SPI_ERR_CUDA;
   int64_t tiles = (A.dom.n_cells + TC - 1) / TC;
   if (tiles > 0x7fffffff) return SPI_ERR_TOO_LARGE;
-  dim3 grid((unsigned)tiles, (unsigned)A.sys.n_sys);
+  // up to 16 CTAs per SM over all systems, and each its own tile below that
+  int64_t gx = (152 * 16 + A.sys.n_sys - 1) / A.sys.n_sys;
+  if (gx < 16) gx = 16;
+  dim3 grid((unsigned)(tiles < gx ? tiles : gx), (unsigned)A.sys.n_sys);
   kern<<<grid, CT, smem, st>>>(A, npad);
   SPI_LAUNCH_CHECK();
   return SPI_OK;
@@ -523,17 +537,25 @@ static int dispatch_cells(const CellsArgs& A, int tile, cudaStream_t st) {
   if (tile) {
     const int npad = (A.sys.max_n + GA + KC - 1) / KC * KC;
     const size_t cap = 227 * 1024;
-    if (tile == 64 && cells_smem<T, 64>(npad) <= cap) return launch_cells<T, 64, OutT>(A, st);
-    if (tile == 32 && cells_smem<T, 32>(npad) <= cap) return launch_cells<T, 32, OutT>(A, st);
-    if (tile == 16 && cells_smem<T, 16>(npad) <= cap) return launch_cells<T, 16, OutT>(A, st);
+    if (tile == 64 && cells_smem<T, 64>(npad) <= cap) return launch_tile<T, 64, OutT>(A, st);
+    if (tile == 32 && cells_smem<T, 32>(npad) <= cap) return launch_tile<T, 32, OutT>(A, st);
+    if (tile == 16 && cells_smem<T, 16>(npad) <= cap) return launch_tile<T, 16, OutT>(A, st);
     return SPI_ERR_TOO_LARGE;
   }
   int tc = pick_tc<T>(A.sys.max_n);
-  if (tc == 64) return launch_cells<T, 64, OutT>(A, st);
-  if (tc == 32) return launch_cells<T, 32, OutT>(A, st);
-  if (tc == 16) return launch_cells<T, 16, OutT>(A, st);
+  if (tc == 64) return launch_tile<T, 64, OutT>(A, st);
+  if (tc == 32) return launch_tile<T, 32, OutT>(A, st);
+  if (tc == 16) return launch_tile<T, 16, OutT>(A, st);
   if (A.want_var && A.sys.kind != SPI_KIND_SK) return SPI_ERR_TOO_LARGE;
   return launch_cells_stream(A, sizeof(T) == 8 ? 0 : 1, st);
+}
+
+int launch_cells(const CellsArgs& A, int precision, int tile, cudaStream_t st) {
+  if (precision == 0)
+    return A.out.out_f64 ? dispatch_cells<double, double>(A, tile, st)
+                         : dispatch_cells<double, float>(A, tile, st);
+  return A.out.out_f64 ? dispatch_cells<float, double>(A, tile, st)
+                       : dispatch_cells<float, float>(A, tile, st);
 }
 
 __global__ void k_split_f64(const double* __restrict__ x, float* __restrict__ hi,
@@ -597,12 +619,55 @@ extern "C" int spi_krige_cells_tiled(const spi_domain_t* dom, const spi_systems_
   A.route_filter = route_filter;
   A.cond_split = cond_split;
   A.out = *out;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (precision == 0)
-    return out->out_f64 ? dispatch_cells<double, double>(A, tile, st)
-                        : dispatch_cells<double, float>(A, tile, st);
-  return out->out_f64 ? dispatch_cells<float, double>(A, tile, st)
-                      : dispatch_cells<float, float>(A, tile, st);
+  A.skip = nullptr;
+  A.skip_stride = 0;
+  return launch_cells(A, precision, tile, (cudaStream_t)stream);
+}
+
+// The FP64 pass (precision 0) with the sliced tensor-core contraction for
+// the systems that have one, the FP64 kernels for the others.
+extern "C" int spi_krige_cells_sliced(const spi_domain_t* dom, const spi_systems_t* sys,
+                                      const double* vals, const spi_krige_ws_t* ws,
+                                      int32_t want_var, int32_t route_filter, double cond_split,
+                                      const spi_out_t* out, int32_t tile, int32_t max_steps,
+                                      void* scratch, int64_t scratch_bytes, int32_t* err_flag,
+                                      spi_stream_t stream) {
+  if (!dom || !sys || !out || !ws || !scratch || !err_flag || max_steps < 0) return SPI_ERR_ARG;
+  if (tile != 0 && tile != 16 && tile != 32 && tile != 64) return SPI_ERR_ARG;
+  if (sys->n_sys < 0 || sys->n_sys > 65535) return SPI_ERR_TOO_LARGE;
+  if (dom->n_drift < 0 || dom->n_drift > SPI_MAX_DRIFT) return SPI_ERR_TOO_LARGE;
+  if (route_filter != 0 && route_filter != 2) return SPI_ERR_ARG;
+  if (sys->n_sys == 0 || dom->n_cells == 0) return SPI_OK;
+  if (!vals || !out->est || !ws->route || !ws->shift || !ws->beta || !ws->s_inv ||
+      !ws->g_colsum || !ws->l_arena || !ws->cond || !ws->w_hat || !ws->g_cols)
+    return SPI_ERR_ARG;
+  if (want_var && !ws->linv_arena) return SPI_ERR_ARG;
+  SlicesCall c;
+  c.dom = *dom;
+  c.sys = *sys;
+  c.ws = *ws;
+  c.vals = vals;
+  c.out = *out;
+  c.cond_split = cond_split;
+  c.want_var = want_var && sys->kind != SPI_KIND_SK;
+  c.want_vec = 1;
+  c.filter = route_filter;
+  c.max_vec = 1 + dom->n_drift + max_steps;
+  c.scratch = scratch;
+  c.scratch_bytes = scratch_bytes;
+  c.err = err_flag;
+  CellsArgs A;
+  A.dom = *dom;
+  A.sys = *sys;
+  A.ws = *ws;
+  A.vals = vals;
+  A.want_var = want_var ? 1 : 0;
+  A.route_filter = route_filter;
+  A.cond_split = cond_split;
+  A.out = *out;
+  const int rc = launch_slices(c, &A.skip, &A.skip_stride, (cudaStream_t)stream);
+  if (rc) return rc;
+  return launch_cells(A, 0, tile, (cudaStream_t)stream);
 }
 
 extern "C" int spi_krige_cells(const spi_domain_t* dom, const spi_systems_t* sys,

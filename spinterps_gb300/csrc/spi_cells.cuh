@@ -15,6 +15,9 @@ struct CellsArgs {
   int route_filter;
   double cond_split;
   spi_out_t out;
+  // systems already computed (spi_slices.cu): skip[s * skip_stride] != 0
+  const int32_t* skip;
+  int skip_stride;
 };
 
 // Exact (FP64, reference-ordered) nearest station of a cell among a
@@ -61,6 +64,9 @@ __device__ __forceinline__ bool fp32_tier(const spi_krige_ws_t& ws, int s, doubl
   if (ws.tier) return ws.tier[s] != 0;
   return fp32_route(ws.route[s], sk) && ws.cond[s] <= cond_split;
 }
+
+// The cell kernels' dispatch by shape (spi_cells.cu).
+int launch_cells(const CellsArgs& A, int precision, int tile, cudaStream_t st);
 
 // Host-side dispatch of the streamed kernel (spi_cells_stream.cu): systems
 // too large for the shared-memory right-hand side of k_krige_cells.

@@ -84,7 +84,7 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
   const int s = blockIdx.y;
   const int64_t C = A.dom.n_cells;
   const int64_t c0 = (int64_t)blockIdx.x * STC;
-  if (c0 >= C) return;
+  if (c0 >= C || (A.skip && A.skip[(int64_t)s * A.skip_stride])) return;
   const int route = A.ws.route[s];
   {
     const bool fast = fp32_tier(A.ws, s, A.cond_split, A.sys.kind == SPI_KIND_SK);

@@ -1,0 +1,36 @@
+// The sliced tensor-core contraction (spi_slices.cu) as the cell entry points
+// call it.
+#pragma once
+#include "spi_common.cuh"
+
+namespace spi {
+
+struct Yes {
+  static constexpr bool value = true;
+};
+struct No {
+  static constexpr bool value = false;
+};
+
+struct SlicesCall {
+  spi_domain_t dom;
+  spi_systems_t sys;
+  spi_krige_ws_t ws;
+  const double* vals;   // (fields)
+  spi_out_t out;        // (fields)
+  double cond_split;
+  int want_var, want_vec;
+  int filter;           // 0: every system, 2: not in an FP32 tier, 3: the double-float tier
+  int max_vec;          // dual columns plus the most steps of a system
+  void* scratch;
+  int64_t scratch_bytes;
+  int32_t* err;
+};
+
+int64_t slices_scratch(int max_n, int n_sys, int max_vec, bool var, bool vec);
+
+// Runs the systems that have a sliced form; (*use)[s * *stride] != 0 (on the
+// device, in stream order) marks them, the caller computes the others.
+int launch_slices(const SlicesCall& c, const int32_t** use, int* stride, cudaStream_t st);
+
+}  // namespace spi

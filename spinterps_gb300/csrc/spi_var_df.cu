@@ -17,6 +17,7 @@
 // cells' double-float sums; the 16 row groups are summed at the end.
 #include "spi_cells.cuh"
 #include "spi_rhs.cuh"
+#include "spi_slices.cuh"
 
 namespace spi {
 
@@ -30,6 +31,9 @@ struct VarDfArgs {
   spi_systems_t sys;
   spi_krige_ws_t ws;
   double cond_cap;
+  // systems already computed (spi_slices.cu): skip[s * skip_stride] != 0
+  const int32_t* skip;
+  int skip_stride;
 };
 
 __device__ __forceinline__ bool var_df_system(const spi_krige_ws_t& ws, int s, double cap) {
@@ -51,10 +55,9 @@ __device__ __forceinline__ void df_fma_acc(df& acc, float ah, float al, float bh
 __global__ __launch_bounds__(VD_T) void k_var_df(VarDfArgs A) {
   const int s = blockIdx.y;
   const int64_t C = A.dom.n_cells;
-  const int64_t c0 = (int64_t)blockIdx.x * VD_C;
-  if (c0 >= C) return;
   if (A.sys.kind == SPI_KIND_SK) return;
   if (!var_df_system(A.ws, s, A.cond_cap)) return;
+  if (A.skip && A.skip[(int64_t)s * A.skip_stride]) return;
   const int64_t soff = A.sys.stn_off[s];
   const int n = (int)(A.sys.stn_off[s + 1] - soff);
   const int32_t* idx = A.sys.stn_idx + soff;
@@ -71,6 +74,10 @@ __global__ __launch_bounds__(VD_T) void k_var_df(VarDfArgs A) {
   __shared__ double part[VD_T / (VD_C / 2)][VD_C];
   __shared__ RhsDf kd;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // (a CTA walks over tiles: a launch over every system of a batch costs
+  // little for those that do not take part)
+  for (int64_t c0 = (int64_t)blockIdx.x * VD_C; c0 < C; c0 += (int64_t)gridDim.x * VD_C) {
+  __syncthreads();
   if (tid == 0) kd.init(A.sys.vg[s], sh, A.dom.min_vg_val);
   // staging role: this lane's cell for the right-hand sides
   const int64_t gc = c0 + lane;
@@ -153,6 +160,27 @@ __global__ __launch_bounds__(VD_T) void k_var_df(VarDfArgs A) {
     for (int g = 0; g < VD_T / (VD_C / 2); ++g) t += part[g][tid];
     A.ws.cell_yy[(int64_t)s * C + c0 + tid] = t;
   }
+  }
+}
+
+static int launch_var_df(const VarDfArgs& A, cudaStream_t st) {
+  const int64_t tiles = (A.dom.n_cells + VD_C - 1) / VD_C;
+  int64_t gx = (152 * 64 + A.sys.n_sys - 1) / A.sys.n_sys;
+  if (gx < 32) gx = 32;
+  dim3 grid((unsigned)(tiles < gx ? tiles : gx), (unsigned)A.sys.n_sys);
+  k_var_df<<<grid, VD_T, 0, st>>>(A);
+  SPI_LAUNCH_CHECK();
+  return SPI_OK;
+}
+
+static int check_var_df(const spi_domain_t* dom, const spi_systems_t* sys,
+                        const spi_krige_ws_t* ws) {
+  if (!ws->cell_yy || !ws->linv_hi || !ws->linv_lo || !ws->route || !ws->cond || !ws->shift ||
+      !dom->cell_split || !dom->stn_split || !sys->vg || !sys->stn_off || !sys->stn_idx ||
+      !sys->mat_off)
+    return SPI_ERR_ARG;
+  if ((dom->n_cells + VD_C - 1) / VD_C > 0x7fffffff) return SPI_ERR_TOO_LARGE;
+  return SPI_OK;
 }
 
 }  // namespace spi
@@ -164,15 +192,32 @@ extern "C" int spi_krige_var_df(const spi_domain_t* dom, const spi_systems_t* sy
   if (!dom || !sys || !ws) return SPI_ERR_ARG;
   if (sys->n_sys < 0 || sys->n_sys > 65535) return SPI_ERR_TOO_LARGE;
   if (sys->n_sys == 0 || dom->n_cells == 0) return SPI_OK;
-  if (!ws->cell_yy || !ws->linv_hi || !ws->linv_lo || !ws->route || !ws->cond || !ws->shift ||
-      !dom->cell_split || !dom->stn_split || !sys->vg || !sys->stn_off || !sys->stn_idx ||
-      !sys->mat_off)
-    return SPI_ERR_ARG;
-  const int64_t tiles = (dom->n_cells + VD_C - 1) / VD_C;
-  if (tiles > 0x7fffffff) return SPI_ERR_TOO_LARGE;
-  VarDfArgs A{*dom, *sys, *ws, cond_cap};
-  dim3 grid((unsigned)tiles, (unsigned)sys->n_sys);
-  k_var_df<<<grid, VD_T, 0, (cudaStream_t)stream>>>(A);
-  SPI_LAUNCH_CHECK();
-  return SPI_OK;
+  if (int rc = check_var_df(dom, sys, ws)) return rc;
+  return launch_var_df(VarDfArgs{*dom, *sys, *ws, cond_cap, nullptr, 0}, (cudaStream_t)stream);
+}
+
+// The same systems' |Linv c|^2 by the sliced tensor-core contraction, the
+// double-float kernel for those without a sliced form.
+extern "C" int spi_krige_var_sliced(const spi_domain_t* dom, const spi_systems_t* sys,
+                                    const spi_krige_ws_t* ws, double cond_cap, void* scratch,
+                                    int64_t scratch_bytes, int32_t* err_flag,
+                                    spi_stream_t stream) {
+  if (!dom || !sys || !ws || !scratch || !err_flag) return SPI_ERR_ARG;
+  if (sys->n_sys < 0 || sys->n_sys > 65535) return SPI_ERR_TOO_LARGE;
+  if (sys->kind == SPI_KIND_SK || sys->n_sys == 0 || dom->n_cells == 0) return SPI_OK;
+  if (int rc = check_var_df(dom, sys, ws)) return rc;
+  if (!ws->linv_arena) return SPI_ERR_ARG;
+  SlicesCall c = {};
+  c.dom = *dom;
+  c.sys = *sys;
+  c.ws = *ws;
+  c.cond_split = cond_cap;
+  c.want_var = 1;
+  c.filter = 3;
+  c.scratch = scratch;
+  c.scratch_bytes = scratch_bytes;
+  c.err = err_flag;
+  VarDfArgs A{*dom, *sys, *ws, cond_cap, nullptr, 0};
+  const int rc = launch_slices(c, &A.skip, &A.skip_stride, (cudaStream_t)stream);
+  return rc ? rc : launch_var_df(A, (cudaStream_t)stream);
 }

@@ -71,6 +71,12 @@ _TILE_CACHE = {}
 # the step-by-step Gauss-Jordan elimination over the whole GPU on the
 # exact-inverse path (2 launches per row); smaller ones one CTA each
 GJ_MULTI_MIN_M = 256
+# systems of at least this many stations take the FP64 cell pass through the
+# sliced tensor-core contraction (spi_krige_cells_sliced): at 64 stations the
+# two take the same time (0.31 ms a plan on 128 cells, launches), from 65 on
+# the sliced one is faster (150 stations: 2.5 -> 0.34 ms); below, a stage of
+# 16 stations and a block of 64 rows are mostly padding
+SLICES_MIN_N = 64
 
 
 def parse_vg(vg_str):
@@ -376,10 +382,51 @@ class _KrigeBatch:
                                      None, **extra)
         self.ws_probe_df = (nat.KrigeWsT(*ptrs, _ptr(self.probe_df[0]), None, None, **extra)
                             if self.probe_df else None)
+        # the FP64 pass on the tensor cores: (scratch, error flag), set by
+        # the plan for its batches (None: the FP64 kernels)
+        self.slices = None
+        self.n_drift = dom.st.n_drift if kind == "EDK" else 0
+        self.max_steps = max(len(x) for x in steps_l)
         # algorithmic FLOP of the cell kernel: per (system, cell) the
         # triangular variance n(n+1), the dual columns 2na; per cell-step 2n
         self.n = ns
         self.n_steps = np.array([len(x) for x in steps_l], dtype=np.int64)
+
+    def slices_bytes(self, want_var):
+        """Scratch of the sliced tensor-core contraction: 0 for systems too
+        small for it."""
+        n = int(self.n.max())
+        if n < SLICES_MIN_N:
+            return 0
+        lib = nat.lib()
+        need = lib.spi_slices_scratch_bytes(n, len(self.ch), self.max_steps, self.n_drift,
+                                            int(want_var), 1)
+        if self.precision == 1 and want_var:
+            need = max(need, lib.spi_slices_scratch_bytes(n, len(self.ch), 0, 0, 1, 0))
+        return int(need)
+
+    def cells_fp64(self, dom, out, want_var, filt, cond_split, tile, s):
+        """The FP64 cell pass on the cells of dom: the sliced tensor-core
+        contraction where the batch has its scratch, else the FP64
+        kernels."""
+        args = (ctypes.byref(dom.st), ctypes.byref(self.sy), _ptr(self.vals),
+                ctypes.byref(self.ws if out[1] else self.ws_probe), 1 if want_var else 0)
+        if self.slices is None:
+            nat.call("spi_krige_cells_tiled", *args, 0, filt, float(cond_split),
+                     ctypes.byref(out[0]), tile, s)
+            return
+        scratch, err = self.slices
+        nat.call("spi_krige_cells_sliced", *args, filt, float(cond_split), ctypes.byref(out[0]),
+                 tile, self.max_steps, _ptr(scratch), scratch.numel(), _ptr(err), s)
+
+    def var_df(self, dom, ws, cond_cap, s):
+        """|Linv c|^2 of the double-float tier's systems on the cells of dom."""
+        args = (ctypes.byref(dom.st), ctypes.byref(self.sy), ctypes.byref(ws), float(cond_cap))
+        if self.slices is None:
+            nat.call("spi_krige_var_df", *args, s)
+            return
+        scratch, err = self.slices
+        nat.call("spi_krige_var_sliced", *args, _ptr(scratch), scratch.numel(), _ptr(err), s)
 
     def cell_flops(self, C, want_var, a):
         per = 2 * self.n * a + 2 * self.n * self.n_steps
@@ -461,16 +508,14 @@ class _KrigeBatch:
             # regenerates the right-hand sides for every four dual vectors:
             # slower than FP64 on systems shared by hundreds of steps)
             cap = max(float(cond_split), cond_df) if self.probe_df else float(cond_split)
-            for prec, filt, o in ((1, 1, o32), (0, 0, o64)):
-                nat.call("spi_krige_cells", ctypes.byref(pdom.st), ctypes.byref(self.sy),
-                         _ptr(self.vals), wp, 1 if want_var else 0, prec, filt,
-                         cap if prec == 1 else float(cond_split), ctypes.byref(o), s)
+            nat.call("spi_krige_cells", ctypes.byref(pdom.st), ctypes.byref(self.sy),
+                     _ptr(self.vals), wp, 1 if want_var else 0, 1, 1, cap, ctypes.byref(o32), s)
+            self.cells_fp64(pdom, (o64, False), want_var, 0, cond_split, 0, s)
             pv32d = None
             if self.probe_df is not None and want_var:
                 pyy_d, _, pv32d, o32d = self.probe_df
                 wpd = ctypes.byref(self.ws_probe_df)
-                nat.call("spi_krige_var_df", ctypes.byref(pdom.st), ctypes.byref(self.sy), wpd,
-                         cap, s)
+                self.var_df(pdom, self.ws_probe_df, cap, s)
                 nat.call("spi_krige_cells", ctypes.byref(pdom.st), ctypes.byref(self.sy),
                          _ptr(self.vals), wpd, 1, 1, 1, cap, ctypes.byref(o32d), s)
             nat.call("spi_krige_tier", ctypes.byref(self.sy), ws, pdom.C, _ptr(pe64), _ptr(pe32),
@@ -482,12 +527,14 @@ class _KrigeBatch:
                 "spi_krige_var_tc", ctypes.byref(dom.st), ctypes.byref(self.sy), ws,
                 float(cond_split), _ptr(self.tc_err), s))
             if self.tier is not None:
-                timed("var_df", lambda: nat.call(
-                    "spi_krige_var_df", ctypes.byref(dom.st), ctypes.byref(self.sy), ws,
-                    float(cond_split), s))
+                timed("var_df", lambda: self.var_df(dom, self.ws, cond_split, s))
         self.var_cells.zero_()
         for prec, filt in self.passes():
             tile = self.tiles.get((prec, filt), 0)
+            if prec == 0:
+                timed("cells_fp64", lambda filt=filt, tile=tile: self.cells_fp64(
+                    dom, (out, True), want_var, filt, cond_split, tile, s))
+                continue
             timed("cells_fp32" if prec == 1 else "cells_fp64", lambda prec=prec, filt=filt,
                   tile=tile: nat.call(
                 "spi_krige_cells_tiled", ctypes.byref(dom.st), ctypes.byref(self.sy),
@@ -516,6 +563,20 @@ class _KrigeBatch:
         panels = (n + 31) // 32 - 1
         levels = panels.bit_length()
         return (2 * panels + 2 * levels + 1) * (3 if self.l32 is not None else 1)
+
+    def slices_launches(self, fields):
+        """Kernels of a sliced contraction beside the FP64 kernel's own: the
+        coordinates' range, and per group of systems the selection, the row
+        exponents, the pack and the contraction."""
+        if self.slices is None:
+            return 0
+        n, lib = int(self.n.max()), nat.lib()
+        var = int(self.X is not None)
+        args = (self.max_steps if fields else 0, self.n_drift if fields else 0, var, int(fields))
+        one, two = (lib.spi_slices_scratch_bytes(n, k, *args) for k in (1, 2))
+        room = self.slices[0].numel() - one
+        group = min(256, 1 + max(0, room) // max(1, two - one))
+        return 1 + 4 * (-(-len(self.ch) // group))
 
     def passes(self):
         """The cell-kernel passes of run(): (precision, route filter)."""
@@ -670,6 +731,18 @@ class InterpPlan:
                     _fill_args(dev, mean_steps, means[mean_steps], np.zeros(len(mean_steps))))
                 a = 1 + self.dom.st.n_drift if kind == "EDK" else 1
                 self.krig.append((kind, out, var is not None, batches, fills, a))
+        # scratch of the sliced tensor-core contraction, shared by the
+        # batches, which run in stream order
+        self.slices_err = None
+        if tensor_cores and self.krig:
+            need = [(b, b.slices_bytes(k[2])) for k in self.krig for b in k[3]]
+            most = max((n for _, n in need), default=0)
+            if most > 0:
+                self.slices_err = torch.zeros(1, dtype=torch.int32, device=dev)
+                shared = (torch.empty(most, dtype=torch.uint8, device=dev), self.slices_err)
+                for b, n in need:
+                    if n > 0:
+                        b.slices = shared
         self.idw = []
         self.idw_pack = self.idw_err = None
         if any(t in ("IDW", "NNB") for t in types):
@@ -823,6 +896,8 @@ class InterpPlan:
         if self.idw_err is not None and int(self.idw_err.item()):
             raise RuntimeError("spi_idw_cells_tc: a tensor-core wait timed out (its cells hold "
                                "NaN)")
+        if self.slices_err is not None and int(self.slices_err.item()):
+            raise RuntimeError("spi_krige_cells_sliced: a tensor-core wait timed out")
         for kind, out, want_var, batches, fills, a in self.krig:
             failed, routed, cond, pinv = [], [], {}, []
             for b in batches:
@@ -915,6 +990,13 @@ class InterpPlan:
                 n += 1 if (b.yy is not None and want_var) else 0
                 n += 1 if (b.yy is not None and want_var and b.tier is not None) else 0
                 n += 2 if b.precision == 1 else 1
+                # the FP64 pass, its probe, the double-float tier's two
+                n += b.slices_launches(True) * (1 + (b.probe is not None
+                                                     and self.pdom is not None))
+                if b.yy is not None and want_var:
+                    n += b.slices_launches(False) * (
+                        (b.tier is not None) + (b.probe_df is not None
+                                                and self.pdom is not None))
         n += len(self.post_fills)
         for t, out, fill, p in self.idw:
             n += (fill is not None) + (len(self.multi) > 0) * (

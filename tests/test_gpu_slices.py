@@ -1,0 +1,87 @@
+"""The FP64 cell pass as sliced tensor-core products (csrc/spi_slices.cu) at
+the sizes where it can go wrong: around a 16-station stage, a 64-row block, a
+128-station drain, a 128-cell tile; several blocks of steps; every model with
+a fixed-point form, nests, and models without one (which keep the FP64
+kernels) in the same batch.
+
+Against the oracle at the FP64 path's bar, 1e-9 of the field's largest
+magnitude, and against the FP64 kernels (tensor_cores=False) at 1e-11: both
+are FP64 evaluations of the same formulas from the same factor (condition up
+to 1e5, so rounding of 1e-16 may grow to 1e-11).
+"""
+import numpy as np
+import pytest
+
+pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from oracle import port  # noqa: E402
+
+
+def _run(n, T, C, methods, vgs, seed, drifts=0, min_vg=1e-4, oracle=True, precision="fp64"):
+    from spinterps_gb300 import steps
+    rng = np.random.default_rng(seed)
+    box = 8e3 * np.sqrt(n)
+    sx, sy = rng.uniform(0, box, n), rng.uniform(0, box, n)
+    z = 3.0 + rng.normal(size=(T, n))
+    cx, cy = rng.uniform(0, box, C), rng.uniform(0, box, C)
+    cx[0], cy[0] = sx[1], sy[1]          # a cell on a station
+    est_vars = "OK" in methods
+    args = port.interp_args_for(methods, est_vars=est_vars)
+    kw = dict(est_vars=est_vars, min_vg_val=min_vg, intrp_dtype=np.float64)
+    if drifts:
+        kw.update(stn_drifts=rng.uniform(0, 1, (n, drifts)),
+                  cell_drifts=rng.uniform(0, 1, (drifts, C)))
+    vgs = [vgs[t % len(vgs)] for t in range(T)]
+    got, plain = (steps.interp_steps(sx, sy, z, cx, cy, vgs, args, precision=precision,
+                                     tensor_cores=tc, **kw)[0] for tc in (True, False))
+    bar = 1e-11 if precision == "fp64" else 1e-5
+    for lab in plain:
+        sc = np.nanmax(np.abs(plain[lab]))
+        assert np.nanmax(np.abs(got[lab] - plain[lab])) <= bar * sc, (n, lab)
+    if oracle:
+        ref, _ = port.interp_steps(sx, sy, z, cx, cy, vgs, args, **kw)
+        for lab in ref:
+            sc = np.nanmax(np.abs(ref[lab]))
+            assert np.nanmax(np.abs(got[lab] - ref[lab])) <= max(bar, 1e-9) * sc, (n, lab)
+
+
+EXP = "0.05 Nug(0.0) + 0.95 Exp(20000)"
+
+
+@pytest.mark.parametrize("n", [64, 65, 79, 80, 81, 127, 128, 129, 144, 145, 192, 193, 257])
+def test_station_counts(n):
+    _run(n, 3, 131, ["OK", "SK"], [EXP], 10 + n)
+
+
+@pytest.mark.parametrize("C", [1, 127, 128, 129, 257])
+def test_cell_counts(C):
+    _run(70, 2, C + 1, ["OK"], [EXP], 30 + C)
+
+
+@pytest.mark.parametrize("T,drifts", [(63, 0), (64, 0), (65, 0), (62, 1), (130, 3)])
+def test_blocks_of_steps(T, drifts):
+    _run(66, T, 40, ["EDK"] if drifts else ["OK"], [EXP], 50 + T, drifts)
+
+
+@pytest.mark.parametrize("vg", ["0.9 Sph(60000)", "0.9 Lin(400000)", "0.00001 Exp(1.0) + 0.9 Gau(15000)",
+                                "0.3 Sph(50000) + 0.1 Nug(0.0) + 0.6 Exp(90000)",
+                                "0.00005 Nug(0.0) + 1.4 Sph(30000)"])
+def test_models(vg):
+    _run(100, 2, 150, ["OK", "SK"], [vg], 70, oracle="Lin" not in vg)
+
+
+def test_models_without_a_sliced_form():
+    """Hol and Pow beside Exp in one batch."""
+    _run(90, 6, 140, ["OK"], [EXP, "0.9 Hol(9000) + 0.3 Exp(20000)", "0.0001 Pow(0.9)"], 80,
+         oracle=False)
+
+
+@pytest.mark.parametrize("min_vg", [0.0, 0.02, 0.3])
+def test_cut(min_vg):
+    _run(80, 2, 200, ["OK"], ["0.95 Exp(30000)"], 90, min_vg=min_vg, oracle=min_vg < 0.1)
+
+
+def test_double_float_tier():
+    """Mixed precision: ill-conditioned systems take the sliced variance."""
+    _run(150, 3, 300, ["OK"], ["0.00001 Exp(1.0) + 0.9 Gau(25000)"], 95, precision="mixed")
