@@ -468,6 +468,10 @@ int spi_krige_var_sliced(const spi_domain_t *dom, const spi_systems_t *sys,
                          const spi_krige_ws_t *ws, double cond_cap, void *scratch,
                          int64_t scratch_bytes, int32_t *err_flag, spi_stream_t stream);
 
+/* Device scratch of a sliced contraction of n entries per cell against
+ * `rows` rows (spi_legacy_points_sliced). */
+int64_t spi_slices_one_scratch_bytes(int32_t n, int32_t rows);
+
 /* Device scratch of spi_krige_cells_sliced (want_fields 1) or
  * spi_krige_var_sliced (want_fields 0) on the current device. */
 int64_t spi_slices_scratch_bytes(int32_t max_n, int32_t n_sys, int32_t max_steps,
@@ -829,6 +833,18 @@ int spi_legacy_points(int32_t kind, const double *xi, const double *yi, const do
                       const spi_vg_t *vg, const double *lhs_inv, double *rhss,
                       double *lambdas, double *mus, double *zk, double *est, double *ik,
                       spi_stream_t stream);
+
+/* The same with lambda = P r as sliced tensor-core products (55-bit
+ * operands, exact sums). scratch: spi_slices_one_scratch_bytes(m, m), m the
+ * matrix's rows; err_flag (device, 0 on entry): set to 1 when a tensor-core
+ * wait ran out, and the FP64 kernel then computes the weights. */
+int spi_legacy_points_sliced(int32_t kind, const double *xi, const double *yi, const double *zi,
+                      const double *ixi, int32_t n, const double *xk, const double *yk,
+                      const double *sk_drift, int64_t n_out, int32_t n_drift,
+                      const spi_vg_t *vg, const double *lhs_inv, double *rhss,
+                      double *lambdas, double *mus, double *zk, double *est, double *ik,
+                      void *scratch, int64_t scratch_bytes,
+                             int32_t *err_flag, spi_stream_t stream);
 
 /* The pseudo-inverse P of a symmetric m x m matrix M (device arrays,
  * row-major, m <= SPI_PINV_MAX_M), for the single-neighbourhood classes'

@@ -164,6 +164,9 @@ _SIGS = {
     "spi_legacy_points": [c_i32, c_ptr, c_ptr, c_ptr, c_ptr, c_i32, c_ptr, c_ptr, c_ptr, c_i64,
                           c_i32, ctypes.POINTER(VgT), c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
                           c_ptr, c_ptr],
+    "spi_legacy_points_sliced": [c_i32, c_ptr, c_ptr, c_ptr, c_ptr, c_i32, c_ptr, c_ptr, c_ptr,
+                                 c_i64, c_i32, ctypes.POINTER(VgT), c_ptr, c_ptr, c_ptr, c_ptr,
+                                 c_ptr, c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_ptr],
     "spi_sym_pinv": [c_ptr, c_i32, c_dbl, c_ptr, c_ptr, c_ptr, c_ptr],
     "spi_local_groups": [ctypes.POINTER(DomainT), c_i32, c_i32, c_ptr, c_i32, c_ptr, c_ptr,
                          c_i32, c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_ptr, c_dbl, c_i32,
@@ -174,7 +177,8 @@ _SIGS = {
 
 # every entry point the header declares (checked by the CPU tests)
 EXPORTS = sorted(list(_SIGS) + ["spi_version", "spi_cuda_error", "spi_mlp_n_params",
-                                 "spi_local_groups_scratch_bytes", "spi_slices_scratch_bytes"])
+                                 "spi_local_groups_scratch_bytes", "spi_slices_scratch_bytes",
+                                 "spi_slices_one_scratch_bytes"])
 
 _lib = None
 _lock = threading.Lock()
@@ -203,6 +207,8 @@ def load(path=LIB_PATH):
         lib.spi_mlp_n_params.argtypes = [c_i32, c_i32, c_i32, c_i32]
         lib.spi_local_groups_scratch_bytes.restype = c_i64
         lib.spi_local_groups_scratch_bytes.argtypes = [c_i32, c_i32, c_i32, c_i32, c_i32]
+        lib.spi_slices_one_scratch_bytes.restype = c_i64
+        lib.spi_slices_one_scratch_bytes.argtypes = [c_i32, c_i32]
         lib.spi_slices_scratch_bytes.restype = c_i64
         lib.spi_slices_scratch_bytes.argtypes = [c_i32] * 6
         _lib = lib

@@ -6,9 +6,9 @@
 // 32 x 32 -> 64 bit products among them at half rate: the coordinates as
 // 62-bit integers on a common grid, the distance's square and root by
 // normalised 64-bit products, the model in fixed point. The result is the
-// correlation-like c / (the structures' sills) as an integer of FX_BITS = 54 bits with an
-// error of about one unit, 2^-54 of those sills: FP64's own rounding of
-// entries near the sill, and less than it of the intermediate steps.
+// correlation-like c / (the structures' sills) as an integer of FX_BITS = 62 bits with an
+// error of about 2^-56 of those sills (rms 2^-58 for one structure), where an
+// FP64 evaluation is off by 2^-54 (rms).
 //
 // The functions are host and device code, so that their error can be
 // measured against wider arithmetic on the CPU.
@@ -22,7 +22,7 @@
 
 namespace spi {
 
-constexpr int FX_BITS = 54;                    // an entry of the structures' sills is 2^54
+constexpr int FX_BITS = 62;                    // an entry of the structures' sills is 2^62
 constexpr int FX_GRID = 61;                    // coordinates: |X| <= 2^61
 
 #define FX_HD __host__ __device__ __forceinline__
@@ -63,6 +63,14 @@ FX_HD float fx_rsqrt(float x) {
 #endif
 }
 
+FX_HD float fx_rcpf(float x) {
+#ifdef __CUDA_ARCH__
+  return __fdividef(1.0f, x);
+#else
+  return 1.0f / x;
+#endif
+}
+
 // The common grid of a domain: X = (x - ox) 2^q.
 struct FxGrid {
   double ox, oy;
@@ -75,6 +83,22 @@ FX_HD int64_t fx_coord(double x, double o, int q) {
   const double b = d - x;
   const double e = (x - (d - b)) - (o + b);
   return llrint(ldexp(d, q)) + llrint(ldexp(e, q));
+}
+
+// x on the grid without an origin, by integer shifts: X = x 2^q, for
+// |x| < 2^(FX_GRID - q); places finer than the grid are cut off.
+FX_HD int64_t fx_coord0(double x, int q) {
+#ifdef __CUDA_ARCH__
+  const int64_t b = __double_as_longlong(x);
+#else
+  int64_t b;
+  __builtin_memcpy(&b, &x, 8);
+#endif
+  const int e = (int)((b >> 52) & 0x7ff);
+  const int64_t m = (b & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
+  const int sh = (e ? e : 1) - 1075 + q;  // x = m 2^(e - 1075)
+  const int64_t v = sh >= 0 ? m << (sh < 63 ? sh : 63) : m >> (-sh < 63 ? -sh : 63);
+  return b < 0 ? -v : v;
 }
 
 // A positive double as a 64-bit mantissa and an exponent: v = m 2^e, m with
@@ -100,7 +124,7 @@ struct FxVg {
   int sk;
   int64_t cut;    // min_vg_val's boundary, in units; < 0: no cut
   int64_t over;   // what an entry past the cut becomes
-  double sill;    // the structures' total sill: an entry's unit is sill 2^-54
+  double sill;    // the structures' total sill: an entry's unit is sill 2^-FX_BITS
 };
 
 // x / y of two positive doubles as Q64 (x <= y; the ratio 1 saturates).
@@ -237,6 +261,17 @@ FX_HD uint64_t fx_sqrt(uint64_t S) {
   return H + (uint64_t)(int64_t)i2;
 }
 
+// 2^126 / M in Q62 of a normalised M (top bit set): FP32's reciprocal, then
+// two Newton steps (relative 2^-44, 2^-60).
+FX_HD uint64_t fx_rcp(uint64_t M) {
+  const float y = fx_rcpf((float)(uint32_t)(M >> 32));
+  uint64_t R = (uint64_t)(uint32_t)(y * 4611686018427387904.0f) << 32;
+  int64_t E = (int64_t)((1ull << 62) - fx_mulh(M, R));  // (1 - m r) 2^62
+  R += (uint64_t)(((int64_t)(R >> 32) * (int32_t)(E >> 16)) >> 14);
+  E = (int64_t)((1ull << 62) - fx_mulh(M, R));
+  return R + (uint64_t)(((int64_t)(R >> 32) * (int32_t)E) >> 30);
+}
+
 // A cell-station distance on the grid: S = h^2 2^(2 L - 66) in [2^60, 2^63),
 // 0 when the points coincide.
 struct FxDist {
@@ -275,19 +310,19 @@ FX_HD int64_t fx_rho(int code, const FxComp& k, FxDist d, uint64_t H, const uint
       // h / r in Q62
       const bool out = sh < 0 || t0 >= (1ull << 62);
       if (code == SPI_VG_LIN) {
-        v = (int64_t)(((1ull << 62) - t0 + 128) >> 8);
+        v = (int64_t)((1ull << 62) - t0);
       } else {
         // 1 - t (3 - t^2) / 2
         const uint64_t t = t0 << 1;                             // Q63
         const uint64_t t2 = fx_mulh(t, t);                     // Q62
         const uint64_t b = fx_mulh(t, (3ull << 62) - t2);      // Q61
-        v = ((int64_t)1 << FX_BITS) - (int64_t)((b + 128) >> 8);
+        v = ((int64_t)1 << FX_BITS) - (int64_t)b;
       }
       v = out ? 0 : v;
     }
   }
   v = d.S == 0 ? (int64_t)1 << FX_BITS : v;
-  return k.w == ~0ull ? v : (int64_t)(fx_mulh((uint64_t)v << 9, k.w) >> 9);
+  return k.w == ~0ull ? v : (int64_t)(fx_mulh((uint64_t)v << 1, k.w) >> 1);
 }
 
 // N entries of one cell, before the min_vg_val cut. CODE: the model of a
@@ -317,6 +352,33 @@ FX_HD int64_t fx_entry(const FxVg& f, int64_t cx, int64_t cy, int64_t sx, int64_
   int64_t v[1];
   fx_entries<-1, 1>(f, d, tab, v);
   return v[0];
+}
+
+// A squared distance as a monotone key: the exponent above 55 bits of the
+// normalised square (its top bit set). 0: the points coincide.
+FX_HD uint64_t fx_key(FxDist d) {
+  const int z = fx_clz(d.S | 1);
+  return d.S ? ((uint64_t)(200 - 2 * d.L - z) << 55) + ((d.S << z) >> 9) : 0ull;
+}
+
+// The inverse-square weight (h_ref / h)^2 <= 1 as a double, by its bits (no
+// FP64 operation); ref: the key of the smallest distance. Relative error
+// 2^-53 (the rounding) and a few 2^-59. d.S != 0.
+FX_HD double fx_weight2(FxDist d, uint64_t ref) {
+  const int z = fx_clz(d.S | 1);
+  const uint64_t q = fx_mulh((ref & ((1ull << 55) - 1)) << 9, fx_rcp(d.S << z));  // Q62
+  const int c = fx_clz(q);
+  // the top 53 bits, rounded (a carry into the exponent comes out right)
+  const uint64_t m = ((q << c) >> 11) + (((q << c) >> 10) & 1);
+  const int e = 1024 - c - ((200 - 2 * d.L - z) - (int)(ref >> 55));
+  const uint64_t b = ((uint64_t)(e - 1) << 52) + m;
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)b);
+#else
+  double w;
+  __builtin_memcpy(&w, &b, 8);
+  return w;
+#endif
 }
 
 }  // namespace spi

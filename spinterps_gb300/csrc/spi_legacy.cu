@@ -13,13 +13,16 @@
 //   krige() subtracts gamma off the diagonal (lines 397-399, 413, 432-442); its
 //   right-hand side is total sill - gamma (total sill at distance 0).
 //
-// Kernels: k_leg_system (one CTA: distances, the matrix, its Gauss-Jordan
-// inverse in place of numpy.linalg.pinv); k_leg_rhs (every point's
-// right-hand side, grid-stride); k_leg_lambda (lambda = P r for every
-// point: an FP64 tiled contraction R P' over shared-memory tiles);
-// k_leg_finish (a warp per point: estimate, variance, indicator).
+// Kernels: the distances, the matrix and its Gauss-Jordan inverse in place of
+// numpy.linalg.pinv (k_leg_system, one CTA, for small matrices; else k_leg_fill
+// .. k_leg_dists, every elimination step spread over the GPU); k_leg_rhs
+// (every point's right-hand side, grid-stride); lambda = P r for every point
+// as sliced tensor-core products (spi_slices.cu; without their scratch
+// k_leg_lambda, an FP64 tiled contraction); k_leg_finish (a warp per point:
+// estimate, variance, indicator).
 #include "spi_common.cuh"
 #include "spi_gj.cuh"
+#include "spi_slices.cuh"
 
 namespace spi {
 
@@ -45,6 +48,22 @@ __device__ __forceinline__ double leg_total_sill(const spi_vg_t& vg) {
   return t;
 }
 
+// Entry (i, j) of the kriging matrix.
+__device__ __forceinline__ double leg_entry(int sk, const double* xi, const double* yi, int n,
+                                            const double* si, const spi_vg_t& vg, int i, int j) {
+  if (i < n && j < n) {
+    if (i == j) return 0.0;
+    const int lo = min(i, j), hi = max(i, j);
+    const double g = leg_gamma(vg, dist_f64(xi[lo], yi[lo], xi[hi], yi[hi]));
+    // SK: 0.0 - g_0 - g_1 ... == -(g_0 + g_1 + ...) exactly
+    return sk ? -g : g;
+  }
+  if (i >= n && j >= n) return 0.0;
+  const int st = (i < n) ? i : j;
+  const int k = (i < n) ? (j - n) : (i - n);
+  return (k == 0) ? 1.0 : si[(int64_t)(k - 1) * n + st];
+}
+
 // Distances, the kriging matrix and its inverse of one station set.
 __global__ __launch_bounds__(LT) void k_leg_system(int sk, const double* __restrict__ xi,
                                                    const double* __restrict__ yi, int n,
@@ -59,24 +78,10 @@ __global__ __launch_bounds__(LT) void k_leg_system(int sk, const double* __restr
   const int m = n + a;
   for (int64_t e = tid; e < (int64_t)m * m; e += LT) {
     const int i = (int)(e / m), j = (int)(e - (int64_t)i * m);
-    double val;
+    const double val = leg_entry(sk, xi, yi, n, si, vg, i, j);
     if (i < n && j < n) {
-      double d = 0.0;
-      val = 0.0;
-      if (i != j) {
-        const int lo = min(i, j), hi = max(i, j);
-        d = dist_f64(xi[lo], yi[lo], xi[hi], yi[hi]);
-        const double g = leg_gamma(vg, d);
-        // SK: 0.0 - g_0 - g_1 ... == -(g_0 + g_1 + ...) exactly
-        val = sk ? -g : g;
-      }
-      dists[(int64_t)i * n + j] = d;
-    } else if (i >= n && j >= n) {
-      val = 0.0;
-    } else {
-      const int st = (i < n) ? i : j;
-      const int k = (i < n) ? (j - n) : (i - n);
-      val = (k == 0) ? 1.0 : si[(int64_t)(k - 1) * n + st];
+      const int lo = min(i, j), hi = max(i, j);
+      dists[(int64_t)i * n + j] = i == j ? 0.0 : dist_f64(xi[lo], yi[lo], xi[hi], yi[hi]);
     }
     lhs[e] = val;
     inv[e] = val;
@@ -116,6 +121,160 @@ __global__ __launch_bounds__(LT) void k_leg_system(int sk, const double* __restr
   }
 }
 
+// ---- the same spread over the GPU ----
+// One CTA updates an m x m matrix at a few FP64 operations per clock: 48 ms at
+// m = 401, where the step-by-step launches below take 2 m launches of a few
+// microseconds. The operations are those of gj_invert in its order, so the
+// inverse is the same to the last bit. The pivots sit in the distance array,
+// filled last; *status holds 0, or the failing step + 1.
+constexpr int LS_MIN_M = 96;  // below, 2 m launches outlast the one CTA (2.4 ms at 96)
+
+__global__ void k_leg_fill(int sk, const double* __restrict__ xi, const double* __restrict__ yi,
+                           int n, const double* __restrict__ si, int m, spi_vg_t vg,
+                           double* __restrict__ lhs, double* __restrict__ inv,
+                           int32_t* __restrict__ status) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)m * m;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(e / m), j = (int)(e - (int64_t)i * m);
+    lhs[e] = inv[e] = leg_entry(sk, xi, yi, n, si, vg, i, j);
+  }
+}
+
+// Step k: the pivot (first row of maximum |A[i][k]|, i >= k), the row swap,
+// the pivot row scaled.
+__global__ __launch_bounds__(LT) void k_leg_pivot(double* __restrict__ A, int m, int k,
+                                                  int32_t* __restrict__ piv,
+                                                  int32_t* __restrict__ status) {
+  if (*status) return;
+  __shared__ double rv[LT / 32];
+  __shared__ int ri[LT / 32];
+  __shared__ double dk;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double best = -1.0;
+  int bi = 0x7fffffff;
+  auto take = [&](double x, int i) {
+    if (x > best || (x == best && i < bi)) {
+      best = x;
+      bi = i;
+    }
+  };
+  for (int i = k + tid; i < m; i += LT) {
+    const double x = fabs(A[(int64_t)i * m + k]);
+    take(isnan(x) ? __longlong_as_double(0x7ff0000000000000LL) : x, i);
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    take(__shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, bi, o));
+  if (lane == 0) {
+    rv[warp] = best;
+    ri[warp] = bi;
+  }
+  __syncthreads();
+  best = rv[0];
+  bi = ri[0];
+  for (int w = 1; w < LT / 32; ++w) take(rv[w], ri[w]);
+  if (!(best > 0.0) || isinf(best)) {
+    if (tid == 0) *status = k + 1;
+    return;
+  }
+  const int p = bi;
+  if (tid == 0) {
+    piv[k] = p;
+    dk = A[(int64_t)p * m + k];
+  }
+  __syncthreads();
+  const double dd = dk;
+  for (int j = tid; j < m; j += LT) {
+    const double x = A[(int64_t)p * m + j];
+    if (p != k) A[(int64_t)p * m + j] = A[(int64_t)k * m + j];
+    A[(int64_t)k * m + j] = (j == k ? 1.0 : x) / dd;
+  }
+}
+
+// Step k: column k eliminated from every other row, a warp per row.
+__global__ __launch_bounds__(256) void k_leg_update(double* __restrict__ A, int m, int k,
+                                                    const int32_t* __restrict__ status) {
+  if (*status) return;
+  const int lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (i >= m || i == k) return;
+  const double* prow = A + (int64_t)k * m;
+  double* row = A + (int64_t)i * m;
+  const double fi = row[k];
+  __syncwarp();  // (read before the lane of column k writes it)
+  for (int j = lane; j < m; j += 32) {
+    const double base = (j == k) ? 0.0 : row[j];
+    row[j] = base - fi * prow[j];
+  }
+}
+
+// Columns back into place: the reverse pivot swaps as one permutation, a row
+// at a time through shared memory.
+__global__ __launch_bounds__(256) void k_leg_unscramble(double* __restrict__ A, int m,
+                                                        const int32_t* __restrict__ piv,
+                                                        const int32_t* __restrict__ status) {
+  if (*status) return;
+  extern __shared__ double buf[];  // [m] a row, then the permutation
+  int* at = reinterpret_cast<int*>(buf + m);
+  for (int j = threadIdx.x; j < m; j += 256) at[j] = j;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int k = m - 1; k >= 0; --k) {
+      const int p = piv[k];
+      const int t = at[k];
+      at[k] = at[p];
+      at[p] = t;
+    }
+  for (int i = blockIdx.x; i < m; i += gridDim.x) {
+    __syncthreads();
+    for (int j = threadIdx.x; j < m; j += 256) buf[j] = A[(int64_t)i * m + j];
+    __syncthreads();
+    for (int j = threadIdx.x; j < m; j += 256) A[(int64_t)i * m + j] = buf[at[j]];
+  }
+}
+
+// ||lhs||_F ||inv||_F, one CTA (a fixed order of summation).
+__global__ __launch_bounds__(1024) void k_leg_norms(const double* __restrict__ lhs,
+                                                    const double* __restrict__ inv, int m,
+                                                    const int32_t* __restrict__ status,
+                                                    double* __restrict__ cond) {
+  __shared__ double red[2][32];
+  const bool fail = *status != 0;
+  double sa = 0.0, sb = 0.0;
+  if (!fail)
+    for (int64_t e = threadIdx.x; e < (int64_t)m * m; e += 1024) {
+      sa = fma(lhs[e], lhs[e], sa);
+      sb = fma(inv[e], inv[e], sb);
+    }
+  for (int o = 16; o > 0; o >>= 1) {
+    sa += __shfl_xor_sync(0xffffffffu, sa, o);
+    sb += __shfl_xor_sync(0xffffffffu, sb, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = sa;
+    red[1][threadIdx.x >> 5] = sb;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sa = sb = 0.0;
+    for (int w = 0; w < 32; ++w) {
+      sa += red[0][w];
+      sb += red[1][w];
+    }
+    *cond = fail ? __longlong_as_double(0x7ff0000000000000LL) : sqrt(sa) * sqrt(sb);
+  }
+}
+
+__global__ void k_leg_dists(const double* __restrict__ xi, const double* __restrict__ yi, int n,
+                            double* __restrict__ dists) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n * n;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(e / n), j = (int)(e - (int64_t)i * n);
+    const int lo = min(i, j), hi = max(i, j);
+    dists[e] = i == j ? 0.0 : dist_f64(xi[lo], yi[lo], xi[hi], yi[hi]);
+  }
+}
+
 // rhss[k, :] of every point k.
 __global__ void k_leg_rhs(int sk, const double* __restrict__ xi, const double* __restrict__ yi,
                           int n, const double* __restrict__ xk, const double* __restrict__ yk,
@@ -151,7 +310,10 @@ __global__ void k_leg_rhs(int sk, const double* __restrict__ xi, const double* _
 __global__ __launch_bounds__(256) void k_leg_lambda(const double* __restrict__ rhss,
                                                     const double* __restrict__ inv, int64_t n_out,
                                                     int n, int m, double* __restrict__ lambdas,
-                                                    double* __restrict__ mus) {
+                                                    double* __restrict__ mus,
+                                                    const int32_t* __restrict__ done,
+                                                    const int32_t* __restrict__ err) {
+  if (done && *done && !*err) return;  // (after a timed-out wait: computed here)
   __shared__ double rs[LG_K][LG_T + 1];
   __shared__ double ps[LG_K][LG_T + 1];
   const int tid = threadIdx.x;
@@ -264,6 +426,25 @@ extern "C" int spi_legacy_system(int32_t kind, const double* xi, const double* y
   const int64_t m = (int64_t)n + (sk ? 0 : 1 + n_drift);
   const size_t smem = (size_t)m * (2 * sizeof(double) + sizeof(int));
   if (smem > 200 * 1024) return SPI_ERR_TOO_LARGE;
+  if (m >= spi::LS_MIN_M) {
+    cudaStream_t st = (cudaStream_t)stream;
+    const int mi = (int)m;
+    int32_t* piv = reinterpret_cast<int32_t*>(in_dists);  // n^2 doubles >= m ints
+    const int gx = (int)((m * m + 2047) / 2048);
+    spi::k_leg_fill<<<gx, 256, 0, st>>>(sk, xi, yi, n, si, mi, *vg, lhs, lhs_inv, status);
+    for (int k = 0; k < mi; ++k) {
+      spi::k_leg_pivot<<<1, spi::LT, 0, st>>>(lhs_inv, mi, k, piv, status);
+      spi::k_leg_update<<<(mi + 7) / 8, 256, 0, st>>>(lhs_inv, mi, k, status);
+    }
+    SPI_LAUNCH_CHECK();
+    const size_t us = (size_t)m * (sizeof(double) + sizeof(int));
+    if (!spi::smem_opt_in(spi::k_leg_unscramble, us)) return SPI_ERR_CUDA;
+    spi::k_leg_unscramble<<<mi < 304 ? mi : 304, 256, us, st>>>(lhs_inv, mi, piv, status);
+    if (cond) spi::k_leg_norms<<<1, 1024, 0, st>>>(lhs, lhs_inv, mi, status, cond);
+    spi::k_leg_dists<<<gx, 256, 0, st>>>(xi, yi, n, in_dists);
+    SPI_LAUNCH_CHECK();
+    return SPI_OK;
+  }
   if (!spi::smem_opt_in(spi::k_leg_system, smem)) return SPI_ERR_CUDA;
   spi::k_leg_system<<<1, spi::LT, smem, (cudaStream_t)stream>>>(sk, xi, yi, n, si, n_drift, *vg,
                                                                 in_dists, lhs, lhs_inv, status,
@@ -272,13 +453,13 @@ extern "C" int spi_legacy_system(int32_t kind, const double* xi, const double* y
   return SPI_OK;
 }
 
-extern "C" int spi_legacy_points(int32_t kind, const double* xi, const double* yi,
-                                 const double* zi, const double* ixi, int32_t n,
-                                 const double* xk, const double* yk, const double* sk_drift,
-                                 int64_t n_out, int32_t n_drift, const spi_vg_t* vg,
-                                 const double* lhs_inv, double* rhss, double* lambdas,
-                                 double* mus, double* zk, double* est, double* ik,
-                                 spi_stream_t stream) {
+// scratch (with err_flag): lambda = P r as sliced tensor-core products.
+static int leg_points(int32_t kind, const double* xi, const double* yi, const double* zi,
+                      const double* ixi, int32_t n, const double* xk, const double* yk,
+                      const double* sk_drift, int64_t n_out, int32_t n_drift, const spi_vg_t* vg,
+                      const double* lhs_inv, double* rhss, double* lambdas, double* mus,
+                      double* zk, double* est, double* ik, void* scratch, int64_t scratch_bytes,
+                      int32_t* err_flag, spi_stream_t stream) {
   int rc = leg_check(kind, xi, yi, n, sk_drift, n_drift, vg);
   if (rc) return rc;
   if (n_out < 0) return SPI_ERR_ARG;
@@ -297,10 +478,46 @@ extern "C" int spi_legacy_points(int32_t kind, const double* xi, const double* y
   SPI_LAUNCH_CHECK();
   dim3 grid((unsigned)((n_out + spi::LG_T - 1) / spi::LG_T),
             (unsigned)((m + spi::LG_T - 1) / spi::LG_T));
-  spi::k_leg_lambda<<<grid, 256, 0, st>>>(rhss, lhs_inv, n_out, n, m, lambdas, mus);
+  const int32_t* done = nullptr;
+  if (scratch) {
+    rc = spi::launch_slices_rows(spi::SlRows{rhss, lhs_inv, m, n, n_out, lambdas, mus}, scratch,
+                                 scratch_bytes, err_flag, &done, st);
+    if (rc) return rc;
+  }
+  spi::k_leg_lambda<<<grid, 256, 0, st>>>(rhss, lhs_inv, n_out, n, m, lambdas, mus, done,
+                                          err_flag);
   SPI_LAUNCH_CHECK();
   spi::k_leg_finish<<<(unsigned)((n_out * 32 + 255) / 256), 256, 0, st>>>(
       sk, zi, ixi, n, n_out, m, *vg, rhss, lambdas, mus, zk, est, ik);
   SPI_LAUNCH_CHECK();
   return SPI_OK;
+}
+
+extern "C" int spi_legacy_points(int32_t kind, const double* xi, const double* yi,
+                                 const double* zi, const double* ixi, int32_t n,
+                                 const double* xk, const double* yk, const double* sk_drift,
+                                 int64_t n_out, int32_t n_drift, const spi_vg_t* vg,
+                                 const double* lhs_inv, double* rhss, double* lambdas,
+                                 double* mus, double* zk, double* est, double* ik,
+                                 spi_stream_t stream) {
+  return leg_points(kind, xi, yi, zi, ixi, n, xk, yk, sk_drift, n_out, n_drift, vg, lhs_inv, rhss,
+                    lambdas, mus, zk, est, ik, nullptr, 0, nullptr, stream);
+}
+
+extern "C" int spi_legacy_points_sliced(int32_t kind, const double* xi, const double* yi,
+                                        const double* zi, const double* ixi, int32_t n,
+                                        const double* xk, const double* yk,
+                                        const double* sk_drift, int64_t n_out, int32_t n_drift,
+                                        const spi_vg_t* vg, const double* lhs_inv, double* rhss,
+                                        double* lambdas, double* mus, double* zk, double* est,
+                                        double* ik, void* scratch, int64_t scratch_bytes,
+                                        int32_t* err_flag, spi_stream_t stream) {
+  if (!scratch || !err_flag) return SPI_ERR_ARG;
+  return leg_points(kind, xi, yi, zi, ixi, n, xk, yk, sk_drift, n_out, n_drift, vg, lhs_inv, rhss,
+                    lambdas, mus, zk, est, ik, scratch, scratch_bytes, err_flag, stream);
+}
+
+extern "C" int64_t spi_slices_one_scratch_bytes(int32_t n, int32_t rows) {
+  if (n < 1 || rows < 1) return 0;
+  return spi::slices_scratch_one(n, rows);
 }

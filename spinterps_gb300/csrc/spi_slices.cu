@@ -7,19 +7,21 @@
 // GB300 does about 2 per SM and clock, 1800 times fewer than FP16 products
 // on the tensor cores.
 //
-// Every operand is an integer of 55 bits: a right-hand side entry c as
-// VA = c 2^54 / (the structures' sills) (spi_fx.cuh, generated in integers), a row of
-// Linv, of the dual columns or of the steps' dual weights as
-// VB = b 2^(54 - e), 2^e at least the row's largest magnitude. Each is cut into 7
-// balanced digits of 8 bits, VA = sum_i a_i 256^(6 - i), |a_i| <= 128, exact
-// in FP16. Products a_i b_j of one level i + j = l share an accumulator:
-// |sum| <= 7 * 2^14 * 128 < 2^24 over 128 stations, so its FP32 sums are
-// exact integers, whatever their order. Levels 0..7 (34 digit products) are
-// kept; the rest is under 2^-57 of full scale per product. After each 128
+// Every operand is an integer of 63 bits: a right-hand side entry c as
+// VA = c 2^62 / (the structures' sills) (spi_fx.cuh, generated in integers), a
+// row of Linv, of the dual columns or of the steps' dual weights as
+// VB = b 2^(62 - e), 2^e at least the row's largest magnitude. Each is cut
+// into 8 balanced digits of 8 bits, VA = sum_i a_i 256^(7 - i), |a_i| <= 128,
+// exact in FP16. Products a_i b_j of one level i + j = l share an accumulator:
+// |sum| <= 7.2 * 2^14 * 128 < 2^24 over 128 stations (a leading digit is at
+// most 80), so its FP32 sums are exact integers, whatever their order. Levels
+// 0..7 (36 digit products) are kept; the rest is under 2^-57 of full scale per
+// product. After each 128
 // stations the eight accumulators are added into a 96-bit integer per
 // (cell, row). Rounding happens in the
-// operands only, at 2^-55 of the largest entry, where FP64 rounds every
-// product and sum.
+// operands only, at 2^-63 of the largest entry, where FP64 rounds every
+// product and sum. (With 7 digits, 2^-55, the multipliers of 400 stations,
+// sums that cancel, were 8.5e-13 off where FP64 is 4.7e-13.)
 //
 // One persistent CTA per SM; a work item is (system, 128 cells).
 //   1. The threads generate the item's right-hand sides into the CTA's slot of
@@ -28,7 +30,7 @@
 //   2. Blocks of 64 rows (the 8 accumulators of 64 columns fill tensor
 //      memory): Linv's rows up to their diagonal, then dual columns and
 //      steps. Per 16 stations, the threads cut the slot's entries into FP16
-//      digits in shared memory, one thread copies the packed row digits (14
+//      digits in shared memory, one thread copies the packed row digits (16
 //      KB by a bulk copy, packed once per system) and issues 12 MMAs: digit
 //      i of the cells against digits 0..7-i of the rows, stacked along N,
 //      lands on levels i..7 at once. A ring of 5 stages; while a chunk's last
@@ -61,27 +63,31 @@ namespace {
 
 constexpr int SL_M = 128;                       // cells per item (MMA M)
 constexpr int SL_R = 64;                        // rows per block
-constexpr int SL_D = 7;                         // digits
+constexpr int SL_D = 8;                         // digits
 constexpr int SL_LV = 8;                        // levels kept
 constexpr int SL_K = 16;                        // stations per stage (one MMA K)
 constexpr int SL_KD = 128 / SL_K;               // stages per drain
-constexpr int SL_ST = 5;                        // ring stages
+constexpr int SL_ST = 4;                        // ring stages
 constexpr int SL_W = 16;                        // working warps
 constexpr int SL_WT = SL_W * 32;
 constexpr int SL_T = SL_WT + 64;                // and one each for MMAs and copies
 constexpr int SL_RT = SL_R * SL_M / SL_WT;      // rows of a block per working thread
 constexpr uint32_t SL_A_SLICE = SL_M * SL_K * 2;             // one digit of the cells
-constexpr uint32_t SL_A_BYTES = SL_D * SL_A_SLICE;           // 28 KB
-constexpr uint32_t SL_B_BYTES = SL_D * SL_R * SL_K * 2;      // 14 KB, one packed chunk
+constexpr uint32_t SL_A_BYTES = SL_D * SL_A_SLICE;           // 32 KB
+constexpr uint32_t SL_B_BYTES = SL_D * SL_R * SL_K * 2;      // 16 KB, one packed chunk
 constexpr uint32_t SL_STAGE = SL_A_BYTES + SL_B_BYTES;
 constexpr int SL_CAP = 256;                     // systems per launch
-constexpr uint64_t SL_BIAS = 0x80808080808080ull;
-constexpr int SL_BAND = 64;                     // units around the min_vg_val cut taken in FP64
+constexpr uint64_t SL_BIAS = 0x8080808080808080ull;
+constexpr int64_t SL_BAND = 64ll << (FX_BITS - 54);  // units around the min_vg_val cut taken in FP64
 
 // The launch's device-side header at the start of the scratch.
 struct SlHead {
   unsigned long long mn[2], mx[2];  // ordered encodings of the coordinates' range
 };
+
+// What a launch contracts: the kriging systems of a batch; given right-hand
+// sides against the rows of a matrix (the single-neighbourhood classes).
+enum SlMode { kKrige, kRows };
 
 // Per-system record.
 struct SlSys {
@@ -114,6 +120,7 @@ struct SlArgs {
   unsigned char* pack;
   unsigned char* slots;
   long slot_bytes;
+  SlRows rows;       // (kRows)
 };
 
 __device__ __forceinline__ unsigned long long enc(double x) {
@@ -156,6 +163,21 @@ __device__ __forceinline__ int dual_rows(const SlArgs& A, int route) {
   return extra_rows(A.sys.kind, A.dom.n_drift);
 }
 
+// The common grid of the range; false where it has none.
+__device__ bool sl_grid(const SlArgs& A, FxGrid& g) {
+  const double x0 = dec(A.head->mn[0]), x1 = dec(A.head->mx[0]);
+  const double y0 = dec(A.head->mn[1]), y1 = dec(A.head->mx[1]);
+  double ext = fmax(x1 - x0, y1 - y0);
+  g.ox = x0;
+  g.oy = y0;
+  const bool ok = ext >= 0.0 && ext < 1e200 && x0 > -1e250 && y0 > -1e250;
+  if (!(ext > 1e-200)) ext = 1e-200;
+  int e = 0;
+  frexp(ext, &e);
+  g.q = FX_GRID - 1 - e;
+  return ok;
+}
+
 // The grid, and which systems of the launch take this path: on the Cholesky
 // path (SK: also the exact-inverse path, whose estimates contract the same
 // covariances), every structure with a fixed-point form, and in the pass by
@@ -164,16 +186,7 @@ __global__ __launch_bounds__(256) void k_sl_select(SlArgs A) {
   __shared__ FxGrid g;
   __shared__ int ok;
   if (threadIdx.x == 0) {
-    const double x0 = dec(A.head->mn[0]), x1 = dec(A.head->mx[0]);
-    const double y0 = dec(A.head->mn[1]), y1 = dec(A.head->mx[1]);
-    double ext = fmax(x1 - x0, y1 - y0);
-    g.ox = x0;
-    g.oy = y0;
-    ok = ext >= 0.0 && ext < 1e200 && x0 > -1e250 && y0 > -1e250;
-    if (!(ext > 1e-200)) ext = 1e-200;
-    int e = 0;
-    frexp(ext, &e);
-    g.q = FX_GRID - 1 - e;
+    ok = sl_grid(A, g);
     if (blockIdx.x == 0) *A.grid = g;
   }
   __syncthreads();
@@ -198,24 +211,53 @@ __global__ __launch_bounds__(256) void k_sl_select(SlArgs A) {
   r.unit = e - 55;
 }
 
-// The row a block's row index names: variance rows first (blocks of 64),
-// then the dual columns and the steps. nullptr past the end.
-__device__ __forceinline__ const double* row_ptr(const SlArgs& A, int s, int n, int nvb, int row,
-                                                 int& len) {
-  const int64_t soff = A.sys.stn_off[s];
-  len = n;
-  if (row < nvb * SL_R) {
-    if (row >= n) return nullptr;
-    len = row + 1;
-    return A.ws.linv_arena + A.sys.mat_off[s] + (int64_t)row * n;
+// A row of the second operand: its first len values, zeros past them.
+struct RowRef {
+  const double* p;
+  int len;
+  __device__ __forceinline__ double at(int k) const { return k < len ? p[k] : 0.0; }
+};
+
+// The other mode's only "system".
+__global__ void k_sl_select_one(SlArgs A) { A.rec[0].use = 1; }
+
+// The row a block's row index names: variance rows first (in blocks), then
+// the dual columns and the steps.
+template <int MODE>
+__device__ __forceinline__ RowRef row_ref(const SlArgs& A, int s, int n, int nvb, int row) {
+  if constexpr (MODE == kRows) {
+    if (row >= n) return {nullptr, 0};
+    return {A.rows.inv + (int64_t)row * n, n};
+  } else {
+    const int64_t soff = A.sys.stn_off[s];
+    if (row < nvb * SL_R) {
+      if (row >= n) return {nullptr, 0};
+      return {A.ws.linv_arena + A.sys.mat_off[s] + (int64_t)row * n, row + 1};
+    }
+    if (!A.want_vec) return {nullptr, 0};
+    const int v = row - nvb * SL_R;
+    const int nd = dual_rows(A, A.ws.route[s]);
+    if (v < nd) return {A.ws.g_cols + soff * GA + (int64_t)v * n, n};
+    const int64_t st = A.sys.step_off[s] + (v - nd);
+    if (st >= A.sys.step_off[s + 1]) return {nullptr, 0};
+    return {A.ws.w_hat + A.sys.val_off[A.sys.steps[st]], n};
   }
-  if (!A.want_vec) return nullptr;
-  const int v = row - nvb * SL_R;
-  const int nd = dual_rows(A, A.ws.route[s]);
-  if (v < nd) return A.ws.g_cols + soff * GA + (int64_t)v * n;
-  const int64_t st = A.sys.step_off[s] + (v - nd);
-  if (st >= A.sys.step_off[s + 1]) return nullptr;
-  return A.ws.w_hat + A.sys.val_off[A.sys.steps[st]];
+}
+
+// Entries per cell of a system.
+template <int MODE>
+__device__ __forceinline__ int n_entries(const SlArgs& A, int s) {
+  if constexpr (MODE == kRows) return A.rows.m;
+  else return (int)(A.sys.stn_off[s + 1] - A.sys.stn_off[s]);
+}
+// Rows besides the variance's.
+template <int MODE>
+__device__ __forceinline__ int n_vec(const SlArgs& A, int s) {
+  if constexpr (MODE == kRows) return A.rows.m;
+  else
+    return A.want_vec ? dual_rows(A, A.ws.route[s]) +
+                            (int)(A.sys.step_off[s + 1] - A.sys.step_off[s])
+                      : 0;
 }
 
 __device__ __forceinline__ int var_blocks(const SlArgs& A, int n) {
@@ -225,37 +267,36 @@ __device__ __forceinline__ int var_blocks(const SlArgs& A, int n) {
 // A row's exponent: 2^e >= its largest magnitude. A row with a value that is
 // not finite takes its system off this path. Station grid coordinates are
 // filled in on the side.
+template <int MODE>
 __global__ __launch_bounds__(256) void k_sl_rows(SlArgs A) {
   const int i = blockIdx.y, s = A.s0 + i;
   if (!A.rec[s].use) return;
-  const int64_t soff = A.sys.stn_off[s];
-  const int n = (int)(A.sys.stn_off[s + 1] - soff);
-  const int nvb = var_blocks(A, n);
+  const int n = n_entries<MODE>(A, s);
+  const int nvb = MODE == kKrige ? var_blocks(A, n) : 0;
   const int lane = threadIdx.x & 31;
-  const FxGrid g = *A.grid;
-  for (int k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256) {
-    const int st = A.sys.stn_idx[soff + k];
-    A.sg[(int64_t)i * A.sgs + k] = longlong2{fx_coord(A.dom.stn_x[st], g.ox, g.q),
-                                             fx_coord(A.dom.stn_y[st], g.oy, g.q)};
+  if constexpr (MODE == kKrige) {
+    const FxGrid g = *A.grid;
+    for (int k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256) {
+      const int st = A.sys.stn_idx[A.sys.stn_off[s] + k];
+      A.sg[(int64_t)i * A.sgs + k] = longlong2{fx_coord(A.dom.stn_x[st], g.ox, g.q),
+                                               fx_coord(A.dom.stn_y[st], g.oy, g.q)};
+    }
   }
   for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < A.rs; row += gridDim.x * 8) {
-    int len;
-    const double* p = row_ptr(A, s, n, nvb, row, len);
+    const RowRef p = row_ref<MODE>(A, s, n, nvb, row);
     // the largest biased exponent by the high words
     int mx = 0;
-    if (p)
-      for (int j = lane; j < len; j += 32)
-        mx = max(mx, __double2hiint(p[j]) & 0x7fffffff);
+    for (int j = lane; j < p.len; j += 32) mx = max(mx, __double2hiint(p.at(j)) & 0x7fffffff);
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) {
-      int e = (mx >> 20) - 1022;  // |b| < 2^e
+      const int e = (mx >> 20) - 1022;  // |b| < 2^e
       if ((mx >> 20) == 0x7ff) A.rec[s].use = 0;
       A.row_e[(int64_t)i * A.rs + row] = max(e, -900);
     }
   }
 }
 
-// 8 biased entries of one row or cell into 7 digits: byte 6 - i of each, as
+// 8 biased entries of one row or cell into 8 digits: byte 7 - i of each, as
 // FP16 (0x6400 + u is 1024 + u; minus 1152 is u - 128).
 __device__ __forceinline__ void digits8(const uint64_t (&v)[8], uint4 (&o)[SL_D]) {
 #pragma unroll
@@ -281,39 +322,35 @@ __device__ __forceinline__ int var_block_of(int chunk) {
   return b;
 }
 
-// Packed row digits: per (block, 16 stations) 448 rows (digit, row) of 16
+// Packed row digits: per (block, 16 stations) 512 rows (digit, row) of 16
 // FP16 values in the MMA's tile order. Variance block b starts at chunk
 // 2 b (b + 1), its stations ending at its last row.
+template <int MODE>
 __global__ __launch_bounds__(128) void k_sl_pack(SlArgs A) {
   const int i = blockIdx.y, s = A.s0 + i;
   if (!A.rec[s].use) return;
-  const int n = (int)(A.sys.stn_off[s + 1] - A.sys.stn_off[s]);
-  const int k16 = (n + SL_K - 1) / SL_K, nvb = var_blocks(A, n);
+  const int n = n_entries<MODE>(A, s);
+  const int k16 = (n + SL_K - 1) / SL_K, nvb = MODE == kKrige ? var_blocks(A, n) : 0;
   const int nvc = nvb ? 2 * (nvb - 1) * nvb + k16 : 0;
   int c = blockIdx.x, blk, kc;
   if (c < nvc) {
     blk = min(var_block_of(c), nvb - 1);
     kc = c - 2 * blk * (blk + 1);
   } else {
-    if (!A.want_vec) return;
     blk = (c - nvc) / k16;
     kc = (c - nvc) - blk * k16;
-    const int nv = dual_rows(A, A.ws.route[s]) +
-                   (int)(A.sys.step_off[s + 1] - A.sys.step_off[s]);
-    if (blk * SL_R >= nv) return;
+    if (blk * SL_R >= n_vec<MODE>(A, s)) return;
     blk += nvb;
   }
   const int r = threadIdx.x & 63, k8 = threadIdx.x >> 6, row = blk * SL_R + r;
-  int len = 0;
-  const double* p = row_ptr(A, s, n, nvb, row, len);
+  const RowRef p = row_ref<MODE>(A, s, n, nvb, row);
   uint64_t v[8];
   const int e = A.row_e[(int64_t)i * A.rs + row];
   const double sc = ldexp(1.0, FX_BITS - e);
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int k = kc * SL_K + k8 * 8 + q;
-    const double b = (p && k < len) ? p[k] * sc : 0.0;
-    v[q] = (uint64_t)__double2ll_rn(b) + SL_BIAS;
+    v[q] = (uint64_t)__double2ll_rn(p.at(k) * sc) + SL_BIAS;
   }
   uint4 o[SL_D];
   digits8(v, o);
@@ -420,9 +457,7 @@ struct Near {
   unsigned long long best = ~0ull;
   int bj = -1, amb = 0;
   __device__ __forceinline__ void add(FxDist d, int j) {
-    const int z = __clzll((long long)(d.S | 1));
-    const unsigned long long key =
-        d.S ? ((unsigned long long)(200 - 2 * d.L - z) << 55) + ((d.S << z) >> 9) : 0ull;
+    const unsigned long long key = fx_key(d);
     merge(key, j, 0);
   }
   __device__ __forceinline__ void merge(unsigned long long key, int j, int a) {
@@ -488,7 +523,7 @@ __device__ __forceinline__ void sl_gen_any(int code, Args&&... a) {
   }
 }
 
-// 4 biased entries into 7 digits of 4 FP16 values (a byte of each, as
+// 4 biased entries into 8 digits of 4 FP16 values (a byte of each, as
 // digits8).
 __device__ __forceinline__ void digits4(const uint64_t (&v)[4], uint2 (&o)[SL_D]) {
 #pragma unroll
@@ -507,7 +542,33 @@ __device__ __forceinline__ void digits4(const uint64_t (&v)[4], uint2 (&o)[SL_D]
   }
 }
 
-template <typename OutT>
+// Given right-hand sides, scaled by a power of two per point. S.nnb: its
+// exponent, or kNotFinite.
+constexpr int kNotFinite = 0x7fffffff;
+__device__ __forceinline__ void sl_gen_rows(const SlArgs& A, SlSmem& S, int m, int k16,
+                                            int64_t gc, int cell, int part, ulonglong2* slot) {
+  constexpr int PARTS = SL_WT / SL_M;
+  const double* r = A.rows.rhs + gc * m;
+  int mx = 0;
+  for (int j = part; j < m; j += PARTS) mx = max(mx, __double2hiint(r[j]) & 0x7fffffff);
+  int* km = reinterpret_cast<int*>(&S.q[0][0]);
+  km[part * SL_M + cell] = mx;
+  work_sync();
+  for (int q = 0; q < PARTS; ++q) mx = max(mx, km[q * SL_M + cell]);
+  const bool bad = (mx >> 20) == 0x7ff;
+  const int e = max((mx >> 20) - 1022, -900);
+  if (part == 0) S.nnb[cell] = bad ? kNotFinite : e;
+  const double sc = bad ? 0.0 : ldexp(1.0, FX_BITS - e);
+  for (int p = part; p < k16 * (SL_K / 2); p += PARTS) {
+    ulonglong2 v{SL_BIAS, SL_BIAS};
+    const int j = 2 * p;
+    if (j < m && !bad) v.x += (uint64_t)__double2ll_rn(r[j] * sc);
+    if (j + 1 < m && !bad) v.y += (uint64_t)__double2ll_rn(r[j + 1] * sc);
+    slot[(int64_t)p * SL_M + cell] = v;
+  }
+}
+
+template <int MODE, typename OutT>
 __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
   extern __shared__ __align__(1024) unsigned char ring[];
   SlSmem& S = *reinterpret_cast<SlSmem*>(ring + SL_ST * SL_STAGE);
@@ -546,8 +607,8 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = S.tbase;
   const int items = S.nact * tiles;
-  const int64_t C = A.dom.n_cells;
-  const int sk = A.sys.kind == SPI_KIND_SK;
+  const int64_t C = MODE == kRows ? A.rows.points : A.dom.n_cells;
+  const int sk = MODE == kKrige && A.sys.kind == SPI_KIND_SK;
   int g = 0;     // stages of the earlier items (every role counts them alike)
   int nch = 0;   // their chunks (drains)
   bool ok = true;
@@ -555,16 +616,11 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
   for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
     const int li = S.list[item / tiles], s = A.s0 + li;
     const int64_t c0 = (int64_t)(item % tiles) * SL_M;
-    const int64_t soff = A.sys.stn_off[s];
-    const int n = (int)(A.sys.stn_off[s + 1] - soff);
-    const int64_t st0 = A.sys.step_off[s];
-    const int nsteps = (int)(A.sys.step_off[s + 1] - st0);
-    const int route = A.ws.route[s];
-    const int nd = dual_rows(A, route);
+    const int n = n_entries<MODE>(A, s), vecs = n_vec<MODE>(A, s);
     Walk W;
-    W.nvb = var_blocks(A, n);
+    W.nvb = MODE == kKrige ? var_blocks(A, n) : 0;
     W.k16 = (n + SL_K - 1) / SL_K;
-    W.nb = W.nvb + (A.want_vec ? (nd + nsteps + SL_R - 1) / SL_R : 0);
+    W.nb = W.nvb + (vecs + SL_R - 1) / SL_R;
 
     if (warp == SL_W + 1) {
       // ---- copies of the packed rows ----
@@ -609,10 +665,9 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
                       db + (uint64_t)(j * (SL_R / 8) * 8), f16_idesc(SL_R * len), a);
             };
             go(0, 0, 4, acc);
-            go(0, 4, 3, acc);
+            go(0, 4, 4, acc);
             go(1, 0, 4, 1u);
-            go(1, 4, 2, 1u);
-            go(1, 6, 1, acc);
+            go(1, 4, 3, 1u);
             go(2, 0, 3, 1u);
             go(2, 3, 3, 1u);
             go(3, 0, 3, 1u);
@@ -620,6 +675,7 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
             go(4, 0, 4, 1u);
             go(5, 0, 3, 1u);
             go(6, 0, 2, 1u);
+            go(7, 0, 1, 1u);
             tc_commit(smem_u32(&S.empty[st]));
             if (k % SL_KD == SL_KD - 1 || k == ks - 1) {
               tc_commit(smem_u32(&S.chunk));
@@ -640,11 +696,22 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
     ulonglong2* slot = reinterpret_cast<ulonglong2*>(A.slots + (long)blockIdx.x * A.slot_bytes);
     const int cell = tid & (SL_M - 1), part = tid >> 7;
     work_sync();  // the previous item is done with the shared state
-    if (tid == 0) S.any_bad = 0;
-    for (int e = tid; e < (int)(sizeof(FxVg) / 4); e += SL_WT)
-      reinterpret_cast<int*>(&S.vg)[e] = reinterpret_cast<const int*>(&A.rec[s].vg)[e];
-    work_sync();
-    {
+    int64_t soff = 0, st0 = 0;
+    int route = 0, nd = 0, nsteps = 0;
+    if constexpr (MODE == kKrige) {
+      soff = A.sys.stn_off[s];
+      st0 = A.sys.step_off[s];
+      nsteps = (int)(A.sys.step_off[s + 1] - st0);
+      route = A.ws.route[s];
+      nd = dual_rows(A, route);
+      if (tid == 0) S.any_bad = 0;
+      for (int e = tid; e < (int)(sizeof(FxVg) / 4); e += SL_WT)
+        reinterpret_cast<int*>(&S.vg)[e] = reinterpret_cast<const int*>(&A.rec[s].vg)[e];
+      work_sync();
+    }
+    if constexpr (MODE == kRows) {
+      sl_gen_rows(A, S, n, W.k16, min(c0 + cell, C - 1), cell, part, slot);
+    } else {
       const int64_t gc = min(c0 + cell, C - 1);
       const FxGrid gr = *A.grid;
       const int64_t cx = fx_coord(A.dom.cell_x[gc], gr.ox, gr.q);
@@ -681,8 +748,8 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
     const int dcell = (warp & 3) * 32 + lane;  // this thread's cell in a drain
     const int64_t dg = c0 + dcell;
     const int32_t* row_e = A.row_e + (int64_t)li * A.rs + rq * SL_RT;
-    const double sill = S.vg.sill;
-    const int unit = A.rec[s].unit;
+    const double sill = MODE == kKrige ? S.vg.sill : 1.0;
+    const int unit = MODE == kKrige ? A.rec[s].unit : 0;
     // a row's sum, acc_h 2^32 + acc_l (units of level 7)
     long long acc_h[SL_RT];
     uint32_t acc_l[SL_RT];
@@ -781,6 +848,26 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
       if (work_or(!ok)) {
         ok = false;
         break;
+      }
+      if constexpr (MODE == kRows) {
+        // (b + row) 0 .. of this thread's point
+        const int row0 = b * SL_R + rq * SL_RT;
+        const int ec = S.nnb[dcell];
+        if (dg < C) {
+          double* lam = A.rows.lambdas + dg * A.rows.n + row0;
+#pragma unroll
+          for (int q = 0; q < SL_RT; ++q) {
+            const int row = row0 + q;
+            const double y =
+                ec == kNotFinite
+                    ? __longlong_as_double(0x7ff8000000000000LL)
+                    : scalbn(fma((double)acc_h[q], 4294967296.0, (double)acc_l[q]),
+                             ec + row_e[b * SL_R + q] - 68);
+            if (row < A.rows.n) lam[q] = y;
+            else if (row < n) A.rows.mus[(int64_t)(row - A.rows.n) * C + dg] = y;
+          }
+        }
+        continue;
       }
       if (b < W.nvb) {
         // squares of y / sill in units of 2^unit
@@ -1012,20 +1099,85 @@ int launch_slices(const SlicesCall& c, const int32_t** use, int* use_stride, cud
     return SPI_ERR_CUDA;
   k_sl_range<<<2 * sms, 256, 0, st>>>(c.dom, A.head);
   SPI_LAUNCH_CHECK();
-  auto kern = c.out.out_f64 ? k_sl_gemm<double> : k_sl_gemm<float>;
+  auto kern = c.out.out_f64 ? k_sl_gemm<kKrige, double> : k_sl_gemm<kKrige, float>;
   if (!smem_opt_in(kern, SL_SMEM)) return SPI_ERR_CUDA;
   for (int s0 = 0; s0 < c.sys.n_sys; s0 += grp) {
     A.s0 = s0;
     A.ns = c.sys.n_sys - s0 < grp ? c.sys.n_sys - s0 : grp;
     k_sl_select<<<(A.ns + 255) / 256, 256, 0, st>>>(A);
-    k_sl_rows<<<dim3((p.rs + 31) / 32, A.ns), 256, 0, st>>>(A);
-    k_sl_pack<<<dim3((unsigned)p.pc, A.ns), 128, 0, st>>>(A);
+    k_sl_rows<kKrige><<<dim3((p.rs + 31) / 32, A.ns), 256, 0, st>>>(A);
+    k_sl_pack<kKrige><<<dim3((unsigned)p.pc, A.ns), 128, 0, st>>>(A);
     SPI_LAUNCH_CHECK();
     const int64_t items = tiles * A.ns;
     kern<<<(unsigned)(items < sms ? items : sms), SL_T, SL_SMEM, st>>>(A, (int)tiles);
     SPI_LAUNCH_CHECK();
   }
   return SPI_OK;
+}
+
+namespace {
+
+// One "system" of n entries and `rows` rows, its parts laid out in the
+// scratch.
+int one_layout(SlArgs& A, SlPlan& p, int n, void* scratch, int64_t scratch_bytes, int sms) {
+  unsigned char* q = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(scratch) + 255) / 256 * 256);
+  if (q + p.fixed + p.per_sys > static_cast<unsigned char*>(scratch) + scratch_bytes)
+    return SPI_ERR_WORKSPACE;
+  A.s0 = 0;
+  A.ns = 1;
+  A.rs = p.rs;
+  A.pc = p.pc;
+  A.sgs = p.sgs;
+  A.slot_bytes = (long)p.slot;
+  A.head = reinterpret_cast<SlHead*>(q);
+  q += al(sizeof(SlHead));
+  A.grid = reinterpret_cast<FxGrid*>(q);
+  q += al(sizeof(FxGrid));
+  A.rec = reinterpret_cast<SlSys*>(q);
+  q += al(sizeof(SlSys));
+  A.slots = q;
+  q += p.slot * sms;
+  A.sg = reinterpret_cast<longlong2*>(q);
+  q += al((size_t)p.sgs * sizeof(longlong2));
+  A.row_e = reinterpret_cast<int32_t*>(q);
+  q += al((size_t)p.rs * 4);
+  A.pack = q;
+  return SPI_OK;
+}
+
+template <int MODE, typename K>
+int one_launch(SlArgs& A, const SlPlan& p, K kern, int64_t points, int sms, cudaStream_t st) {
+  const int64_t tiles = (points + SL_M - 1) / SL_M;
+  if (tiles > 0x7fffffff) return SPI_ERR_TOO_LARGE;
+  if (!smem_opt_in(kern, SL_SMEM)) return SPI_ERR_CUDA;
+  k_sl_rows<MODE><<<dim3((p.rs + 31) / 32, 1), 256, 0, st>>>(A);
+  k_sl_pack<MODE><<<dim3((unsigned)p.pc, 1), 128, 0, st>>>(A);
+  kern<<<(unsigned)(tiles < sms ? tiles : sms), SL_T, SL_SMEM, st>>>(A, (int)tiles);
+  SPI_LAUNCH_CHECK();
+  return SPI_OK;
+}
+
+}  // namespace
+
+int64_t slices_scratch_one(int n, int rows) {
+  const int sms = n_sms();
+  const SlPlan p(n, 1, rows, false, true, sms > 0 ? sms : 160);
+  return (int64_t)(p.fixed + p.per_sys + 256);
+}
+
+int launch_slices_rows(const SlRows& r, void* scratch, int64_t scratch_bytes, int32_t* err,
+                       const int32_t** use, cudaStream_t st) {
+  const int sms = n_sms();
+  if (sms <= 0) return SPI_ERR_CUDA;
+  SlPlan p(r.m, 1, r.m, false, true, sms);
+  SlArgs A = {};
+  if (int rc = one_layout(A, p, r.m, scratch, scratch_bytes, sms)) return rc;
+  A.err = err;
+  A.rows = r;
+  *use = &A.rec[0].use;
+  k_sl_select_one<<<1, 1, 0, st>>>(A);
+  return one_launch<kRows>(A, p, k_sl_gemm<kRows, double>, r.points, sms, st);
 }
 
 }  // namespace spi

@@ -12,6 +12,17 @@ struct No {
   static constexpr bool value = false;
 };
 
+// Right-hand sides rhs [points, m] against the rows of inv [m, m]: the first
+// n results to lambdas [points, n], the rest to mus [m - n, points].
+struct SlRows {
+  const double* rhs;
+  const double* inv;
+  int m, n;
+  int64_t points;
+  double* lambdas;
+  double* mus;
+};
+
 struct SlicesCall {
   spi_domain_t dom;
   spi_systems_t sys;
@@ -31,6 +42,12 @@ int64_t slices_scratch(int max_n, int n_sys, int max_vec, bool var, bool vec);
 
 // Runs the systems that have a sliced form; (*use)[s * *stride] != 0 (on the
 // device, in stream order) marks them, the caller computes the others.
+// The other contraction: *use != 0 (on the device) where it ran, else the
+// caller computes it.
+int64_t slices_scratch_one(int n, int rows);
+int launch_slices_rows(const SlRows& r, void* scratch, int64_t scratch_bytes, int32_t* err,
+                       const int32_t** use, cudaStream_t st);
+
 int launch_slices(const SlicesCall& c, const int32_t** use, int* stride, cudaStream_t st);
 
 }  // namespace spi

@@ -58,6 +58,10 @@ _CODES = {b"Rng": 0, b"Nug": 1, b"Sph": 2, b"Exp": 3, b"Lin": 4, b"Gau": 5, b"Po
 # ||A||_F ||A^-1||_F bound under which numpy.linalg.pinv (rcond 1e-15)
 # drops no singular value: the Gauss-Jordan inverse is its matrix
 PINV_COND = 1e15
+# from here on the points' weights are sliced tensor-core products
+# (spi_legacy_points_sliced)
+SLICES_MIN_M = 64
+SLICES_MIN_POINTS = 512
 
 
 def parse_model(model):
@@ -154,9 +158,16 @@ def krige_points(kind, xi, yi, zi, xk, yk, model, si=None, sk=None, ixi=None, wa
     zk = torch.empty(n_out, **f64)
     est = torch.empty(n_out, **f64) if (want_est and kind != "EDK") or ixi is not None else None
     ik = torch.empty(n_out, **f64) if ixi is not None else None
-    nat.call("spi_legacy_points", code, _ptr(xi), _ptr(yi), _ptr(zi), _ptr(ixi), n, _ptr(xk),
-             _ptr(yk), _ptr(sk), n_out, n_drift, ctypes.byref(vg), _ptr(inv), _ptr(rhss),
-             _ptr(lambdas), _ptr(mus), _ptr(zk), _ptr(est), _ptr(ik), st)
+    args = (code, _ptr(xi), _ptr(yi), _ptr(zi), _ptr(ixi), n, _ptr(xk), _ptr(yk), _ptr(sk),
+            n_out, n_drift, ctypes.byref(vg), _ptr(inv), _ptr(rhss), _ptr(lambdas), _ptr(mus),
+            _ptr(zk), _ptr(est), _ptr(ik))
+    if m >= SLICES_MIN_M and n_out >= SLICES_MIN_POINTS:
+        scratch = torch.empty(nat.lib().spi_slices_one_scratch_bytes(m, m), dtype=torch.uint8,
+                              device=dev)
+        err = torch.zeros(1, dtype=torch.int32, device=dev)
+        nat.call("spi_legacy_points_sliced", *args, _ptr(scratch), scratch.numel(), _ptr(err), st)
+    else:
+        nat.call("spi_legacy_points", *args, st)
     return dict(in_dists=in_dists, lhs=lhs, lhs_inv=inv, rhss=rhss, lambdas=lambdas, mus=mus,
                 zk=zk, est=est, ik=ik, route=route)
 

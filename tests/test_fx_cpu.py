@@ -1,12 +1,12 @@
 """The fixed-point covariance entries (csrc/spi_fx.cuh) on the CPU: the same
 functions compiled for the host, against decimal arithmetic of 50 digits.
 
-An entry's unit is 2^-54 of the structures' sills. Its error bound, in units:
-the grid's 2^-61 of the extent on each coordinate (at most 3 sqrt(2) / 50 of
-it per range used here: under 1), the distance's and its root's 2^-59
+An entry's unit is 2^-62 of the structures' sills. Its error bound, in units of
+2^-54: the grid's 2^-61 of the extent on each coordinate (3 sqrt(2) e^4 e^-1 of
+it for the shortest range used here: 0.7), the distance's and its root's 2^-59
 relative (3 e^-1 of that: 0.04), the products' 2 units of 2^-61 relative, the
-exponential's 2^-60, each structure's weight rounding (1 unit), the final
-rounding (0.5): 8 units hold with room.
+exponential's 2^-60, each structure's weight rounding (2^-62): 2 hold with
+room.
 """
 import random
 import shutil
@@ -70,13 +70,15 @@ def fx(tmp_path_factory):
 
 
 def _exact(vg, x):
-    """(sum s rho, sum of the structures' s) in decimals."""
+    """sum s rho in decimals, and the unit's sum of the structures' s (in
+    doubles, as the device forms it)."""
     dx, dy = Decimal(x[0]) - Decimal(x[2]), Decimal(x[1]) - Decimal(x[3])
     h = (dx * dx + dy * dy).sqrt()
-    c = tot = Decimal(0)
+    c, tot = Decimal(0), 0.0
     for name, s, r in vg:
         if name == "Nug":
             continue
+        tot += s
         s, r = Decimal(s), Decimal(r)
         t = h / r
         if name == "Exp":
@@ -88,8 +90,7 @@ def _exact(vg, x):
         else:
             rho = 1 - t if t < 1 else Decimal(0)
         c += s * rho
-        tot += s
-    return c, tot
+    return c, Decimal(tot)
 
 
 def _cases(rng, names, count):
@@ -120,7 +121,7 @@ def test_entries_against_decimals(fx, names):
     for c, (ok, v, cut, over) in zip(cases, fx(cases)):
         assert ok == 1 and cut == -1
         want, tot = _exact(c["vg"], c["x"])
-        assert abs(v * unit - want / tot) <= 8 * unit, c
+        assert abs(v * unit / 256 - want / tot) <= 2 * unit, c
 
 
 def test_min_vg_cut(fx):
@@ -128,13 +129,13 @@ def test_min_vg_cut(fx):
     kinds; a cut that no entry reaches, or that every entry passes."""
     base = dict(q=40, o=(0.0, 0.0), x=(1e3, 2e3, 1.5e3, 2.5e3))
     exp = [("Exp", 0.9, 2e4)]
-    one = 1 << 54
+    one = 1 << 62
     got = fx([dict(base, vg=exp, sk=0, mv=1e-4), dict(base, vg=exp, sk=1, mv=1e-4),
               dict(base, vg=[("Nug", 0.1, 0.0), *exp], sk=0, mv=1e-4),
               dict(base, vg=[("Nug", 5e-5, 0.0), *exp], sk=0, mv=1e-4),
               dict(base, vg=exp, sk=0, mv=2.0), dict(base, vg=exp, sk=1, mv=2.0)])
     assert [g[0] for g in got] == [1, 1, 1, 1, 0, 0]
-    assert abs(got[0][2] - round(one * (0.9 - 1e-4) / 0.9)) <= 64 and got[0][3] == one
-    assert abs(got[1][2] - round(one * 1e-4 / 0.9)) <= 64 and got[1][3] == 0
+    assert abs(got[0][2] - round(one * (0.9 - 1e-4) / 0.9)) <= 1 << 14 and got[0][3] == one
+    assert abs(got[1][2] - round(one * 1e-4 / 0.9)) <= 1 << 14 and got[1][3] == 0
     assert got[2][2] == -1  # the nugget alone exceeds the cut
-    assert abs(got[3][3] - round(one * 0.90005 / 0.9)) <= 64
+    assert abs(got[3][3] - round(one * 0.90005 / 0.9)) <= 1 << 14

@@ -85,3 +85,27 @@ def test_cut(min_vg):
 def test_double_float_tier():
     """Mixed precision: ill-conditioned systems take the sliced variance."""
     _run(150, 3, 300, ["OK"], ["0.00001 Exp(1.0) + 0.9 Gau(25000)"], 95, precision="mixed")
+
+
+@pytest.mark.parametrize("kind", ["OK", "SK", "EDK"])
+@pytest.mark.parametrize("n,C", [(63, 600), (64, 513), (95, 640), (96, 700), (127, 515), (200, 900)])
+def test_single_neighbourhood(kind, n, C):
+    """The classes' weights as sliced products and their matrix inverted step
+    by step over the GPU, against the oracle's restatement of the classes:
+    1e-9 of each array's largest value (condition up to 1e5)."""
+    import torch
+    from spinterps_gb300 import legacy
+    rng = np.random.default_rng(n)
+    xi, yi, zi = rng.uniform(0, 1e5, n), rng.uniform(0, 1e5, n), rng.gamma(1.2, 3.0, n)
+    xk, yk = rng.uniform(0, 1e5, C), rng.uniform(0, 1e5, C)
+    xk[0], yk[0] = xi[2], yi[2]
+    si = rng.uniform(0, 2, (2, n)) if kind == "EDK" else None
+    sk = rng.uniform(0, 2, (2, C)) if kind == "EDK" else None
+    model = "0.1 Nug(0.0) + 0.9 Exp(30000)"
+    d = lambda a: None if a is None else torch.as_tensor(a, device="cuda")  # noqa: E731
+    got = legacy.krige_points(kind, d(xi), d(yi), d(zi), d(xk), d(yk), model, si=d(si), sk=d(sk))
+    cls = {"OK": "OrdinaryKriging", "SK": "SimpleKriging", "EDK": "ExternalDriftKriging_MD"}[kind]
+    ref = port.legacy_krige(cls, xi, yi, zi, xk, yk, model, si=si, sk=sk)
+    for k in ("zk", "lambdas", "rhss", "in_dists"):
+        a, b = got[k].cpu().numpy(), ref[k]
+        assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max(), k
