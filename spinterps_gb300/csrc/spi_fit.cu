@@ -12,15 +12,19 @@
 //     495-520), summed in numpy's pairwise order so that the bins agree with
 //     the reference to the last bits;
 //   - the differential-evolution fits of every model permutation
-//     (vgs.py:680-764): one CTA per (step, permutation), population
+//     (vgs.py:680-764): one cluster per (step, permutation), population
 //     50 * D^2 in [0,1]^D as scipy scales it, best/1/bin with a dithered
 //     F in [0.5, 1) and CR 0.7, out-of-range components redrawn, stopping
 //     when the population energies' std <= tol * |mean| (scipy's rule).
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "spi_common.cuh"
 
 namespace spi {
+
+namespace cg = cooperative_groups;
 
 // x^4 rounded once, as the correctly rounded pow of the host libm that the
 // reference's ``** 4`` calls: x^2 = p + e and p^2 = hi + lo are exact
@@ -500,9 +504,11 @@ __global__ __launch_bounds__(RF_T) void k_vg_refine(int n_prob, const spi_de_pro
   }
 }
 
-constexpr int DE_T = 256;
+constexpr int DE_T = 256;        // threads of a CTA, and lanes of the sums' trees
 constexpr int DE_MAXNP = 800;    // 50 * 4^2
-constexpr int DE_MAXBINS = 16384;   // bins kept in shared memory (more: read from L2)
+constexpr int DE_CL = 4;         // CTAs of one problem with two structures
+constexpr int DE_MEM = DE_MAXNP / DE_CL;   // members of a CTA, one thread each
+constexpr int DE_BINS = 2048;    // bins in shared memory at a time
 
 struct DeArgs {
   int32_t n_prob;
@@ -517,12 +523,143 @@ struct DeArgs {
   int32_t* n_gen;
 };
 
-__global__ __launch_bounds__(DE_T) void k_de(DeArgs A) {
-  const int q = blockIdx.x;
+// Bins of one member's energy, in their order, by a compensated sum.
+struct DeSum {
+  float acc = 0.f, cmp = 0.f;
+  __device__ __forceinline__ void add(float d) {
+    const float y = d * d - cmp;
+    const float t = acc + y;
+    cmp = (t - acc) - y;
+    acc = t;
+  }
+};
+
+// h / r rounded to nearest from y = 1/r rounded to nearest (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): one step makes the quotient faithful, the next one
+// exact. For r and h (or h = 0) in [2^-40, 2^60]: nothing under- or
+// overflows. r is the same for all bins of a member, so this costs 5
+// instructions instead of a division with its test for special values.
+__device__ __forceinline__ float div_by(float h, float r, float y) {
+  float q = __fmul_rn(h, y);
+  q = fmaf(fmaf(-q, r, h), y, q);
+  return fmaf(fmaf(-q, r, h), y, q);
+}
+__device__ __forceinline__ bool div_by_ok(float v) { return v >= 0x1p-40f && v <= 0x1p60f; }
+
+// fit_model with the structure known at compile time, same roundings
+template <int CODE>
+__device__ __forceinline__ float fit_model_c(float h, float r, float y, float s) {
+  if (CODE == SPI_VG_NUG) return s;
+  const float t = div_by(h, r, y);
+  if (CODE == SPI_VG_SPH) {
+    const float v = s * (1.5f * t - 0.5f * t * t * t);
+    return h > r ? s : v;
+  }
+  if (CODE == SPI_VG_EXP) return s * (1.0f - expf(-3.0f * t));
+  if (CODE == SPI_VG_LIN) return h > r ? s : s * t;
+  return s * (1.0f - expf(-3.0f * t * t));   // SPI_VG_GAU
+}
+// One structure, or a nugget (s0) before it. The sums with the model are
+// kept out of fused multiply-adds, as they are behind fit_model's switch.
+template <int CODE, bool NUG>
+__device__ __forceinline__ void de_bins(const float2* __restrict__ hg, int n, float s0, float r,
+                                        float s, DeSum& sum) {
+  const float y = CODE == SPI_VG_NUG ? 0.f : __frcp_rn(r);
+#pragma unroll 4
+  for (int b = 0; b < n; ++b) {
+    const float2 v = hg[b];
+    const float m = fit_model_c<CODE>(v.x, r, y, s);
+    sum.add(__fsub_rn(v.y, NUG ? __fadd_rn(s0, m) : m));
+  }
+}
+template <bool NUG>
+__device__ __forceinline__ bool de_bins_code(int code, const float2* hg, int n, float s0, float r,
+                                             float s, DeSum& sum) {
+  switch (code) {
+    case SPI_VG_NUG: de_bins<SPI_VG_NUG, NUG>(hg, n, s0, r, s, sum); return true;
+    case SPI_VG_SPH: de_bins<SPI_VG_SPH, NUG>(hg, n, s0, r, s, sum); return true;
+    case SPI_VG_EXP: de_bins<SPI_VG_EXP, NUG>(hg, n, s0, r, s, sum); return true;
+    case SPI_VG_LIN: de_bins<SPI_VG_LIN, NUG>(hg, n, s0, r, s, sum); return true;
+    case SPI_VG_GAU: de_bins<SPI_VG_GAU, NUG>(hg, n, s0, r, s, sum); return true;
+  }
+  return false;
+}
+
+// sum of v over the CTA's DE_T lanes: lane t takes lane t + o for o = 128,
+// 64, .., 1
+__device__ __forceinline__ double de_tree_sum(double v, double* red) {
+  const int t = threadIdx.x;
+  red[t] = v;
+  __syncthreads();
+  double a = 0.0;
+  if (t < 32) {
+    a = ((red[t] + red[t + 128]) + (red[t + 64] + red[t + 192])) +
+        ((red[t + 32] + red[t + 160]) + (red[t + 96] + red[t + 224]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+  }
+  __syncthreads();
+  if (t == 0) red[0] = a;
+  __syncthreads();
+  a = red[0];
+  __syncthreads();
+  return a;
+}
+// the first member of the least energy (0 where every energy is NaN)
+__device__ __forceinline__ int de_best(const float* E, int NP, float* redf, int* redi) {
+  const int t = threadIdx.x, w = t >> 5;
+  float bv = __int_as_float(0x7f800000);
+  int bi = 0x7fffffff;
+  for (int i = t; i < NP; i += DE_T)
+    if (E[i] < bv || (E[i] == bv && i < bi)) { bv = E[i]; bi = i; }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (ov < bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+  }
+  if ((t & 31) == 0) { redf[w] = bv; redi[w] = bi; }
+  __syncthreads();
+  bv = redf[0];
+  bi = redi[0];
+  for (int k = 1; k < DE_T / 32; ++k)
+    if (redf[k] < bv || (redf[k] == bv && redi[k] < bi)) { bv = redf[k]; bi = redi[k]; }
+  __syncthreads();
+  return bi < NP ? bi : 0;
+}
+
+struct DeSmem {
+  double pop[DE_MAXNP * 4];      // [NP][4] unit cube
+  double red[DE_T];
+  double lo[4], sc[4];
+  float E[DE_MAXNP];
+  union {
+    float2 hg[DE_BINS];
+    int16_t perm[2][4][DE_MAXNP];   // the start's strata
+  };
+  float redf[DE_T / 32];
+  int redi[DE_T / 32];
+};
+
+// One cluster per problem, one thread per member: a problem with two
+// structures (800 members) takes 4 CTAs, one with a single structure (200)
+// the first of them, the others leave. Every CTA holds the population and
+// its energies; a generation's accepted trials go to all copies, between
+// two cluster barriers, and each CTA takes the best member and the stop from
+// its own copy, in the same order of sums.
+//
+// Bound by the energies' instructions: bins x members x generations, each a
+// dependent chain (compensated sum) per member. One CTA per problem with
+// four members to a thread left most of the chip idle behind the problems
+// with two structures, at two warps to a scheduler: 32.9 ms before, 2.15 ms
+// now for 30 steps of 300 stations (150 problems, about 450 bins each).
+__global__ __launch_bounds__(DE_T) __cluster_dims__(DE_CL, 1, 1) void k_de(DeArgs A) {
+  const int q = blockIdx.x / DE_CL, rank = blockIdx.x % DE_CL;
   const spi_de_problem_t P = A.prob[q];
   if (P.n_comp < 1 || P.n_comp > 2 || A.n_bins[P.step] < 1) {
     // unsupported problem size or no bins: no fit
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && rank == 0) {
       for (int j = 0; j < 4; ++j) A.best_x[(int64_t)q * 4 + j] = __longlong_as_double(0x7ff8000000000000LL);
       A.best_f[q] = __longlong_as_double(0x7ff8000000000000LL);
       A.n_gen[q] = 0;
@@ -531,27 +668,16 @@ __global__ __launch_bounds__(DE_T) void k_de(DeArgs A) {
   }
   const int D = 2 * P.n_comp;
   const int NP = 50 * D * D;
+  const bool split = NP > DE_MEM;
+  if (!split && rank > 0) return;
   const int tid = threadIdx.x;
   extern __shared__ __align__(16) unsigned char sm[];
-  double* pop = reinterpret_cast<double*>(sm);           // [NP][4] unit cube
-  double* tri = pop + DE_MAXNP * 4;                       // [NP][4]
-  double* E = tri + DE_MAXNP * 4;                          // [NP]
-  double* Et = E + DE_MAXNP;                               // [NP]
-  float* hb = reinterpret_cast<float*>(Et + DE_MAXNP);     // [nb]
-  float* gb = hb + DE_MAXBINS;                             // [nb]
-  __shared__ double lo[4], sc[4];
-  __shared__ double red[DE_T];
-  __shared__ int redi[DE_T];
-  __shared__ int best, stop;
-  __shared__ double Fsh;
+  DeSmem& S = *reinterpret_cast<DeSmem*>(sm);
   const int64_t bo = A.bin_off[P.step];
   const int nb = A.n_bins[P.step];
-  const bool bins_in_smem = nb <= DE_MAXBINS;
-  if (bins_in_smem)
-    for (int b = tid; b < nb; b += DE_T) {
-      hb[b] = (float)A.bin_h[bo + b];
-      gb[b] = (float)A.bin_g[bo + b];
-    }
+  cg::cluster_group cl = cg::this_cluster();
+  const int mi = rank * DE_MEM + tid;           // this thread's member
+  const bool member = tid < DE_MEM && mi < NP;
   if (tid == 0) {
     // bounds of vgs.py:731-753
     const double h0 = A.bin_h[bo], g0 = A.bin_g[bo];
@@ -564,87 +690,114 @@ __global__ __launch_bounds__(DE_T) void k_de(DeArgs A) {
       } else {
         rl = h0; rh = 1e9; sl = 1e-5; shh = P.var2;
       }
-      lo[2 * k] = rl; sc[2 * k] = rh - rl;
-      lo[2 * k + 1] = sl; sc[2 * k + 1] = shh - sl;
+      S.lo[2 * k] = rl; S.sc[2 * k] = rh - rl;
+      S.lo[2 * k + 1] = sl; S.sc[2 * k + 1] = shh - sl;
     }
-    stop = 0;
   }
+  // initial population: Latin hypercube, or the warm-start box. Stratum i of
+  // dimension j goes to member perm(i) (Fisher-Yates): the draws by all
+  // threads, the swaps by one thread of each dimension.
+  for (int k = tid; k < NP * D; k += DE_T) {
+    const int j = k / NP, i = k - j * NP;
+    S.perm[0][j][i] = (int16_t)i;
+    S.perm[1][j][i] = (int16_t)(int)(urand(P.seed, 0, j, i) * (i + 1));
+  }
+  for (int k = tid; k < NP * 4; k += DE_T) S.pop[k] = 0.0;
   __syncthreads();
-  auto energy = [&](const double* u) -> float {
-    float r[2], s[2];
-    for (int k = 0; k < P.n_comp; ++k) {
-      r[k] = (float)(lo[2 * k] + u[2 * k] * sc[2 * k]);
-      s[k] = (float)(lo[2 * k + 1] + u[2 * k + 1] * sc[2 * k + 1]);
-    }
-    float acc = 0.f, cmp = 0.f;
-    for (int b = 0; b < nb; ++b) {
-      const float hv = bins_in_smem ? hb[b] : (float)A.bin_h[bo + b];
-      const float gv = bins_in_smem ? gb[b] : (float)A.bin_g[bo + b];
-      float m = 0.f;
-      for (int k = 0; k < P.n_comp; ++k) m += fit_model(P.code[k], hv, r[k], s[k]);
-      float d = gv - m;
-      // compensated sum
-      float y = d * d - cmp;
-      float t = acc + y;
-      cmp = (t - acc) - y;
-      acc = t;
-    }
-    return acc;
-  };
-  // initial population: Latin hypercube, or the warm-start box
-  for (int i = tid; i < NP; i += DE_T)
-    for (int j = 0; j < 4; ++j) pop[i * 4 + j] = 0.0;
-  __syncthreads();
-  if (tid < D) {
-    const int j = tid;
-    // stratum i of dimension j goes to member perm(i): Fisher-Yates
-    int* perm = reinterpret_cast<int*>(tri) + j * DE_MAXNP;  // scratch
-    for (int i = 0; i < NP; ++i) perm[i] = i;
+  if ((tid & 31) == 0 && tid / 32 < D) {
+    int16_t* perm = S.perm[0][tid / 32];
+    const int16_t* draw = S.perm[1][tid / 32];
     for (int i = NP - 1; i > 0; --i) {
-      int k = (int)(urand(P.seed, 0, j, i) * (i + 1));
-      int t = perm[i];
+      const int k = draw[i];
+      const int16_t t = perm[i];
       perm[i] = perm[k];
       perm[k] = t;
     }
+  }
+  __syncthreads();
+  for (int k = tid; k < NP * D; k += DE_T) {
+    const int j = k / NP, i = k - j * NP;
     double wl = 0.0, ww = 1.0;
     if (P.warm) {
       wl = P.warm_lo[j];
       ww = P.warm_hi[j] - P.warm_lo[j];
     }
-    for (int i = 0; i < NP; ++i) {
-      double u = (i + urand(P.seed, 1, j, i)) / NP;
-      pop[perm[i] * 4 + j] = wl + u * ww;
-    }
+    double u = (i + urand(P.seed, 1, j, i)) / NP;
+    S.pop[S.perm[0][j][i] * 4 + j] = wl + u * ww;
   }
   __syncthreads();
-  for (int i = tid; i < NP; i += DE_T) E[i] = energy(pop + i * 4);
-  __syncthreads();
+  bool plain = true;    // every distance allows div_by
+  auto load_bins = [&](int b0) {
+    const int n = min(DE_BINS, nb - b0);
+    bool ok = true;
+    for (int b = tid; b < n; b += DE_T) {
+      const float h = (float)A.bin_h[bo + b0 + b];
+      S.hg[b] = make_float2(h, (float)A.bin_g[bo + b0 + b]);
+      ok = ok && (h == 0.f || div_by_ok(h));
+    }
+    plain = __syncthreads_and(ok) != 0;
+    return n;
+  };
+  if (nb <= DE_BINS) load_bins(0);
+  // all threads of the CTA come here together
+  auto energy = [&](const double* u) -> float {
+    float r[2] = {0.f, 0.f}, s[2] = {0.f, 0.f};
+    for (int k = 0; k < P.n_comp; ++k) {
+      r[k] = (float)(S.lo[2 * k] + u[2 * k] * S.sc[2 * k]);
+      s[k] = (float)(S.lo[2 * k + 1] + u[2 * k + 1] * S.sc[2 * k + 1]);
+    }
+    const bool nug = P.n_comp == 2 && P.code[0] == SPI_VG_NUG;
+    const int last = P.n_comp - 1;
+    DeSum sum;
+    for (int b0 = 0; b0 < nb; b0 += DE_BINS) {
+      int n = nb;
+      if (nb > DE_BINS) {
+        __syncthreads();
+        n = load_bins(b0);
+      }
+      if (!member) continue;
+      // the range of a nugget is not used, that of a power model no divisor
+      const bool fast = plain && (P.n_comp == 1 || nug) &&
+                        __all_sync(__activemask(), div_by_ok(r[last]));
+      if (fast && (nug ? de_bins_code<true>(P.code[last], S.hg, n, s[0], r[last], s[last], sum)
+                       : de_bins_code<false>(P.code[last], S.hg, n, 0.f, r[last], s[last], sum)))
+        continue;
+      for (int b = 0; b < n; ++b) {
+        float m = 0.f;
+        for (int k = 0; k < P.n_comp; ++k) m += fit_model(P.code[k], S.hg[b].x, r[k], s[k]);
+        sum.add(S.hg[b].y - m);
+      }
+    }
+    return sum.acc;
+  };
+  // this thread's member and its energy into every copy
+  auto put = [&](const double* x, float e) {
+    for (int c = 0; c < (split ? DE_CL : 1); ++c) {
+      DeSmem* R = split ? cl.map_shared_rank(&S, c) : &S;
+      for (int j = 0; j < D; ++j) R->pop[mi * 4 + j] = x[j];
+      R->E[mi] = e;
+    }
+  };
+  auto sync_all = [&]() {
+    if (split)
+      cl.sync();
+    else
+      __syncthreads();
+  };
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  if (member)
+    for (int j = 0; j < 4; ++j) v[j] = S.pop[mi * 4 + j];
+  float e = energy(v);
+  sync_all();
+  if (member) put(v, e);
+  sync_all();
   int gen = 0;
   for (gen = 1; gen <= A.maxiter; ++gen) {
-    // best member (first of the minimum energy)
-    double bv = __longlong_as_double(0x7ff0000000000000LL);
-    int bi = 0x7fffffff;
-    for (int i = tid; i < NP; i += DE_T)
-      if (E[i] < bv || (E[i] == bv && i < bi)) { bv = E[i]; bi = i; }
-    red[tid] = bv;
-    redi[tid] = bi;
-    __syncthreads();
-    for (int o = DE_T / 2; o > 0; o >>= 1) {
-      if (tid < o && (red[tid + o] < red[tid] ||
-                      (red[tid + o] == red[tid] && redi[tid + o] < redi[tid]))) {
-        red[tid] = red[tid + o];
-        redi[tid] = redi[tid + o];
-      }
-      __syncthreads();
-    }
-    if (tid == 0) {
-      best = redi[0];
-      Fsh = 0.5 + 0.5 * urand(P.seed, 2, gen, 0);
-    }
-    __syncthreads();
-    const double F = Fsh;
-    const double* pb = pop + best * 4;
-    for (int i = tid; i < NP; i += DE_T) {
+    const int best = de_best(S.E, NP, S.redf, S.redi);
+    const double F = 0.5 + 0.5 * urand(P.seed, 2, gen, 0);
+    const double* pb = S.pop + best * 4;
+    if (member) {
+      const int i = mi;
       // two distinct members other than i (bounded redraws)
       int r1 = (int)(urand(P.seed, 3, gen, (uint64_t)i * 64) * NP);
       for (int c = 1; c < 32 && r1 == i; ++c) r1 = (int)(urand(P.seed, 3, gen, (uint64_t)i * 64 + c) * NP);
@@ -654,83 +807,45 @@ __global__ __launch_bounds__(DE_T) void k_de(DeArgs A) {
         r2 = (int)(urand(P.seed, 7, gen, (uint64_t)i * 64 + c) * NP);
       if (r2 == i || r2 == r1) r2 = (max(i, r1) + 1) % NP == min(i, r1) ? (max(i, r1) + 2) % NP : (max(i, r1) + 1) % NP;
       const int jr = (int)(urand(P.seed, 4, gen, i) * D);
+#pragma unroll
       for (int j = 0; j < 4; ++j) {
-        double v = pop[i * 4 + j];
+        v[j] = S.pop[i * 4 + j];
         if (j < D && (urand(P.seed, 5, gen, (uint64_t)i * 4 + j) < 0.7 || j == jr)) {
-          v = pb[j] + F * (pop[r1 * 4 + j] - pop[r2 * 4 + j]);
-          if (v < 0.0 || v > 1.0) v = urand(P.seed, 6, gen, (uint64_t)i * 4 + j);
+          v[j] = pb[j] + F * (S.pop[r1 * 4 + j] - S.pop[r2 * 4 + j]);
+          if (v[j] < 0.0 || v[j] > 1.0) v[j] = urand(P.seed, 6, gen, (uint64_t)i * 4 + j);
         }
-        tri[i * 4 + j] = v;
       }
-      Et[i] = energy(tri + i * 4);
     }
-    __syncthreads();
-    for (int i = tid; i < NP; i += DE_T)
-      if (Et[i] <= E[i]) {
-        E[i] = Et[i];
-        for (int j = 0; j < 4; ++j) pop[i * 4 + j] = tri[i * 4 + j];
-      }
-    __syncthreads();
+    e = energy(v);
+    sync_all();
+    if (member && e <= S.E[mi]) put(v, e);
+    sync_all();
     // convergence: std(E) <= tol * |mean(E)|
     double s1 = 0.0;
-    for (int i = tid; i < NP; i += DE_T) s1 += E[i];
-    red[tid] = s1;
-    __syncthreads();
-    for (int o = DE_T / 2; o > 0; o >>= 1) {
-      if (tid < o) red[tid] += red[tid + o];
-      __syncthreads();
-    }
-    const double mean = red[0] / NP;
-    __syncthreads();
+    for (int i = tid; i < NP; i += DE_T) s1 += (double)S.E[i];
+    const double mean = de_tree_sum(s1, S.red) / NP;
     double s2 = 0.0;
-    for (int i = tid; i < NP; i += DE_T) s2 += (E[i] - mean) * (E[i] - mean);
-    red[tid] = s2;
-    __syncthreads();
-    for (int o = DE_T / 2; o > 0; o >>= 1) {
-      if (tid < o) red[tid] += red[tid + o];
-      __syncthreads();
-    }
-    if (tid == 0) stop = sqrt(red[0] / NP) <= A.tol * fabs(mean);
-    __syncthreads();
-    if (stop) break;
+    for (int i = tid; i < NP; i += DE_T) s2 += ((double)S.E[i] - mean) * ((double)S.E[i] - mean);
+    const double dev = de_tree_sum(s2, S.red);
+    if (sqrt(dev / NP) <= A.tol * fabs(mean)) break;
   }
+  if (rank > 0) return;
   // best member, its FP64 objective
-  double bv = __longlong_as_double(0x7ff0000000000000LL);
-  int bi = 0x7fffffff;
-  for (int i = tid; i < NP; i += DE_T)
-    if (E[i] < bv || (E[i] == bv && i < bi)) { bv = E[i]; bi = i; }
-  red[tid] = bv;
-  redi[tid] = bi;
-  __syncthreads();
-  for (int o = DE_T / 2; o > 0; o >>= 1) {
-    if (tid < o && (red[tid + o] < red[tid] ||
-                    (red[tid + o] == red[tid] && redi[tid + o] < redi[tid]))) {
-      red[tid] = red[tid + o];
-      redi[tid] = redi[tid + o];
-    }
-    __syncthreads();
-  }
-  const int b = redi[0];
-  __syncthreads();
+  const int b = de_best(S.E, NP, S.redf, S.redi);
   double x[4];
-  for (int j = 0; j < 4; ++j) x[j] = (j < D) ? lo[j] + pop[b * 4 + j] * sc[j] : 0.0;
+  for (int j = 0; j < 4; ++j) x[j] = (j < D) ? S.lo[j] + S.pop[b * 4 + j] * S.sc[j] : 0.0;
   double part = 0.0;
-  for (int k = tid; k < A.n_bins[P.step]; k += DE_T) {
+  for (int k = tid; k < nb; k += DE_T) {
     double h = A.bin_h[bo + k];
     double m = 0.0;
     for (int c = 0; c < P.n_comp; ++c) m += fit_model_f64(P.code[c], h, x[2 * c], x[2 * c + 1]);
     double d = A.bin_g[bo + k] - m;
     part += d * d;
   }
-  red[tid] = part;
-  __syncthreads();
-  for (int o = DE_T / 2; o > 0; o >>= 1) {
-    if (tid < o) red[tid] += red[tid + o];
-    __syncthreads();
-  }
+  const double f = de_tree_sum(part, S.red);
   if (tid == 0) {
     for (int j = 0; j < 4; ++j) A.best_x[(int64_t)q * 4 + j] = x[j];
-    A.best_f[q] = red[0];
+    A.best_f[q] = f;
     A.n_gen[q] = gen > A.maxiter ? A.maxiter : gen;
   }
 }
@@ -779,12 +894,13 @@ extern "C" int spi_vg_de(int32_t n_prob, const spi_de_problem_t* prob, const int
   if (n_prob == 0) return SPI_OK;
   if (!prob || !bin_off || !n_bins || !bin_h || !bin_g || !best_x || !best_f || !n_gen)
     return SPI_ERR_ARG;
-  size_t smem = (size_t)DE_MAXNP * 4 * 8 * 2 + (size_t)DE_MAXNP * 8 * 2 + (size_t)DE_MAXBINS * 4 * 2;
+  if (n_prob > INT32_MAX / DE_CL) return SPI_ERR_TOO_LARGE;
+  const size_t smem = sizeof(DeSmem);
   if (cudaFuncSetAttribute(k_de, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return SPI_ERR_CUDA;
   DeArgs A{n_prob, prob, bin_off, n_bins, bin_h, bin_g, maxiter, tol, best_x, best_f, n_gen};
-  k_de<<<n_prob, DE_T, smem, (cudaStream_t)stream>>>(A);
+  k_de<<<n_prob * DE_CL, DE_T, smem, (cudaStream_t)stream>>>(A);
   SPI_LAUNCH_CHECK();
   return SPI_OK;
 }
