@@ -4,19 +4,27 @@
 // stations with external drifts. Estimates only: the right-hand side of a
 // cell is used once per pass, so it is generated on the fly, never stored.
 //
-// Layout: one CTA = 32 cells x 8 warps. A lane owns a cell; the 8 warps
-// split the system's stations (warp w takes stations w, w + 8, ...). Each
-// lane generates its cell's entry for the warp's station (coordinates and
-// station data are warp-uniform broadcast loads) and accumulates it against
-// up to 4 vectors: the system's dual columns (Lagrange / drift rows, for
-// the sum check of interp/steps.py:419) and the steps' dual weights. The 8
-// partial sums per cell are reduced in shared memory; more steps than fit
+// Layout: one CTA = 8 warps over 32 cells (FP64) or 64 (FP32 tier, two to a
+// lane). The 8 warps split the system's stations (warp w takes stations w,
+// w + 8, ...). Each lane generates its cells' entries for the warp's station
+// (station data are warp-uniform broadcast loads) and accumulates them
+// against up to 4 vectors: the system's dual columns (Lagrange / drift rows,
+// for the sum check of interp/steps.py:419) and the steps' dual weights. The
+// 8 partial sums per cell are reduced in shared memory; more steps than fit
 // in one pass regenerate the right-hand side. Precision as k_krige_cells:
 // FP64 throughout, or (the mixed path's FP32 tier) double-float entries
-// (rhs_df, ~1e-9) against FP32 hi/lo vector pairs, accumulated in
-// double-float and flushed to FP64 every 256 terms: the estimate's error is
-// sum_i dc_i w_i, which large dual weights amplify. With ws.cell_yy (the
-// tensor-core |Linv c|^2) the FP32 tier also writes the OK variance.
+// against FP32 hi/lo vector pairs, accumulated in double-float and flushed
+// to FP64 every 256 terms: the estimate's error is sum_i dc_i w_i, which
+// large dual weights amplify. With ws.cell_yy (the tensor-core |Linv c|^2)
+// the FP32 tier also writes the OK variance.
+//
+// The FP32 tier is bound by the instructions of an entry: about 165 as
+// normalised double-floats (rhs_df_single's sqrt, exp and products), about 80
+// as the pairs of rho_pair, which are no further from exact (rms 2^-44 of
+// the sill for Exp and Gau instead of 2^-41.5, 2^-45 both for Sph and Lin).
+// One cell to a lane also left every second issue slot empty, waiting on the
+// chain of one entry. 8 systems of 2900 stations, 10^6 cells, 4 vectors:
+// 203 ms before, 90 ms now; 8 of 750 stations, 250 000 cells: 33 to 19.4 ms.
 #include <type_traits>
 
 #include "spi_cells.cuh"
@@ -24,56 +32,81 @@
 
 namespace spi {
 
-constexpr int STC = 32;  // cells per CTA (one per lane)
+constexpr int STC = 32;  // cells per CTA and cell of a lane
+constexpr int SC4 = 2;   // cells of a lane in the FP32 tier
 constexpr int SNW = 8;   // warps per CTA (station groups)
 constexpr int SSV = 4;   // vectors per pass
 constexpr int SCH = 256; // stations per shared-memory chunk (FP32 tier)
 
-// One shared-memory chunk of stations against the pass's vectors (FP32
-// tier): double-float entries (rhs_df, or rhs_df_single<CODE> for a
-// single-structure variogram) times hi/lo vector pairs, the product's head
-// by the FMA error, the cross terms, TwoSum into a double-float partial,
-// flushed to FP64 every 256 terms. Dual columns that feed only the sum
-// check (v0 + v < plain_duals) take a plain FP32 product.
-template <int CODE, bool TRACK>
-__device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t* vgp,
-                                             const RhsDf& kd, int sk, double sh, float4 cp,
-                                             bool live, int64_t gc, const int32_t* idxc,
-                                             const float4* s_sp, const float2 (*s_w)[SCH],
-                                             int nj, int warp, int nv, int v0, int plain_duals,
-                                             float (&ph)[SSV], float (&pl)[SSV],
-                                             double (&acc)[SSV], int& cnt, NearDf& nf,
-                                             int j0, float esp) {
-  for (int jj = warp; jj < nj; jj += SNW) {
-    df c = {0.f, 0.f};
-    if (live) {
-      const df d2 = df_dist2(cp, s_sp[jj]);
-      if constexpr (TRACK) nf.add(d2, j0 + jj, esp);
-      if constexpr (CODE < 0)
-        c = rhs_df_d2(A.dom, vgp, kd, sk, sh, d2, gc, idxc + jj);
-      else
-        c = rhs_df_single_d2<CODE>(A.dom, vgp, kd, sk, sh, d2, gc, idxc + jj);
+// An entry of either form in the stream's inner loop. CODE: the single
+// structure's model (rho_pair, in units of its sill), or -1 (rhs_df_d2).
+// SK's entries at or below the cut are zero, OK's / EDK's past it the whole
+// sill; entries near it take the exact form (rho_cut).
+template <int CODE, bool SK, bool TRACK>
+__device__ __forceinline__ df stream_entry(const CellsArgs& A, const spi_vg_t* vgp,
+                                           const RhsDf& kd, const RhsOne& ko, const float2* tab,
+                                           double sh, float4 cp, float4 sp, int64_t gc,
+                                           const int32_t* stp, int j, float esp, NearDf& nf) {
+  if constexpr (CODE < 0) {
+    const df d2 = df_dist2(cp, sp);
+    if constexpr (TRACK) nf.add(d2, j, esp);
+    return rhs_df_d2(A.dom, vgp, kd, SK, sh, d2, gc, stp);
+  } else {
+    const df s = dist2_pair(cp, sp);
+    if constexpr (TRACK) nf.add(s, j, esp);
+    df v = rho_pair<CODE>(ko, s, tab);
+    if constexpr (SK) {
+      const bool z = v.h < ko.lo;
+      v.h = z ? 0.f : v.h;
+      v.l = z ? 0.f : v.l;
+      if (!z && v.h <= ko.hi) v = rho_cut(A.dom, vgp, kd, ko, 1, sh, gc, stp, v);
+    } else {
+      if (v.h >= ko.hi) v = rho_cut(A.dom, vgp, kd, ko, 0, sh, gc, stp, v);
     }
+    return v;
+  }
+}
+
+// One shared-memory chunk of stations against the pass's vectors (FP32
+// tier): double-float entries times hi/lo vector pairs, the product's head
+// by the FMA error, the cross terms, TwoSum into a double-float partial that
+// the caller flushes to FP64 every 256 terms. The first np vectors, dual
+// columns that feed only the sum check, take a plain FP32 product. A lane's
+// two cells share the loads, and their chains overlap.
+template <int CODE, bool SK, bool TRACK>
+__device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t* vgp,
+                                             const RhsDf& kd, const RhsOne& ko,
+                                             const float2* tab, double sh, const float4 (&cp)[2],
+                                             const int64_t (&gc)[2], const int32_t* idxc,
+                                             const float4* s_sp, const float2 (*s_w)[SSV],
+                                             int nj, int warp, int np, int nv,
+                                             float (&ph)[SSV][2], float (&pl)[SSV][2],
+                                             NearDf (&nf)[2], int j0, float esp) {
+  for (int jj = warp; jj < nj; jj += SNW) {
+    const float4 sp = s_sp[jj];
+    df c[2];
 #pragma unroll
-    for (int v = 0; v < SSV; ++v)
-      if (v < nv && v0 + v < plain_duals) {
-        ph[v] = __fmaf_rn(c.h, s_w[v][jj].x, ph[v]);
-      } else if (v < nv) {
-        const float2 w = s_w[v][jj];
-        const float p = __fmul_rn(c.h, w.x);
-        float e = __fmaf_rn(c.h, w.x, -p);
-        e = __fmaf_rn(c.h, w.y, e);
-        e = __fmaf_rn(c.l, w.x, e);
-        const df s2 = two_sum(ph[v], p);
-        ph[v] = s2.h;
-        pl[v] += s2.l + e;
-      }
-    if (++cnt == 256) {
-      cnt = 0;
+    for (int u = 0; u < 2; ++u)
+      c[u] = stream_entry<CODE, SK, TRACK>(A, vgp, kd, ko, tab, sh, cp[u], sp, gc[u], idxc + jj,
+                                           j0 + jj, esp, nf[u]);
 #pragma unroll
-      for (int v = 0; v < SSV; ++v) {
-        acc[v] += (double)ph[v] + (double)pl[v];
-        ph[v] = pl[v] = 0.f;
+    for (int v = 0; v < SSV; ++v) {
+      if (v >= nv) continue;
+      const float2 w = s_w[jj][v];
+      if (v < np) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) ph[v][u] = __fmaf_rn(c[u].h, w.x, ph[v][u]);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const float p = __fmul_rn(c[u].h, w.x);
+          float e = __fmaf_rn(c[u].h, w.x, -p);
+          e = __fmaf_rn(c[u].h, w.y, e);
+          e = __fmaf_rn(c[u].l, w.x, e);
+          const df s2 = two_sum(ph[v][u], p);
+          ph[v][u] = s2.h;
+          pl[v][u] += s2.l + e;
+        }
       }
     }
   }
@@ -81,9 +114,11 @@ __device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t*
 
 template <typename T, typename OutT>
 __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A) {
+  constexpr int NC = sizeof(T) == 4 ? SC4 : 1;  // cells of a lane
+  constexpr int TC = STC * NC;                  // cells of the CTA
   const int s = blockIdx.y;
   const int64_t C = A.dom.n_cells;
-  const int64_t c0 = (int64_t)blockIdx.x * STC;
+  const int64_t c0 = (int64_t)blockIdx.x * TC;
   if (c0 >= C || (A.skip && A.skip[(int64_t)s * A.skip_stride])) return;
   const int route = A.ws.route[s];
   {
@@ -113,30 +148,36 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
   const spi_vg_t vg = A.sys.vg[s];
   const double sh = A.ws.shift[s];
 
-  __shared__ double red[SNW][SSV][STC];
-  __shared__ double vres[SSV][STC];
-  __shared__ double qsh[GA][STC];  // dual columns (more than a pass holds: EDK, 4 drifts on)
-  __shared__ int okf[STC], nnb[STC];
-  __shared__ double cvar[STC];
+  __shared__ double red[SNW][SSV][TC];
+  __shared__ double vres[SSV][TC];
+  __shared__ double qsh[GA][TC];  // dual columns (more than a pass holds: EDK, 4 drifts on)
+  __shared__ int okf[TC], nnb[TC];
+  __shared__ double cvar[TC];
   __shared__ const double* vp64[SSV];
   __shared__ const float* vph[SSV];
   __shared__ const float* vpl[SSV];
   __shared__ int any_bad;
   __shared__ int any_chk;
   __shared__ float4 s_sp[sizeof(T) == 4 ? SCH : 1];
-  __shared__ float2 s_w[SSV][sizeof(T) == 4 ? SCH : 1];
+  __shared__ __align__(16) float2 s_w[sizeof(T) == 4 ? SCH : 1][SSV];
+  __shared__ float2 s_tab[sizeof(T) == 4 ? 256 : 1];
   // the FP32 tier's nearest-station candidates per station group (warp)
   // and cell, from the first pass's right-hand sides (written over red once
   // the pass's sums are reduced), and the cells they leave ambiguous
   NearDf* s_nf = reinterpret_cast<NearDf*>(&red[0][0][0]);
-  static_assert(sizeof(NearDf) * SNW * STC <= sizeof(red), "candidates fit in red");
-  __shared__ int namb[STC];
+  static_assert(sizeof(NearDf) * SNW * TC <= sizeof(red), "candidates fit in red");
+  __shared__ int namb[TC];
   const bool fuse_nnb = sizeof(T) == 4 && A.dom.split_res > 0.0;
   const float esp = (float)(A.dom.split_res * 0x1p-24);
   bool nf_ready = false;
 
-  const int64_t gc = c0 + lane;
-  const bool live = gc < C;
+  // this lane's cells c0 + lane, c0 + lane + 32 (past the grid: its last)
+  int64_t gc[NC];
+#pragma unroll
+  for (int u = 0; u < NC; ++u) {
+    gc[u] = c0 + u * STC + lane;
+    if (gc[u] >= C) gc[u] = C - 1;
+  }
   OutT* est_out = reinterpret_cast<OutT*>(A.out.est);
   // the OK variance needs |Linv c|^2 per cell from the tensor-core kernel
   const bool var_out = sizeof(T) == 4 && A.want_var && A.out.var != nullptr && !sk &&
@@ -167,13 +208,13 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
   auto nearest = [&]() {
     __syncthreads();
     if (any_bad) {
-      if (tid < STC) {
+      if (tid < TC) {
         int amb = 1;
         if constexpr (sizeof(T) == 4) {
           if (nf_ready) {
             NearDf m = s_nf[tid];
 #pragma unroll
-            for (int w = 1; w < SNW; ++w) m.merge(s_nf[w * STC + tid]);
+            for (int w = 1; w < SNW; ++w) m.merge(s_nf[w * TC + tid]);
             if (!m.amb && m.bj >= 0) {
               nnb[tid] = m.bj;
               amb = 0;
@@ -183,7 +224,7 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
         namb[tid] = amb;
       }
       __syncthreads();
-      for (int cell = warp; cell < STC; cell += SNW) {
+      for (int cell = warp; cell < TC; cell += SNW) {
         const int64_t g = c0 + cell;
         if (g >= C || okf[cell] || !namb[cell]) continue;
         const int j = nnb_f64_warp(A.dom, idx, n, A.dom.cell_x[g], A.dom.cell_y[g]);
@@ -194,30 +235,34 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
   };
 
   if (failed) {
-    if (tid < STC) {
+    if (tid < TC) {
       okf[tid] = 0;
       cvar[tid] = 0.0;
     }
     if (tid == 0) any_bad = 1;
     nearest();
-    for (int e = tid; e < nsteps * STC; e += STC * SNW) emit(e % STC, e / STC, 0.0);
+    for (int e = tid; e < nsteps * TC; e += STC * SNW) emit(e % TC, e / TC, 0.0);
     return;
   }
 
   double cx = 0.0, cy = 0.0;
-  float4 cp = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 cp[NC];
   __shared__ RhsDf kd;
+  __shared__ RhsOne ko;
   // the variogram with its reciprocal ranges (FP64 right-hand sides)
   __shared__ VgPre vgp64;
   if constexpr (sizeof(T) == 8) {
-    if (live) {
-      cx = A.dom.cell_x[gc];
-      cy = A.dom.cell_y[gc];
-    }
+    cx = A.dom.cell_x[gc[0]];
+    cy = A.dom.cell_y[gc[0]];
     if (tid == 0) vgp64.init(vg);
   } else {
-    if (live) cp = reinterpret_cast<const float4*>(A.dom.cell_split)[gc];
-    if (tid == 0) kd.init(vg, sh, A.dom.min_vg_val);
+#pragma unroll
+    for (int u = 0; u < NC; ++u) cp[u] = reinterpret_cast<const float4*>(A.dom.cell_split)[gc[u]];
+    if (tid == 0) {
+      kd.init(vg, sh, A.dom.min_vg_val);
+      if (kd.exact && kd.single >= 0) ko.init(kd, vg, sk, sh, A.dom.min_vg_val);
+    }
+    for (int e = tid; e < 256; e += STC * SNW) s_tab[e] = kExp2.v[e];
   }
   const spi_vg_t* vgp = A.sys.vg + s;
   const float4* sp4 = reinterpret_cast<const float4*>(A.dom.stn_split);
@@ -246,35 +291,42 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
       vpl[tid] = pl;
     }
     __syncthreads();
-    double acc[SSV];
+    double acc[SSV][NC];
 #pragma unroll
-    for (int v = 0; v < SSV; ++v) acc[v] = 0.0;
+    for (int v = 0; v < SSV; ++v)
+#pragma unroll
+      for (int u = 0; u < NC; ++u) acc[v][u] = 0.0;
     // (OK / EDK on the Cholesky path pass the sum check on every cell:
     // their sum(lambda) is 1 up to rounding whatever the right-hand side)
     const bool track = sizeof(T) == 4 && fuse_nnb && v0 == 0 && sk;
-    NearDf nf;
-    nf.init();
+    NearDf nf[NC];
+#pragma unroll
+    for (int u = 0; u < NC; ++u) nf[u].init();
     if constexpr (sizeof(T) == 8) {
       for (int j = warp; j < n; j += SNW) {
         const int st = idx[j];
-        double c = 0.0;
-        if (live) {
-          const double g = vgp64.fill_d2(
-              dist2_f64(cx, cy, A.dom.stn_x[st], A.dom.stn_y[st]), sk, A.dom.min_vg_val);
-          c = (sk || prim) ? g : __dsub_rn(sh, g);
-        }
+        const double g = vgp64.fill_d2(
+            dist2_f64(cx, cy, A.dom.stn_x[st], A.dom.stn_y[st]), sk, A.dom.min_vg_val);
+        const double c = (sk || prim) ? g : __dsub_rn(sh, g);
 #pragma unroll
         for (int v = 0; v < SSV; ++v)
-          if (v < nv) acc[v] = fma(c, vp64[v][j], acc[v]);
+          if (v < nv) acc[v][0] = fma(c, vp64[v][j], acc[v][0]);
       }
     } else {
       // double-float entries against hi/lo vectors (stream_chunk)
-      float ph[SSV], pl[SSV];
+      float ph[SSV][NC], pl[SSV][NC];
+      // the single structure's model, uniform over the CTA; its sums are in
+      // units of its sill
+      const int scode = (kd.exact && kd.single >= 0 && ko.sill > 0.0) ? kd.code[kd.single] : -1;
+      const double unit = scode < 0 ? 1.0 : ko.sill;
+      const int np = min(max(plain_duals - v0, 0), nv);
 #pragma unroll
-      for (int v = 0; v < SSV; ++v) ph[v] = pl[v] = 0.f;
-      int cnt = 0;
+      for (int v = 0; v < SSV; ++v)
+#pragma unroll
+        for (int u = 0; u < NC; ++u) ph[v][u] = pl[v][u] = 0.f;
       // stations in chunks staged in shared memory: split coordinates and
       // the vectors' hi/lo pairs, read by every warp at a shared index
+      int cnt = 0;
       for (int j0 = 0; j0 < n; j0 += SCH) {
         const int nj = min(SCH, n - j0);
         __syncthreads();
@@ -282,55 +334,56 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
           s_sp[e] = sp4[idx[j0 + e]];
 #pragma unroll
           for (int v = 0; v < SSV; ++v)
-            if (v < nv) s_w[v][e] = make_float2(vph[v][j0 + e], vpl[v][j0 + e]);
+            if (v < nv) s_w[e][v] = make_float2(vph[v][j0 + e], vpl[v][j0 + e]);
         }
         __syncthreads();
-        // the single structure's model, uniform over the CTA
-        const int scode = (kd.exact && kd.single >= 0) ? kd.code[kd.single] : -1;
         const int32_t* idxc = idx + j0;
         // the nearest-station tracking as a compile-time choice: kernels
         // that never need it carry none of its state through the loop
-        auto chunk = [&](auto trk) {
-          constexpr bool TR = decltype(trk)::value;
+        auto chunk = [&](auto skt, auto trk) {
+          constexpr bool SK = decltype(skt)::value, TR = decltype(trk)::value;
+#define SPI_STREAM_CHUNK(CODE)                                                                  \
+  stream_chunk<CODE, SK, TR>(A, vgp, kd, ko, s_tab, sh, cp, gc, idxc, s_sp, s_w, nj, warp, np, \
+                             nv, ph, pl, nf, j0, esp)
           switch (scode) {
-            case SPI_VG_EXP:
-              stream_chunk<SPI_VG_EXP, TR>(A, vgp, kd, sk, sh, cp, live, gc, idxc, s_sp, s_w, nj,
-                                           warp, nv, v0, plain_duals, ph, pl, acc, cnt, nf, j0,
-                                           esp);
-              break;
-            case SPI_VG_GAU:
-              stream_chunk<SPI_VG_GAU, TR>(A, vgp, kd, sk, sh, cp, live, gc, idxc, s_sp, s_w, nj,
-                                           warp, nv, v0, plain_duals, ph, pl, acc, cnt, nf, j0,
-                                           esp);
-              break;
-            case SPI_VG_SPH:
-              stream_chunk<SPI_VG_SPH, TR>(A, vgp, kd, sk, sh, cp, live, gc, idxc, s_sp, s_w, nj,
-                                           warp, nv, v0, plain_duals, ph, pl, acc, cnt, nf, j0,
-                                           esp);
-              break;
-            case SPI_VG_LIN:
-              stream_chunk<SPI_VG_LIN, TR>(A, vgp, kd, sk, sh, cp, live, gc, idxc, s_sp, s_w, nj,
-                                           warp, nv, v0, plain_duals, ph, pl, acc, cnt, nf, j0,
-                                           esp);
-              break;
-            default:
-              stream_chunk<-1, TR>(A, vgp, kd, sk, sh, cp, live, gc, idxc, s_sp, s_w, nj, warp, nv,
-                                   v0, plain_duals, ph, pl, acc, cnt, nf, j0, esp);
+            case SPI_VG_EXP: SPI_STREAM_CHUNK(SPI_VG_EXP); break;
+            case SPI_VG_GAU: SPI_STREAM_CHUNK(SPI_VG_GAU); break;
+            case SPI_VG_SPH: SPI_STREAM_CHUNK(SPI_VG_SPH); break;
+            case SPI_VG_LIN: SPI_STREAM_CHUNK(SPI_VG_LIN); break;
+            default: SPI_STREAM_CHUNK(-1);
           }
+#undef SPI_STREAM_CHUNK
         };
         if (track)
-          chunk(std::true_type{});
+          chunk(std::true_type{}, std::true_type{});
+        else if (sk)
+          chunk(std::true_type{}, std::false_type{});
         else
-          chunk(std::false_type{});
+          chunk(std::false_type{}, std::false_type{});
+        cnt += SCH / SNW;
+        if (cnt >= 256 || j0 + SCH >= n) {
+          cnt = 0;
+#pragma unroll
+          for (int v = 0; v < SSV; ++v)
+#pragma unroll
+            for (int u = 0; u < NC; ++u) {
+              acc[v][u] += (double)ph[v][u] + (double)pl[v][u];
+              ph[v][u] = pl[v][u] = 0.f;
+            }
+        }
       }
 #pragma unroll
-      for (int v = 0; v < SSV; ++v) acc[v] += (double)ph[v] + (double)pl[v];
+      for (int v = 0; v < SSV; ++v)
+#pragma unroll
+        for (int u = 0; u < NC; ++u) acc[v][u] *= unit;
     }
 #pragma unroll
-    for (int v = 0; v < SSV; ++v) red[warp][v][lane] = acc[v];
+    for (int v = 0; v < SSV; ++v)
+#pragma unroll
+      for (int u = 0; u < NC; ++u) red[warp][v][u * STC + lane] = acc[v][u];
     __syncthreads();
-    for (int e = tid; e < nv * STC; e += STC * SNW) {
-      const int v = e / STC, cell = e % STC;
+    for (int e = tid; e < nv * TC; e += STC * SNW) {
+      const int v = e / TC, cell = e % TC;
       double t = 0.0;
 #pragma unroll
       for (int w = 0; w < SNW; ++w) t += red[w][v][cell];
@@ -338,17 +391,19 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
     }
     __syncthreads();
     if (track) {
-      s_nf[warp * STC + lane] = nf;  // red is free again
+      // red is free again
+#pragma unroll
+      for (int u = 0; u < NC; ++u) s_nf[warp * TC + u * STC + lane] = nf[u];
       nf_ready = true;
     }
-    for (int e = tid; e < nv * STC; e += STC * SNW)
-      if (v0 + e / STC < ndual) qsh[v0 + e / STC][e % STC] = vres[e / STC][e % STC];
+    for (int e = tid; e < nv * TC; e += STC * SNW)
+      if (v0 + e / TC < ndual) qsh[v0 + e / TC][e % TC] = vres[e / TC][e % TC];
     __syncthreads();
     if (v0 < ndual && v0 + nv >= ndual) {
       // the sum check of every cell, once its dual columns are complete
       if (tid == 0) any_bad = any_chk = 0;
       __syncthreads();
-      if (tid < STC) {
+      if (tid < TC) {
         const int cell = tid;
         const int64_t g = c0 + cell;
         double q[GA], f[GA], nu[GA];
@@ -388,7 +443,7 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
       }
       __syncthreads();
       if (any_chk)
-        for (int cell = warp; cell < STC; cell += SNW) {
+        for (int cell = warp; cell < TC; cell += SNW) {
           if (okf[cell] != 2) continue;
           const int64_t g = c0 + cell;
           const double sl = sk_sum_lambda_f64(A.dom, vg, idx, n, A.ws.g_cols + soff * GA,
@@ -401,15 +456,16 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
         }
       nearest();
     }
-    for (int e = tid; e < nv * STC; e += STC * SNW) {
-      const int v = v0 + e / STC, cell = e % STC;
-      if (v >= ndual) emit(cell, v - ndual, vres[e / STC][cell]);
+    for (int e = tid; e < nv * TC; e += STC * SNW) {
+      const int v = v0 + e / TC, cell = e % TC;
+      if (v >= ndual) emit(cell, v - ndual, vres[e / TC][cell]);
     }
   }
 }
 
 int launch_cells_stream(const CellsArgs& A, int precision, cudaStream_t st) {
-  const int64_t tiles = (A.dom.n_cells + STC - 1) / STC;
+  const int tc = precision == 0 ? STC : STC * SC4;
+  const int64_t tiles = (A.dom.n_cells + tc - 1) / tc;
   if (tiles > 0x7fffffff) return SPI_ERR_TOO_LARGE;
   dim3 grid((unsigned)tiles, (unsigned)A.sys.n_sys);
   const bool f64 = A.out.out_f64 != 0;

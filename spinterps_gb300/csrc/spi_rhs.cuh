@@ -2,6 +2,8 @@
 // variogram term of interp/steps.py:639-650 / cyth/interpmthds.pyx:146-226,
 // generated from coordinates instead of read from a cell x station matrix.
 #pragma once
+#include <cstdint>
+
 #include "spi_common.cuh"
 
 namespace spi {
@@ -329,6 +331,161 @@ __device__ __forceinline__ df rhs_df_single(const spi_domain_t& dom, const spi_v
                                             const RhsDf& k, int sk, double sh, float4 cp,
                                             float4 sp, int64_t gc, const int32_t* stp) {
   return rhs_df_single_d2<CODE>(dom, vgp, k, sk, sh, df_dist2(cp, sp), gc, stp);
+}
+
+// ---- The same entries for a variogram with one structure, at under half
+// the instructions (the streamed kernel's inner loop, which is bound by
+// them): the correlation alone, the sill multiplied into the sums at their
+// end; pairs (h, l) that need not be normalised (|l| may reach 2^-22 |h|);
+// the exponential to base 2 with 1/256 steps, whose reduction is exact and
+// whose remainder needs two FP32 terms only in its linear part. Each pair
+// is good to about 2^-43 of the correlation's scale 1, as rho_df.
+struct Exp2Tab {
+  float2 v[256];  // 2^(-j / 256), head and tail
+};
+constexpr uint64_t exp2_mulhi(uint64_t a, uint64_t b) {
+  const uint64_t ah = a >> 32, al = a & 0xffffffffu, bh = b >> 32, bl = b & 0xffffffffu;
+  const uint64_t m = ah * bl + ((al * bl) >> 32), m2 = al * bh + (m & 0xffffffffu);
+  return ah * bh + (m >> 32) + (m2 >> 32);
+}
+constexpr Exp2Tab exp2_table() {
+  // 2^-(2^-k) as Q64, k = 1..8
+  const uint64_t f[8] = {0xb504f333f9de6484ull, 0xd744fccad69d6af4ull, 0xeac0c6e7dd24392full,
+                         0xf5257d152486cc2cull, 0xfa83b2db722a033aull, 0xfd3e0c0cf486c175ull,
+                         0xfe9e115c7b8f884cull, 0xff4ecb59511ec8a5ull};
+  Exp2Tab t{};
+  for (int j = 0; j < 256; ++j) {
+    uint64_t v = 1ull << 63;  // Q63
+    for (int k = 1; k <= 8; ++k)
+      if (j & (256 >> k)) v = exp2_mulhi(v, f[k - 1]);
+    const uint64_t head = (v + (1ull << 38)) >> 39;  // 24 or 25 bits: 2^-24 units
+    const int64_t tail = (int64_t)(v - (head << 39));
+    t.v[j].x = (float)(double)head * 0x1p-24f;
+    t.v[j].y = (float)((double)tail * 0x1p-63);
+  }
+  return t;
+}
+__device__ const Exp2Tab kExp2 = exp2_table();
+
+struct RhsOne {
+  float kh, kl;      // the distance's factor (Exp, Sph, Lin: to t; Gau: d^2's)
+  float inv_h, inv_l;   // 1 / sill
+  float lo, hi;      // the band of rho that needs the cut's exact form
+  double sill;
+  __device__ __forceinline__ void init(const RhsDf& k, const spi_vg_t& vg, int sk, double sh,
+                                       double min_vg_val) {
+    const int q = k.single, code = vg.code[q];
+    const double r = vg.range[q], k3 = 256.0 * 4.328085122666891;  // 3 / ln 2
+    const double f = code == SPI_VG_EXP ? k3 / r : (code == SPI_VG_GAU ? k3 / (r * r) : 1.0 / r);
+    const df kk = df_from(f);
+    kh = kk.h;
+    kl = kk.l;
+    sill = vg.sill[q];
+    const df iv = df_from(1.0 / sill);
+    inv_h = iv.h;
+    inv_l = iv.l;
+    lo = -1.f;
+    hi = sk ? -1.f : INFINITY;
+    if (k.mvv > 0.f && (sk || !k.nug_clear)) {
+      if (sk) {
+        lo = (float)((min_vg_val - 2.0 * k.band_sk) / sill * (1.0 - 1e-6));
+        hi = (float)((min_vg_val + 2.0 * k.band_sk) / sill * (1.0 + 1e-6));
+      } else {
+        hi = (float)((sh - min_vg_val - 2.0 * k.band_ok) / sill) - 1e-6f;
+      }
+    }
+  }
+};
+
+// d^2 of split coordinates, not normalised: s.h + s.l
+__device__ __forceinline__ df dist2_pair(float4 cp, float4 sp) {
+  const df x = fast_two_sum(__fsub_rn(cp.x, sp.x), __fsub_rn(cp.y, sp.y));
+  const df y = fast_two_sum(__fsub_rn(cp.z, sp.z), __fsub_rn(cp.w, sp.w));
+  const float xx = __fmul_rn(x.h, x.h), yy = __fmul_rn(y.h, y.h);
+  const float ex = __fmaf_rn(__fadd_rn(x.h, x.h), x.l, __fmaf_rn(x.h, x.h, -xx));
+  const float ey = __fmaf_rn(__fadd_rn(y.h, y.h), y.l, __fmaf_rn(y.h, y.h, -yy));
+  const df s = two_sum(xx, yy);
+  return {s.h, __fadd_rn(s.l, __fadd_rn(ex, ey))};
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return 1.0f / sqrtf(x);
+#endif
+}
+// its root (coinciding points: about 1e-19, which every model takes as 0)
+__device__ __forceinline__ df sqrt_pair(df s) {
+  const float u = fmaxf(__fadd_rn(s.h, s.l), 1e-36f);
+  const float r = rsqrt_ftz(u);
+  const float h = __fmul_rn(u, r);
+  const float e = __fadd_rn(__fmaf_rn(-h, h, s.h), s.l);
+  return {h, __fmul_rn(e, __fmul_rn(0.5f, r))};
+}
+__device__ __forceinline__ df mul_pair(df a, float kh, float kl) {
+  const float p = __fmul_rn(a.h, kh);
+  return {p, __fmaf_rn(a.l, kh, __fmaf_rn(a.h, kl, __fmaf_rn(a.h, kh, -p)))};
+}
+// 2^-(t / 256), t >= 0; 0 from 2^-127 on
+__device__ __forceinline__ df exp2_pair(df t, const float2* tab) {
+  const float lim = 127.f * 256.f;
+  const float tl = t.h < lim ? t.l : 0.f;
+  const float th = fminf(t.h, lim);
+  const float big = __fadd_rn(th, 12582912.0f);  // the nearest integer in the low bits
+  const uint32_t m = __float_as_uint(big);
+  const float f = __fsub_rn(th, __fsub_rn(big, 12582912.0f));
+  const float2 T = tab[m & 255u];
+  const float sc = __uint_as_float(0x3F800000u - ((m & 0xffffff00u) << 15));
+  const float x = __fadd_rn(f, tl);
+  // p = 1 - 2^-(x / 256) = A x - B x^2 + C x^3 - D x^4, A = Ah + Al
+  const float Ah = 0.00270760618150234222f, Al = -7.440055859e-12f;
+  const float q = __fmaf_rn(-x, __fmaf_rn(-x, __fmaf_rn(-x, 2.2393951909e-12f, 3.3083026805e-9f),
+                                          3.6655655969e-6f), Al);
+  const float ph = __fmul_rn(f, Ah);
+  const float pl = __fmaf_rn(tl, Ah, __fmaf_rn(x, q, __fmaf_rn(f, Ah, -ph)));
+  const float h = __fmaf_rn(-T.x, ph, T.x);
+  const float e = __fmaf_rn(-T.x, ph, __fsub_rn(T.x, h));
+  const float l = __fadd_rn(__fmaf_rn(-T.x, pl, e), __fmaf_rn(-T.y, ph, T.y));
+  return {__fmul_rn(h, sc), __fmul_rn(l, sc)};
+}
+
+// rho of one entry; s: dist2_pair
+template <int CODE>
+__device__ __forceinline__ df rho_pair(const RhsOne& k, df s, const float2* tab) {
+  if constexpr (CODE == SPI_VG_GAU) {
+    return exp2_pair(mul_pair(s, k.kh, k.kl), tab);
+  } else {
+    const df t = mul_pair(sqrt_pair(s), k.kh, k.kl);
+    if constexpr (CODE == SPI_VG_EXP) {
+      return exp2_pair(t, tab);
+    } else {
+      // 1 - t, and for Sph (1 - t)^2 (1 + t / 2)
+      const float uh = __fsub_rn(1.f, t.h);
+      const float ul = __fsub_rn(__fsub_rn(__fsub_rn(1.f, uh), t.h), t.l);
+      df v = {uh, ul};
+      if constexpr (CODE == SPI_VG_SPH) {
+        const float q = __fmul_rn(uh, uh);
+        const float qe = __fmaf_rn(__fadd_rn(uh, uh), ul, __fmaf_rn(uh, uh, -q));
+        const float wh = __fmaf_rn(0.5f, t.h, 1.f);
+        const float we = __fmaf_rn(0.5f, t.l, __fmaf_rn(0.5f, t.h, __fsub_rn(1.f, wh)));
+        const float c = __fmul_rn(q, wh);
+        v = {c, __fmaf_rn(qe, wh, __fmaf_rn(q, we, __fmaf_rn(q, wh, -c)))};
+      }
+      const bool in = t.h < 1.0f;
+      return {in ? v.h : 0.f, in ? v.l : 0.f};
+    }
+  }
+}
+
+// The cut of an entry near or past it (rhs_df_cut), in units of the sill.
+inline __device__ __noinline__ df rho_cut(const spi_domain_t& dom, const spi_vg_t* vgp, const RhsDf& k,
+                                   const RhsOne& o, int sk, double sh, int64_t gc,
+                                   const int32_t* stp, df rho) {
+  const df c = rhs_df_cut(dom, vgp, k, sk, sh, gc, stp,
+                          df_mul(k.sill[k.single], fast_two_sum(rho.h, rho.l)));
+  return df_mul(c, df{o.inv_h, o.inv_l});
 }
 
 // The nearest station of a cell from the double-float squared distances of
