@@ -22,9 +22,15 @@
 // normalised double-floats (rhs_df_single's sqrt, exp and products), about 80
 // as the pairs of rho_pair, which are no further from exact (rms 2^-44 of
 // the sill for Exp and Gau instead of 2^-41.5, 2^-45 both for Sph and Lin).
-// One cell to a lane also left every second issue slot empty, waiting on the
-// chain of one entry. 8 systems of 2900 stations, 10^6 cells, 4 vectors:
-// 203 ms before, 90 ms now; 8 of 750 stations, 250 000 cells: 33 to 19.4 ms.
+// One cell to a lane and 16 warps to an SM left every second issue slot
+// empty, waiting on the chain of one entry: two cells to a lane, 32 warps
+// (the FP64 totals in shared memory, the entries without a pair form out of
+// line; what still spills at 64 registers lies outside the loop), one
+// branch for both cells' cuts and the usual passes' vectors known at
+// compile time. 8 systems of 2900 stations, 10^6 cells, 4 vectors: 203 ms
+// as double-floats, 90 with the pairs, 72.5 with 32 warps; 8 of 750
+// stations, 250 000 cells: 33, 19.4, 17.4 ms. (Three CTAs of 80 registers
+// are as fast on large grids, a sixth slower on small systems.)
 #include <type_traits>
 
 #include "spi_cells.cuh"
@@ -38,33 +44,12 @@ constexpr int SNW = 8;   // warps per CTA (station groups)
 constexpr int SSV = 4;   // vectors per pass
 constexpr int SCH = 256; // stations per shared-memory chunk (FP32 tier)
 
-// An entry of either form in the stream's inner loop. CODE: the single
-// structure's model (rho_pair, in units of its sill), or -1 (rhs_df_d2).
-// SK's entries at or below the cut are zero, OK's / EDK's past it the whole
-// sill; entries near it take the exact form (rho_cut).
-template <int CODE, bool SK, bool TRACK>
-__device__ __forceinline__ df stream_entry(const CellsArgs& A, const spi_vg_t* vgp,
-                                           const RhsDf& kd, const RhsOne& ko, const float2* tab,
-                                           double sh, float4 cp, float4 sp, int64_t gc,
-                                           const int32_t* stp, int j, float esp, NearDf& nf) {
-  if constexpr (CODE < 0) {
-    const df d2 = df_dist2(cp, sp);
-    if constexpr (TRACK) nf.add(d2, j, esp);
-    return rhs_df_d2(A.dom, vgp, kd, SK, sh, d2, gc, stp);
-  } else {
-    const df s = dist2_pair(cp, sp);
-    if constexpr (TRACK) nf.add(s, j, esp);
-    df v = rho_pair<CODE>(ko, s, tab);
-    if constexpr (SK) {
-      const bool z = v.h < ko.lo;
-      v.h = z ? 0.f : v.h;
-      v.l = z ? 0.f : v.l;
-      if (!z && v.h <= ko.hi) v = rho_cut(A.dom, vgp, kd, ko, 1, sh, gc, stp, v);
-    } else {
-      if (v.h >= ko.hi) v = rho_cut(A.dom, vgp, kd, ko, 0, sh, gc, stp, v);
-    }
-    return v;
-  }
+// An entry without a pair form (rhs_df_d2); out of line, so that its FP64
+// models don't set the registers of the loop below.
+inline __device__ __noinline__ df stream_general(const CellsArgs& A, const spi_vg_t* vgp,
+                                                 const RhsDf& kd, int sk, double sh, df d2,
+                                                 int64_t gc, const int32_t* stp) {
+  return rhs_df_d2(A.dom, vgp, kd, sk, sh, d2, gc, stp);
 }
 
 // One shared-memory chunk of stations against the pass's vectors (FP32
@@ -73,7 +58,11 @@ __device__ __forceinline__ df stream_entry(const CellsArgs& A, const spi_vg_t* v
 // the caller flushes to FP64 every 256 terms. The first np vectors, dual
 // columns that feed only the sum check, take a plain FP32 product. A lane's
 // two cells share the loads, and their chains overlap.
-template <int CODE, bool SK, bool TRACK>
+// CODE: the single structure's model (rho_pair, in units of its sill), or -1.
+// SK's entries at or below the cut are zero, OK's / EDK's past it the whole
+// sill; entries near it take the exact form (rho_cut). NP, NV: np and nv
+// where they are known at compile time, or -1.
+template <int CODE, bool SK, bool TRACK, int NP, int NV>
 __device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t* vgp,
                                              const RhsDf& kd, const RhsOne& ko,
                                              const float2* tab, double sh, const float4 (&cp)[2],
@@ -82,13 +71,39 @@ __device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t*
                                              int nj, int warp, int np, int nv,
                                              float (&ph)[SSV][2], float (&pl)[SSV][2],
                                              NearDf (&nf)[2], int j0, float esp) {
+  const float lo = ko.lo, hi = ko.hi;
   for (int jj = warp; jj < nj; jj += SNW) {
     const float4 sp = s_sp[jj];
     df c[2];
+    if constexpr (CODE < 0) {
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
-      c[u] = stream_entry<CODE, SK, TRACK>(A, vgp, kd, ko, tab, sh, cp[u], sp, gc[u], idxc + jj,
-                                           j0 + jj, esp, nf[u]);
+      for (int u = 0; u < 2; ++u) {
+        const df d2 = df_dist2(cp[u], sp);
+        if constexpr (TRACK) nf[u].add(d2, j0 + jj, esp);
+        c[u] = stream_general(A, vgp, kd, SK, sh, d2, gc[u], idxc + jj);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const df s = dist2_pair(cp[u], sp);
+        if constexpr (TRACK) nf[u].add(s, j0 + jj, esp);
+        c[u] = rho_pair<CODE>(ko, s, tab);
+        if constexpr (SK) {
+          const bool z = c[u].h < lo;
+          c[u].h = z ? 0.f : c[u].h;
+          c[u].l = z ? 0.f : c[u].l;
+        }
+      }
+      // (one branch for both cells)
+      if (SK ? (c[0].h >= lo && c[0].h <= hi) || (c[1].h >= lo && c[1].h <= hi)
+             : fmaxf(c[0].h, c[1].h) >= hi) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (SK ? c[u].h >= lo && c[u].h <= hi : c[u].h >= hi)
+            c[u] = rho_cut(A.dom, vgp, kd, ko, SK, sh, gc[u], idxc + jj, c[u]);
+      }
+    }
+    if constexpr (NV >= 0) np = NP, nv = NV;
 #pragma unroll
     for (int v = 0; v < SSV; ++v) {
       if (v >= nv) continue;
@@ -113,7 +128,8 @@ __device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t*
 }
 
 template <typename T, typename OutT>
-__global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A) {
+__global__ __launch_bounds__(STC * SNW, sizeof(T) == 4 ? 4 : 2) void k_krige_cells_stream(
+    CellsArgs A) {
   constexpr int NC = sizeof(T) == 4 ? SC4 : 1;  // cells of a lane
   constexpr int TC = STC * NC;                  // cells of the CTA
   const int s = blockIdx.y;
@@ -291,18 +307,17 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
       vpl[tid] = pl;
     }
     __syncthreads();
-    double acc[SSV][NC];
-#pragma unroll
-    for (int v = 0; v < SSV; ++v)
-#pragma unroll
-      for (int u = 0; u < NC; ++u) acc[v][u] = 0.0;
     // (OK / EDK on the Cholesky path pass the sum check on every cell:
     // their sum(lambda) is 1 up to rounding whatever the right-hand side)
     const bool track = sizeof(T) == 4 && fuse_nnb && v0 == 0 && sk;
     NearDf nf[NC];
 #pragma unroll
     for (int u = 0; u < NC; ++u) nf[u].init();
+    double unit = 1.0;  // of the sums
     if constexpr (sizeof(T) == 8) {
+      double acc[SSV];
+#pragma unroll
+      for (int v = 0; v < SSV; ++v) acc[v] = 0.0;
       for (int j = warp; j < n; j += SNW) {
         const int st = idx[j];
         const double g = vgp64.fill_d2(
@@ -310,20 +325,25 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
         const double c = (sk || prim) ? g : __dsub_rn(sh, g);
 #pragma unroll
         for (int v = 0; v < SSV; ++v)
-          if (v < nv) acc[v][0] = fma(c, vp64[v][j], acc[v][0]);
+          if (v < nv) acc[v] = fma(c, vp64[v][j], acc[v]);
       }
+#pragma unroll
+      for (int v = 0; v < SSV; ++v) red[warp][v][lane] = acc[v];
     } else {
       // double-float entries against hi/lo vectors (stream_chunk)
       float ph[SSV][NC], pl[SSV][NC];
       // the single structure's model, uniform over the CTA; its sums are in
       // units of its sill
       const int scode = (kd.exact && kd.single >= 0 && ko.sill > 0.0) ? kd.code[kd.single] : -1;
-      const double unit = scode < 0 ? 1.0 : ko.sill;
+      if (scode >= 0) unit = ko.sill;
       const int np = min(max(plain_duals - v0, 0), nv);
 #pragma unroll
       for (int v = 0; v < SSV; ++v)
 #pragma unroll
-        for (int u = 0; u < NC; ++u) ph[v][u] = pl[v][u] = 0.f;
+        for (int u = 0; u < NC; ++u) {
+          ph[v][u] = pl[v][u] = 0.f;
+          red[warp][v][u * STC + lane] = 0.0;  // (this thread's alone)
+        }
       // stations in chunks staged in shared memory: split coordinates and
       // the vectors' hi/lo pairs, read by every warp at a shared index
       int cnt = 0;
@@ -338,13 +358,15 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
         }
         __syncthreads();
         const int32_t* idxc = idx + j0;
-        // the nearest-station tracking as a compile-time choice: kernels
-        // that never need it carry none of its state through the loop
-        auto chunk = [&](auto skt, auto trk) {
+        // compile-time choices: the model, the nearest-station tracking
+        // (kernels that never need it carry none of its state through the
+        // loop), the vectors of the usual passes
+        auto chunk = [&](auto skt, auto trk, auto npt, auto nvt) {
           constexpr bool SK = decltype(skt)::value, TR = decltype(trk)::value;
-#define SPI_STREAM_CHUNK(CODE)                                                                  \
-  stream_chunk<CODE, SK, TR>(A, vgp, kd, ko, s_tab, sh, cp, gc, idxc, s_sp, s_w, nj, warp, np, \
-                             nv, ph, pl, nf, j0, esp)
+          constexpr int NP = decltype(npt)::value, NV = decltype(nvt)::value;
+#define SPI_STREAM_CHUNK(CODE)                                                                 \
+  stream_chunk<CODE, SK, TR, NP, NV>(A, vgp, kd, ko, s_tab, sh, cp, gc, idxc, s_sp, s_w, nj, \
+                                     warp, np, nv, ph, pl, nf, j0, esp)
           switch (scode) {
             case SPI_VG_EXP: SPI_STREAM_CHUNK(SPI_VG_EXP); break;
             case SPI_VG_GAU: SPI_STREAM_CHUNK(SPI_VG_GAU); break;
@@ -354,12 +376,30 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
           }
 #undef SPI_STREAM_CHUNK
         };
-        if (track)
-          chunk(std::true_type{}, std::true_type{});
-        else if (sk)
-          chunk(std::true_type{}, std::false_type{});
-        else
-          chunk(std::false_type{}, std::false_type{});
+        using Yes = std::true_type;
+        using No = std::false_type;
+#define SPI_N(i) std::integral_constant<int, i>{}
+        const int form = scode < 0 ? 0 : np * 8 + nv;
+        if (track) {
+          if (form == 3) chunk(Yes{}, Yes{}, SPI_N(0), SPI_N(3));
+          else chunk(Yes{}, Yes{}, SPI_N(-1), SPI_N(-1));
+        } else if (sk) {
+          if (form == 3) chunk(Yes{}, No{}, SPI_N(0), SPI_N(3));
+          else chunk(Yes{}, No{}, SPI_N(-1), SPI_N(-1));
+        } else {
+          switch (form) {
+            case 1: chunk(No{}, No{}, SPI_N(0), SPI_N(1)); break;
+            case 2: chunk(No{}, No{}, SPI_N(0), SPI_N(2)); break;
+            case 4: chunk(No{}, No{}, SPI_N(0), SPI_N(4)); break;
+            case 10: chunk(No{}, No{}, SPI_N(1), SPI_N(2)); break;
+            case 12: chunk(No{}, No{}, SPI_N(1), SPI_N(4)); break;
+            case 20: chunk(No{}, No{}, SPI_N(2), SPI_N(4)); break;
+            case 19: chunk(No{}, No{}, SPI_N(2), SPI_N(3)); break;
+            case 28: chunk(No{}, No{}, SPI_N(3), SPI_N(4)); break;
+            default: chunk(No{}, No{}, SPI_N(-1), SPI_N(-1));
+          }
+        }
+#undef SPI_N
         cnt += SCH / SNW;
         if (cnt >= 256 || j0 + SCH >= n) {
           cnt = 0;
@@ -367,27 +407,19 @@ __global__ __launch_bounds__(STC * SNW, 2) void k_krige_cells_stream(CellsArgs A
           for (int v = 0; v < SSV; ++v)
 #pragma unroll
             for (int u = 0; u < NC; ++u) {
-              acc[v][u] += (double)ph[v][u] + (double)pl[v][u];
+              red[warp][v][u * STC + lane] += (double)ph[v][u] + (double)pl[v][u];
               ph[v][u] = pl[v][u] = 0.f;
             }
         }
       }
-#pragma unroll
-      for (int v = 0; v < SSV; ++v)
-#pragma unroll
-        for (int u = 0; u < NC; ++u) acc[v][u] *= unit;
     }
-#pragma unroll
-    for (int v = 0; v < SSV; ++v)
-#pragma unroll
-      for (int u = 0; u < NC; ++u) red[warp][v][u * STC + lane] = acc[v][u];
     __syncthreads();
     for (int e = tid; e < nv * TC; e += STC * SNW) {
       const int v = e / TC, cell = e % TC;
       double t = 0.0;
 #pragma unroll
       for (int w = 0; w < SNW; ++w) t += red[w][v][cell];
-      vres[v][cell] = t;
+      vres[v][cell] = t * unit;
     }
     __syncthreads();
     if (track) {
