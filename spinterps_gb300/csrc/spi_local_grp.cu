@@ -5,6 +5,8 @@
 // group's matrix once (np.linalg.pinv, interp/steps.py:351-352) and then
 // forms lmds = inv @ rhs per cell (_fill_krig_idw_dst_data,
 // interp/steps.py:403-435). Here likewise:
+// - k_grp_table: the variogram between every two stations, once per step,
+//   where the groups' matrices together hold more entries than that.
 // - k_grp_factor: one warp per (group, step) builds the group's saddle
 //   matrix ([[Gamma, 1, S], [1', 0, 0], [S', 0, 0]], SK: the covariances)
 //   in shared memory and inverts it in place by Gauss-Jordan with partial
@@ -63,6 +65,7 @@ struct GrpArgs {
   double min_var_thr;
   int32_t want_var;
   int32_t m_max;
+  const double* tab;        // [nq][n_stns][n_stns] (k_grp_table), or null
   spi_out_t out;
   int32_t* prblm;
 };
@@ -79,6 +82,44 @@ __device__ __forceinline__ int group_size(const int32_t* nb, int k) {
   return n;
 }
 
+// Gamma of every two stations (saddle_entry's upper-left part). An entry is
+// some 45 FP64 operations (a root, the model), and neighbouring groups share
+// most of their pairs: 40 000 groups of 16 from 750 stations hold 10 million
+// entries a step, the stations 0.28 million pairs. Gathered instead from a
+// table that stays in L2.
+__global__ __launch_bounds__(256) void k_grp_table(GrpArgs A, int32_t q0,
+                                                   double* __restrict__ tab) {
+  const int q = q0 + blockIdx.y;
+  if (A.nug[q]) return;
+  const int N = A.dom.n_stns;
+  const spi_vg_t vg = A.vg[q];
+  const int sk = A.kind == SPI_KIND_SK;
+  double* T = tab + (int64_t)blockIdx.y * N * N;
+  const int64_t nn = (int64_t)N * N;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nn;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(e / N), j = (int)(e - (int64_t)i * N);
+    if (j < i) continue;
+    const double d = dist_f64(A.dom.stn_x[i], A.dom.stn_y[i], A.dom.stn_x[j], A.dom.stn_y[j]);
+    const double v = vg_fill_f64(vg, d, sk, A.dom.min_vg_val);
+    T[e] = v;
+    T[(int64_t)j * N + i] = v;
+  }
+}
+
+// |x| as an integer in its order (NaN above infinity): the pivot search
+// without FP64 compares, which issue at 1/64 of an integer's rate.
+__device__ __forceinline__ uint64_t abs_key(double x) {
+  return (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+
+// Bound by FP64 issue. Of some 1080 FP64 instructions of a warp for a group
+// of 16 (m = 17), 450 were the entries (k_grp_table takes them), 290 the
+// updates with a lane per column (17 of 32 lanes; spread over all elements
+// here: 153), 140 the pivot search's compares and the tests for zero (integer
+// here) and 200 the divisions by the pivot. 12 steps of 62 500 cells with 16
+// neighbours out of 750: 15.7 ms before, 5.7 and 0.8 for the tables now; 12 of
+// 20 083 cells with 12 out of 270: 6.4, now 2.4 and 0.1.
 __global__ void k_grp_factor(GrpArgs A, int32_t q0, int32_t nq, double* __restrict__ inv,
                              int32_t* __restrict__ status) {
   extern __shared__ double gsm[];
@@ -89,6 +130,7 @@ __global__ void k_grp_factor(GrpArgs A, int32_t q0, int32_t nq, double* __restri
   const int sk = A.kind == SPI_KIND_SK;
   const int a = extra_rows(A.kind, A.dom.n_drift);
   const int64_t G = A.n_grps;
+  const int N = A.dom.n_stns;
   const int64_t ntask = G * nq;
   const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -106,12 +148,20 @@ __global__ void k_grp_factor(GrpArgs A, int32_t q0, int32_t nq, double* __restri
       if (lane == 0) status[t] = GRP_NONE;
       continue;
     }
-    const spi_vg_t vg = A.vg[q];
+    const spi_vg_t& vg = A.vg[q];
+    const double* T = A.tab ? A.tab + (int64_t)ql * N * N : nullptr;
     const int m = n + a;
+    // a lane's elements e = lane, lane + 32, .. as (i, j): from one to the
+    // next di rows and dj columns
+    const int i0 = lane / m, j0 = lane - i0 * m, di = 32 / m, dj = 32 - di * m;
     double fm = 0.0;
-    for (int e = lane; e < m * m; e += 32) {
-      const int i = e / m, j = e - i * m;
-      const double x = saddle_entry(A.dom, vg, nb, n, sk, i, j);
+    for (int i = i0, j = j0; i < m; i += di, j += dj) {
+      if (j >= m) {
+        j -= m;
+        if (++i >= m) break;
+      }
+      const double x = (T && i < n && j < n) ? T[(int64_t)nb[i] * N + nb[j]]
+                                             : saddle_entry(A.dom, vg, nb, n, sk, i, j);
       M[i * mm + j] = x;
       fm += x * x;
     }
@@ -122,24 +172,26 @@ __global__ void k_grp_factor(GrpArgs A, int32_t q0, int32_t nq, double* __restri
     int piv0 = 0, piv1 = 0, piv2 = 0;
     bool zero_piv = false;
     for (int c = 0; c < m; ++c) {
-      double best = -1.0;
+      // the first row of the largest |pivot| (NaN counts as infinite)
+      uint64_t best = 0;
       int bp = 0x7fffffff;
       for (int r = c + lane; r < m; r += 32) {
-        const double x = fabs(M[r * mm + c]);
-        if (x > best || isnan(x)) {
-          best = isnan(x) ? INFINITY : x;
+        uint64_t x = abs_key(M[r * mm + c]);
+        if (x > 0x7ff0000000000000ull) x = 0x7ff0000000000000ull;
+        if (x > best || bp == 0x7fffffff) {
+          best = x;
           bp = r;
         }
       }
       for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const uint64_t ob = __shfl_xor_sync(0xffffffffu, best, o);
         const int op = __shfl_xor_sync(0xffffffffu, bp, o);
         if (ob > best || (ob == best && op < bp)) {
           best = ob;
           bp = op;
         }
       }
-      if (!(best > 0.0) || isinf(best)) {
+      if (best == 0 || best == 0x7ff0000000000000ull) {
         zero_piv = true;
         break;
       }
@@ -160,13 +212,14 @@ __global__ void k_grp_factor(GrpArgs A, int32_t q0, int32_t nq, double* __restri
       for (int j = lane; j < m; j += 32) M[c * mm + j] = (j == c ? 1.0 : M[c * mm + j]) / d;
       for (int i = lane; i < m; i += 32) f[i] = M[i * mm + c];
       __syncwarp();
-      for (int j = lane; j < m; j += 32) {
-        const double rc = M[c * mm + j];
-        for (int i = 0; i < m; ++i) {
-          if (i == c) continue;
-          const double fi = f[i];
-          if (fi != 0.0) M[i * mm + j] = (j == c ? 0.0 : M[i * mm + j]) - fi * rc;
+      for (int i = i0, j = j0; i < m; i += di, j += dj) {
+        if (j >= m) {
+          j -= m;
+          if (++i >= m) break;
         }
+        const double fi = f[i];
+        if (i != c && abs_key(fi) != 0)
+          M[i * mm + j] = (j == c ? 0.0 : M[i * mm + j]) - fi * M[c * mm + j];
       }
       __syncwarp();
     }
@@ -189,8 +242,11 @@ __global__ void k_grp_factor(GrpArgs A, int32_t q0, int32_t nq, double* __restri
     }
     double* P = inv + t * (int64_t)mm * mm;
     double fp = 0.0;
-    for (int e = lane; e < m * m; e += 32) {
-      const int i = e / m, j = e - i * m;
+    for (int i = i0, j = j0; i < m; i += di, j += dj) {
+      if (j >= m) {
+        j -= m;
+        if (++i >= m) break;
+      }
       const double x = M[i * mm + j];
       P[i * mm + j] = x;
       fp += x * x;
@@ -324,13 +380,21 @@ extern "C" int spi_local_groups(const spi_domain_t* dom, int32_t kind, int32_t k
   if (mm > SPI_LOCAL_MAX_NEBS + 8) return SPI_ERR_TOO_LARGE;
   const int64_t per = SPI_LOCAL_GRP_BYTES(mm);
   const int64_t fixed = SPI_LOCAL_GRP_PINV_BYTES(mm);
-  const int64_t per_step = per * n_grps;
+  int64_t per_step = per * n_grps;
   if (scratch_bytes < fixed + per_step) return SPI_ERR_TOO_LARGE;
+  // the table of all stations' pairs, where it has no more entries than the
+  // groups' matrices and the scratch holds it
+  const int64_t tab_n = (int64_t)dom->n_stns * dom->n_stns;
+  const bool tab = tab_n <= (int64_t)n_grps * k * k &&
+                   scratch_bytes >= fixed + per_step + tab_n * (int64_t)sizeof(double);
+  if (tab) per_step += tab_n * (int64_t)sizeof(double);
   const int64_t q_fit = (scratch_bytes - fixed) / per_step;
-  const int32_t nq_max = (int32_t)(q_fit < n_steps ? q_fit : n_steps);
+  int32_t nq_max = (int32_t)(q_fit < n_steps ? q_fit : n_steps);
+  if (tab && nq_max > 65535) nq_max = 65535;  // k_grp_table's grid
   double* pinv_ws = reinterpret_cast<double*>(scratch);
   double* inv = reinterpret_cast<double*>(reinterpret_cast<char*>(scratch) + fixed);
-  int32_t* status = reinterpret_cast<int32_t*>(inv + (int64_t)nq_max * n_grps * mm * mm);
+  double* tabs = inv + (int64_t)nq_max * n_grps * mm * mm;
+  int32_t* status = reinterpret_cast<int32_t*>(tabs + (tab ? nq_max * tab_n : 0));
 
   spi::GrpArgs A;
   A.dom = *dom;
@@ -349,6 +413,7 @@ extern "C" int spi_local_groups(const spi_domain_t* dom, int32_t kind, int32_t k
   A.min_var_thr = min_var_thr;
   A.want_var = want_var;
   A.m_max = mm;
+  A.tab = tab ? tabs : nullptr;
   A.out = *out;
   A.prblm = prblm;
 
@@ -369,6 +434,12 @@ extern "C" int spi_local_groups(const spi_domain_t* dom, int32_t kind, int32_t k
     const int64_t ftask = (int64_t)n_grps * nq;
     int64_t fblocks = (ftask + warps - 1) / warps;
     if (fblocks > 152 * 64) fblocks = 152 * 64;
+    if (tab) {
+      const int64_t tb = (tab_n + 255) / 256;
+      spi::k_grp_table<<<dim3((unsigned)(tb < 152 * 16 ? tb : 152 * 16), (unsigned)nq), 256, 0,
+                         st>>>(A, q0, tabs);
+      SPI_LAUNCH_CHECK();
+    }
     spi::k_grp_factor<<<(unsigned)fblocks, 32 * warps, fsmem, st>>>(A, q0, nq, inv, status);
     SPI_LAUNCH_CHECK();
     const int rc = spi::local_grp_pinv(*dom, kind, k, grp_nebs, n_grps, q0, nq, vg, inv, mm,

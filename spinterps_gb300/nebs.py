@@ -179,6 +179,11 @@ def interp_steps_nebs(stn_x, stn_y, data, cell_x, cell_y, vgs, interp_args, neb_
                     held.append(grp)
                 need = nat.lib().spi_local_groups_scratch_bytes(kind, k, n_drift, G, rows.size)
                 one = nat.lib().spi_local_groups_scratch_bytes(kind, k, n_drift, G, 1)
+                # room for the table of all stations' pairs, which the call
+                # makes where the groups hold more entries than it
+                if sx.size ** 2 <= G * k * k:
+                    need += rows.size * sx.size ** 2 * 8
+                    one += sx.size ** 2 * 8
                 nbytes = max(one, min(need, GRP_SCRATCH_BYTES))
                 if scratch is None or scratch.numel() < nbytes:
                     scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
