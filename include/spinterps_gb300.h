@@ -112,6 +112,15 @@ int spi_neb_select(int32_t method, const double *dst_x, const double *dst_y, int
                    const double *ref_x, const double *ref_y, int32_t n_ref, int32_t n_nebs,
                    int32_t n_pies, int32_t *idxs, spi_stream_t stream);
 
+/* The first row with the same k values, of every row of nb [n, k] (groups of
+ * cells with identical neighbour lists, interp/grps.py:103-138): rep [n].
+ * n <= 2^30; scratch 16-byte aligned, spi_neb_rep_scratch_bytes(n) (-1 for
+ * invalid n). */
+int spi_neb_rep(const int32_t *nb, int64_t n, int32_t k, int32_t *rep, void *scratch,
+                int64_t scratch_bytes, spi_stream_t stream);
+int64_t spi_neb_rep_scratch_bytes(int64_t n);
+
+
 /* ---- batched step engine ------------------------------------------------
  *
  * Replaces the per-group loop of SpInterpSteps._get_interp
@@ -743,7 +752,9 @@ int spi_local_cells(const spi_domain_t *dom, int32_t kind, int32_t k, const int3
  * nug[q]; a single neighbour's value (variance NaN). scratch: 16-byte
  * aligned, at least spi_local_groups_scratch_bytes(kind, k, dom->n_drift,
  * n_grps, 1) bytes; steps are processed in chunks that fit it (all at once
- * with spi_local_groups_scratch_bytes(..., n_steps)). k <=
+ * with spi_local_groups_scratch_bytes(..., n_steps)); where n_stns^2 <=
+ * n_grps k^2, another n_stns^2 8 bytes a step save the groups the
+ * re-evaluation of shared station pairs (the same fields). k <=
  * SPI_LOCAL_MAX_NEBS. Device arrays. */
 int spi_local_groups(const spi_domain_t *dom, int32_t kind, int32_t k,
                      const int32_t *grp_nebs, int32_t n_grps, const int32_t *cell_grp,

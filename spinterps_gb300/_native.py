@@ -140,6 +140,7 @@ _SIGS = {
                   c_ptr],
     "spi_neb_select": [c_i32, c_ptr, c_ptr, c_i64, c_ptr, c_ptr, c_i32, c_i32, c_i32, c_ptr,
                        c_ptr],
+    "spi_neb_rep": [c_ptr, c_i64, c_i32, c_ptr, c_ptr, c_i64, c_ptr],
     "spi_vg_refine": [c_i32, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_dbl, c_ptr, c_ptr,
                       c_ptr, c_ptr],
     "spi_vg_features": [c_i32, c_ptr, c_ptr, c_ptr, c_ptr, c_i32, c_ptr, c_ptr],
@@ -178,7 +179,7 @@ _SIGS = {
 # every entry point the header declares (checked by the CPU tests)
 EXPORTS = sorted(list(_SIGS) + ["spi_version", "spi_cuda_error", "spi_mlp_n_params",
                                  "spi_local_groups_scratch_bytes", "spi_slices_scratch_bytes",
-                                 "spi_slices_one_scratch_bytes"])
+                                 "spi_slices_one_scratch_bytes", "spi_neb_rep_scratch_bytes"])
 
 _lib = None
 _lock = threading.Lock()
@@ -211,6 +212,8 @@ def load(path=LIB_PATH):
         lib.spi_slices_one_scratch_bytes.argtypes = [c_i32, c_i32]
         lib.spi_slices_scratch_bytes.restype = c_i64
         lib.spi_slices_scratch_bytes.argtypes = [c_i32] * 6
+        lib.spi_neb_rep_scratch_bytes.restype = c_i64
+        lib.spi_neb_rep_scratch_bytes.argtypes = [c_i64]
         _lib = lib
         return lib
 

@@ -407,7 +407,78 @@ __global__ __launch_bounds__(NEB_T) void k_neb_pie(const double* __restrict__ dx
   }
 }
 
+// Rows of neighbour lists into a hash table of row indices (open addressing,
+// linear probing; tab: -1 where free, first: the smallest row of a slot's
+// list). Rows are compared in full, so a slot is one list whatever its hash.
+__global__ __launch_bounds__(256) void k_neb_hash(const int32_t* __restrict__ nb, int64_t n, int k,
+                                                  uint32_t mask, int32_t* __restrict__ tab,
+                                                  int32_t* __restrict__ first,
+                                                  int32_t* __restrict__ slot) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int32_t* a = nb + i * k;
+  uint32_t h = 2166136261u;
+  for (int q = 0; q < k; ++q) {
+    h = (h ^ (uint32_t)a[q]) * 0x9e3779b1u;
+    h ^= h >> 15;
+  }
+  for (uint32_t probe = 0; probe <= mask; ++probe) {  // (half the table is free)
+    const uint32_t s = (h + probe) & mask;
+    const int32_t other = atomicCAS(tab + s, -1, (int32_t)i);
+    bool same = true;
+    if (other >= 0 && other != i) {
+      const int32_t* b = nb + (int64_t)other * k;
+      for (int q = 0; q < k && same; ++q) same = a[q] == b[q];
+    }
+    if (same) {
+      atomicMin(first + s, (int32_t)i);
+      slot[i] = (int32_t)s;
+      return;
+    }
+  }
+}
+__global__ __launch_bounds__(256) void k_neb_first(int64_t n, const int32_t* __restrict__ first,
+                                                   const int32_t* __restrict__ slot,
+                                                   int32_t* __restrict__ rep) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) rep[i] = first[slot[i]];
+}
+
 }  // namespace spi
+
+// 2^p >= 2 n slots
+static int64_t neb_slots(int64_t n) {
+  int64_t s = 2;
+  while (s < 2 * n) s *= 2;
+  return s;
+}
+
+extern "C" int64_t spi_neb_rep_scratch_bytes(int64_t n) {
+  if (n < 0 || n > (int64_t)1 << 30) return -1;
+  return (2 * neb_slots(n) + n) * (int64_t)sizeof(int32_t);
+}
+
+extern "C" int spi_neb_rep(const int32_t* nb, int64_t n, int32_t k, int32_t* rep, void* scratch,
+                           int64_t scratch_bytes, spi_stream_t stream) {
+  if (n < 0 || k < 1) return SPI_ERR_ARG;
+  if (n > (int64_t)1 << 30) return SPI_ERR_TOO_LARGE;
+  if (n == 0) return SPI_OK;
+  if (!nb || !rep || !scratch || reinterpret_cast<uintptr_t>(scratch) % 16) return SPI_ERR_ARG;
+  if (scratch_bytes < spi_neb_rep_scratch_bytes(n)) return SPI_ERR_WORKSPACE;
+  const int64_t slots = neb_slots(n);
+  int32_t* tab = static_cast<int32_t*>(scratch);
+  int32_t *first = tab + slots, *slot = first + slots;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (cudaMemsetAsync(tab, 0xff, slots * sizeof(int32_t), st) != cudaSuccess ||
+      cudaMemsetAsync(first, 0x7f, slots * sizeof(int32_t), st) != cudaSuccess)
+    return SPI_ERR_CUDA;
+  const unsigned blocks = (unsigned)((n + 255) / 256);
+  spi::k_neb_hash<<<blocks, 256, 0, st>>>(nb, n, k, (uint32_t)(slots - 1), tab, first, slot);
+  SPI_LAUNCH_CHECK();
+  spi::k_neb_first<<<blocks, 256, 0, st>>>(n, first, slot, rep);
+  SPI_LAUNCH_CHECK();
+  return SPI_OK;
+}
 
 extern "C" int spi_neb_select(int32_t method, const double* dst_x, const double* dst_y,
                               int64_t n_dst, const double* ref_x, const double* ref_y,

@@ -76,3 +76,21 @@ def test_pie_sizes(k, n_pies, n):
     cx[:20], cy[:20] = sx[:20], sy[:20]
     cx[20:30], cy[30:40] = sx[20:30], sy[30:40]
     _check("pie", k, n_pies, sx, sy, cx, cy)
+
+
+@pytest.mark.parametrize("C,k,lists", [(1, 1, 1), (2, 16, 1), (255, 3, 40), (256, 64, 256),
+                                       (4097, 12, 1), (60000, 16, 9000)])
+def test_groups_of_equal_lists(C, k, lists):
+    import torch
+    from spinterps_gb300.nebs import device_groups
+    rng = np.random.default_rng(C + k)
+    pool = np.sort(rng.integers(-1, 50, size=(lists, k)), axis=1).astype(np.int32)
+    nb = pool[rng.integers(0, lists, C)]
+    g, c, o = (t.cpu().numpy() for t in device_groups(torch.as_tensor(nb, device="cuda")))
+    uniq, first, inv = np.unique(nb, axis=0, return_index=True, return_inverse=True)
+    rank = np.empty(first.size, dtype=np.int64)      # groups in order of first cells
+    rank[np.argsort(first)] = np.arange(first.size)
+    assert np.array_equal(g, uniq[np.argsort(first)])
+    assert np.array_equal(c, rank[inv.ravel()])
+    assert np.array_equal(o, np.argsort(c, kind="stable"))
+    assert g.dtype == c.dtype == o.dtype == np.int32
