@@ -212,3 +212,51 @@ def test_local_groups_match_per_cell_solve(kind_name):
             assert np.abs(v1 - v0).max() <= 1e-9 * np.abs(v0).max()
     assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1],
                                                                    equal_nan=True)
+
+
+@pytest.mark.parametrize("kind,p", [(3, 2.0), (3, 1.0), (3, 3.5), (4, 0.0)])
+@pytest.mark.parametrize("k", [1, 2, 16, 33, 64])
+def test_near_cells_vs_numpy(kind, p, k):
+    """spi_local_cells' IDW and NNB (k_local_near): empty slots, destinations
+    on stations (NaN), ties (the first), values under the threshold (mean).
+    FP64 sums of up to 64 positive-weight terms: 64 * 2^-52 and a few ulp for
+    the weights, 1e-13 relative to the largest value."""
+    import ctypes
+    import torch
+    from spinterps_gb300 import _native as nat
+    from spinterps_gb300.steps import _Domain, _out_struct, _ptr, _stream
+    rng = np.random.default_rng(k)
+    N, C, T = 90, 257, 3
+    sx, sy = rng.integers(0, 30, N) * 100.0, rng.integers(0, 30, N) * 100.0
+    cx, cy = rng.integers(0, 60, C) * 50.0, rng.integers(0, 60, C) * 50.0
+    nb = np.sort(np.argsort(rng.uniform(size=(C, N)), axis=1)[:, :k], axis=1).astype(np.int32)
+    nb[1, 1:] = -1
+    nb[2, (k + 1) // 2:] = -1
+    z = rng.gamma(1.0, 2.0, size=(T, N))
+    z[2, rng.uniform(size=N) < 0.9] = 0.0
+    thr = 0.5
+    dom = _Domain(torch.device("cuda"), sx, sy, cx, cy, None, None, 0.0, 0)
+    d_nb, d_z = torch.as_tensor(nb, device="cuda"), torch.as_tensor(z, device="cuda")
+    steps = torch.arange(T, dtype=torch.int32, device="cuda")
+    est = torch.full((T, C), 7.0, dtype=torch.float64, device="cuda")
+    nat.call("spi_local_cells", ctypes.byref(dom.st), kind, k, _ptr(d_nb), T, _ptr(steps),
+             _ptr(steps), _ptr(d_z), N, None, None, thr, p, 0,
+             ctypes.byref(_out_struct(est, None, None, None)), None, _stream())
+    got = est.cpu().numpy()
+    for c in range(C):
+        s = nb[c][nb[c] >= 0]
+        d = np.hypot(sx[s] - cx[c], sy[s] - cy[c])
+        for t in range(T):
+            v = z[t, s]
+            if s.size == 1 or kind == 4:
+                want = v[np.argmin(d)]
+            elif not (v >= thr).any():
+                want = v.mean()
+            else:
+                with np.errstate(all="ignore"):
+                    w = (d / d.max()) ** -p
+                    want = (w * v).sum() / w.sum()
+            if np.isnan(want):
+                assert np.isnan(got[t, c]), (t, c)
+            else:
+                assert abs(got[t, c] - want) <= 1e-13 * z.max(), (t, c)
