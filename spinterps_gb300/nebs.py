@@ -138,8 +138,11 @@ def interp_steps_nebs(stn_x, stn_y, data, cell_x, cell_y, vgs, interp_args, neb_
     if time_steps is None:
         time_steps = np.arange(T)
     g = SpInterpNeighborGrouping(neb_sel_mthd, n_nebs, n_pies, cell_x, cell_y, device=device)
-    keep = np.unique(g.neb_idxs(stn_x, stn_y))
-    keep = keep[keep >= 0]
+    # (the stations in use flagged on the device, an empty slot's -1 in the
+    # place after them: a million indices sorted on the host took 14 ms)
+    used = torch.zeros(stn_x.size + 1, dtype=torch.bool, device=dev)
+    used[g.neb_idxs_device(stn_x, stn_y).long()] = True
+    keep = np.flatnonzero(used[:-1].cpu().numpy())
     sx, sy, data = stn_x[keep], stn_y[keep], np.ascontiguousarray(data[:, keep])
     sd = None if stn_drifts is None else np.asarray(stn_drifts).reshape(stn_x.size, -1)[keep]
     cd = None if cell_drifts is None else np.asarray(cell_drifts).reshape(-1, C)
