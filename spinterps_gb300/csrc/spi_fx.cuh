@@ -77,6 +77,12 @@ struct FxGrid {
   int q;
 };
 
+// It, and whether the points have one (finite, not past FP64's middle range).
+struct FxScene {
+  FxGrid g;
+  int ok;
+};
+
 // x - o on the grid, the difference's rounding error included.
 FX_HD int64_t fx_coord(double x, double o, int q) {
   const double d = x - o;
@@ -352,6 +358,22 @@ FX_HD int64_t fx_entry(const FxVg& f, int64_t cx, int64_t cy, int64_t sx, int64_
   int64_t v[1];
   fx_entries<-1, 1>(f, d, tab, v);
   return v[0];
+}
+
+// An integer v < 2^63 as a double times 2^-FX_BITS, by its bits (no FP64
+// operation), rounded.
+FX_HD double fx_double(uint64_t v) {
+  const int c = fx_clz(v | 1);
+  const uint64_t m = ((v << c) >> 11) + (((v << c) >> 10) & 1);
+  // (a carry into the exponent comes out right)
+  const uint64_t b = v ? ((uint64_t)(1022 + 63 - FX_BITS - c) << 52) + m : 0;
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)b);
+#else
+  double w;
+  __builtin_memcpy(&w, &b, 8);
+  return w;
+#endif
 }
 
 // A squared distance as a monotone key: the exponent above 55 bits of the

@@ -164,9 +164,9 @@ __device__ __forceinline__ int dual_rows(const SlArgs& A, int route) {
 }
 
 // The common grid of the range; false where it has none.
-__device__ bool sl_grid(const SlArgs& A, FxGrid& g) {
-  const double x0 = dec(A.head->mn[0]), x1 = dec(A.head->mx[0]);
-  const double y0 = dec(A.head->mn[1]), y1 = dec(A.head->mx[1]);
+__device__ bool sl_grid(const SlHead* h, FxGrid& g) {
+  const double x0 = dec(h->mn[0]), x1 = dec(h->mx[0]);
+  const double y0 = dec(h->mn[1]), y1 = dec(h->mx[1]);
   double ext = fmax(x1 - x0, y1 - y0);
   g.ox = x0;
   g.oy = y0;
@@ -186,7 +186,7 @@ __global__ __launch_bounds__(256) void k_sl_select(SlArgs A) {
   __shared__ FxGrid g;
   __shared__ int ok;
   if (threadIdx.x == 0) {
-    ok = sl_grid(A, g);
+    ok = sl_grid(A.head, g);
     if (blockIdx.x == 0) *A.grid = g;
   }
   __syncthreads();
@@ -1159,6 +1159,28 @@ int one_launch(SlArgs& A, const SlPlan& p, K kern, int64_t points, int sms, cuda
 }
 
 }  // namespace
+
+namespace {
+__global__ void k_fx_scene(const SlHead* h, FxScene* o) { o->ok = sl_grid(h, o->g); }
+}  // namespace
+
+int launch_fx_scene(const spi_domain_t& dom, void* scratch, const FxScene** scene,
+                    cudaStream_t st) {
+  const int sms = n_sms();
+  if (sms <= 0) return SPI_ERR_CUDA;
+  unsigned char* q = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(scratch) + 255) / 256 * 256);
+  SlHead* h = reinterpret_cast<SlHead*>(q);
+  FxScene* o = reinterpret_cast<FxScene*>(q + al(sizeof(SlHead)));
+  if (cudaMemsetAsync(h->mn, 0xff, sizeof(h->mn), st) != cudaSuccess ||
+      cudaMemsetAsync(h->mx, 0, sizeof(h->mx), st) != cudaSuccess)
+    return SPI_ERR_CUDA;
+  k_sl_range<<<2 * sms, 256, 0, st>>>(dom, h);
+  k_fx_scene<<<1, 1, 0, st>>>(h, o);
+  SPI_LAUNCH_CHECK();
+  *scene = o;
+  return SPI_OK;
+}
 
 int64_t slices_scratch_one(int n, int rows) {
   const int sms = n_sms();

@@ -2,6 +2,7 @@
 // call it.
 #pragma once
 #include "spi_common.cuh"
+#include "spi_fx.cuh"
 
 namespace spi {
 
@@ -47,6 +48,11 @@ int64_t slices_scratch(int max_n, int n_sys, int max_vec, bool var, bool vec);
 int64_t slices_scratch_one(int n, int rows);
 int launch_slices_rows(const SlRows& r, void* scratch, int64_t scratch_bytes, int32_t* err,
                        const int32_t** use, cudaStream_t st);
+
+// The fixed-point grid of a domain's points, at the start of the scratch
+// (a few hundred bytes; valid until the scratch is used for something else).
+int launch_fx_scene(const spi_domain_t& dom, void* scratch, const FxScene** scene,
+                    cudaStream_t st);
 
 int launch_slices(const SlicesCall& c, const int32_t** use, int* stride, cudaStream_t st);
 

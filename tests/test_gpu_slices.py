@@ -109,3 +109,40 @@ def test_single_neighbourhood(kind, n, C):
     for k in ("zk", "lambdas", "rhss", "in_dists"):
         a, b = got[k].cpu().numpy(), ref[k]
         assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max(), k
+
+
+@pytest.mark.parametrize("kind", ["OK", "SK", "EDK"])
+@pytest.mark.parametrize("model", ["0.1 Nug(0.0) + 0.9 Exp(30000)", "2.5 Sph(60000)",
+                                   "0.3 Nug(0.0) + 1.2 Gau(9000)", "1.0 Lin(50000)",
+                                   "0.2 Nug(0.0) + 0.5 Exp(9000) + 0.7 Sph(50000)",
+                                   "0.5 Exp(1e-5)", "0.7 Hol(20000)", "1.0 Pow(1.2)", "2.0 Nug(0.0)"])
+def test_single_neighbourhood_right_hand_sides(kind, model):
+    """Fixed-point right-hand sides (512 points on) against the FP64 formulas
+    (the same points 511 at a time), coinciding pairs included, also a
+    distance of an ulp. Either evaluation rounds a structure at most about 8
+    times at up to 1.5 times its sill: 16 * 2^-53 of the sills, twice."""
+    import torch
+    from spinterps_gb300 import legacy
+    n, C = 97, 1500
+    rng = np.random.default_rng(5)
+    xi, yi, zi = 4e6 + rng.uniform(0, 1e5, n), 5e6 + rng.uniform(0, 1e5, n), rng.gamma(1.2, 3.0, n)
+    xk, yk = 4e6 + rng.uniform(0, 1e5, C), 5e6 + rng.uniform(0, 1e5, C)
+    xk[:3], yk[:3] = xi[2:5], yi[2:5]
+    xk[1] = np.nextafter(xk[1], 0)
+    si = rng.uniform(0, 2, (1, n)) if kind == "EDK" else None
+    sk = rng.uniform(0, 2, (1, C)) if kind == "EDK" else None
+    d = lambda a: None if a is None else torch.as_tensor(a, device="cuda")  # noqa: E731
+
+    def rhss(sl):
+        s = None if sk is None else np.ascontiguousarray(sk[:, sl])
+        return legacy.krige_points(kind, d(xi), d(yi), d(zi), d(xk[sl]), d(yk[sl]), model, si=d(si),
+                                   sk=d(s))["rhss"].cpu().numpy()
+
+    got = rhss(slice(0, C))
+    ref = np.concatenate([rhss(slice(a, a + 511)) for a in range(0, C, 511)])
+    scale = np.abs(ref[:, :n]).max() if "Pow" in model else sum(
+        c[1] for c in legacy.parse_model(model))
+    assert np.abs(got[:, :n] - ref[:, :n]).max() <= 32 * 2.0 ** -53 * scale
+    assert np.array_equal(got[:, n:], ref[:, n:])
+    for i in (0, 2):     # the coinciding pairs
+        assert got[i, 2 + i] == ref[i, 2 + i]
