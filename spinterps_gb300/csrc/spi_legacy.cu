@@ -210,6 +210,156 @@ __global__ __launch_bounds__(256) void k_leg_update(double* __restrict__ A, int 
   }
 }
 
+// The elimination in one cooperative launch: each CTA keeps its rows (r, r +
+// B, ..) in shared memory for all steps, and rows are never moved: a row has a
+// position, and a swap exchanges two positions. A step: every CTA publishes
+// its largest |column k| at a position >= k together with that row; a barrier
+// over the grid; every CTA picks the largest candidate (the first position on
+// ties), scales its row and eliminates column k from its own. The same
+// operations as k_leg_pivot and k_leg_update, which take a launch each per
+// step and pass the matrix through L2 (both stay for matrices whose rows
+// don't fit, m > ~1850). A step is bound by latency, the barrier's and L2's
+// in a chain: m = 401 5.9 ms before, 3.4 now; 201 2.4, 1.2; 801 15.7, 10.5;
+// 1501 41.8, 23.7. (Half as many CTAs: 3.0, 1.2, 11.4.)
+//
+// The barrier's wait is bounded: on expiry the CTA stores a status (the
+// caller then takes its pseudo-inverse path from lhs) and leaves, and so do
+// the others at their next wait.
+struct LegCand {
+  double val;  // |pivot|, NaN as infinity; -1: no row left
+  int pos, pad;
+};
+struct LegGjWs {
+  unsigned* arrived;  // zero at launch
+  LegCand* cand;      // [2][B]
+  double* rows;       // [2][B][m]
+  int32_t* piv;
+};
+constexpr int LGJ_T = 256;
+constexpr int LGJ_WAIT = 1 << 22;  // polls, a second or so
+
+__global__ __launch_bounds__(LGJ_T) void k_leg_gj(double* __restrict__ A, int m, int rp,
+                                                  LegGjWs W, int32_t* __restrict__ status) {
+  extern __shared__ double lrows[];  // [rp][m], prow[m], f[rp], pos[rp]
+  double* prow = lrows + (int64_t)rp * m;
+  double* f = prow + m;
+  int* pos = reinterpret_cast<int*>(f + rp);
+  __shared__ int mine, gone;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int B = gridDim.x, b = blockIdx.x;
+  const int nr = b < m ? (m - 1 - b) / B + 1 : 0;  // (<= rp)
+  for (int q = 0; q < nr; ++q)
+    for (int j = tid; j < m; j += LGJ_T)
+      lrows[(int64_t)q * m + j] = A[(int64_t)(b + q * B) * m + j];
+  for (int q = tid; q < nr; q += LGJ_T) pos[q] = b + q * B;
+  if (tid == 0) gone = 0;
+  __syncthreads();
+  for (int k = 0; k < m; ++k) {
+    LegCand* cand = W.cand + (k & 1) * B;
+    double* rows = W.rows + (int64_t)(k & 1) * B * m;
+    if (tid < 32) {
+      double best = -1.0;
+      int bi = 0x7fffffff, bq = 0;
+      for (int q = lane; q < nr; q += 32) {
+        const double v = lrows[(int64_t)q * m + k];
+        f[q] = v;
+        double x = fabs(v);
+        if (isnan(x)) x = __longlong_as_double(0x7ff0000000000000LL);
+        if (pos[q] >= k && (x > best || (x == best && pos[q] < bi))) {
+          best = x;
+          bi = pos[q];
+          bq = q;
+        }
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        const double x = __shfl_xor_sync(0xffffffffu, best, o);
+        const int i = __shfl_xor_sync(0xffffffffu, bi, o);
+        const int q = __shfl_xor_sync(0xffffffffu, bq, o);
+        if (x > best || (x == best && i < bi)) {
+          best = x;
+          bi = i;
+          bq = q;
+        }
+      }
+      if (lane == 0) {
+        mine = best >= 0.0 ? bq : -1;
+        cand[b] = LegCand{best, bi, 0};
+      }
+    }
+    __syncthreads();
+    if (mine >= 0)
+      for (int j = tid; j < m; j += LGJ_T) rows[(int64_t)b * m + j] = lrows[(int64_t)mine * m + j];
+    __syncthreads();
+    if (tid == 0) {
+      const unsigned want = (unsigned)(k + 1) * (unsigned)B;
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(W.arrived) : "memory");
+      int left = LGJ_WAIT;
+      unsigned seen;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(W.arrived) : "memory");
+      } while (seen < want && --left > 0);
+      if (seen < want) {
+        gone = 1;
+        *status = k + 1;
+      }
+    }
+    __syncthreads();
+    if (gone) return;
+    // every warp finds the pivot for itself
+    double best = -1.0;
+    int p = 0x7fffffff, pb = 0;
+    for (int c = lane; c < B; c += 32) {
+      const double x = __ldcg(&cand[c].val);
+      const int i = __ldcg(&cand[c].pos);
+      if (x > best || (x == best && i < p)) {
+        best = x;
+        p = i;
+        pb = c;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double x = __shfl_xor_sync(0xffffffffu, best, o);
+      const int i = __shfl_xor_sync(0xffffffffu, p, o);
+      const int c = __shfl_xor_sync(0xffffffffu, pb, o);
+      if (x > best || (x == best && i < p)) {
+        best = x;
+        p = i;
+        pb = c;
+      }
+    }
+    if (!(best > 0.0) || isinf(best)) {  // (the same in every CTA)
+      if (b == 0 && tid == 0) *status = k + 1;
+      return;
+    }
+    if (b == 0 && tid == 0) W.piv[k] = p;
+    const double* src = rows + (int64_t)pb * m;
+    const double dd = __ldcg(src + k);
+    // the quotient from dd's reciprocal, rounded the same, within the
+    // exponents where it is (div_rcp)
+    const bool mid = best > 1e-280 && best < 1e280;
+    const double dinv = __drcp_rn(dd);
+    for (int j = tid; j < m; j += LGJ_T) {
+      const double x = j == k ? 1.0 : __ldcg(src + j);
+      const double ax = fabs(x);
+      prow[j] = mid && ax < 1e280 && (ax > 1e-280 || ax == 0.0) ? div_rcp(x, dd, dinv) : x / dd;
+    }
+    __syncthreads();
+    for (int q = 0; q < nr; ++q) {
+      double* row = lrows + (int64_t)q * m;
+      const int at = pos[q];
+      const double fi = f[q];
+      for (int j = tid; j < m; j += LGJ_T)
+        row[j] = at == p ? prow[j] : (j == k ? 0.0 : row[j]) - fi * prow[j];
+    }
+    __syncthreads();
+    for (int q = tid; q < nr; q += LGJ_T) pos[q] = pos[q] == p ? k : (pos[q] == k ? p : pos[q]);
+    __syncthreads();
+  }
+  for (int q = 0; q < nr; ++q)
+    for (int j = tid; j < m; j += LGJ_T)
+      A[(int64_t)pos[q] * m + j] = lrows[(int64_t)q * m + j];
+}
+
 // Columns back into place: the reverse pivot swaps as one permutation, a row
 // at a time through shared memory.
 __global__ __launch_bounds__(256) void k_leg_unscramble(double* __restrict__ A, int m,
@@ -512,6 +662,40 @@ static int leg_check(int32_t kind, const double* xi, const double* yi, int32_t n
   return SPI_OK;
 }
 
+namespace spi {
+// k_leg_gj where its rows fit in shared memory (a quarter as many CTAs as
+// rows at most, so that two published rows of each fit in the n^2 doubles of
+// the workspace); false: not launched.
+static bool leg_gj(double* A, int m, int n, double* ws, int32_t* piv, int32_t* status,
+                   cudaStream_t st) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return false;
+  const int B = m / 4 < sms ? m / 4 : sms;
+  int rp = (m + B - 1) / B;
+  const size_t smem = ((size_t)rp * m + m + rp) * sizeof(double) + rp * sizeof(int);
+  // piv (m ints), the counter, the candidates, the rows
+  const int64_t head = ((int64_t)m * 4 + 15) / 16 * 2 + 2;
+  const int64_t need = head + 2 * (int64_t)B * 2 + 2 * (int64_t)B * m;
+  if (smem > 200 * 1024 || need > (int64_t)n * n || reinterpret_cast<uintptr_t>(ws) % 16) return false;
+  if (!smem_opt_in(k_leg_gj, smem)) return false;
+  LegGjWs W;
+  W.piv = piv;
+  W.arrived = reinterpret_cast<unsigned*>(ws + head - 2);
+  W.cand = reinterpret_cast<LegCand*>(ws + head);
+  W.rows = ws + head + 4 * (int64_t)B;
+  if (cudaMemsetAsync(W.arrived, 0, 16, st) != cudaSuccess) return false;
+  void* args[] = {&A, &m, &rp, &W, &status};
+  if (cudaLaunchCooperativeKernel((const void*)k_leg_gj, dim3(B), dim3(LGJ_T), args, smem, st) !=
+      cudaSuccess) {
+    cudaGetLastError();  // (no room for the grid at once: the steps one by one)
+    return false;
+  }
+  return true;
+}
+}  // namespace spi
+
 extern "C" int spi_legacy_system(int32_t kind, const double* xi, const double* yi, int32_t n,
                                  const double* si, int32_t n_drift, const spi_vg_t* vg,
                                  double* in_dists, double* lhs, double* lhs_inv,
@@ -529,7 +713,9 @@ extern "C" int spi_legacy_system(int32_t kind, const double* xi, const double* y
     int32_t* piv = reinterpret_cast<int32_t*>(in_dists);  // n^2 doubles >= m ints
     const int gx = (int)((m * m + 2047) / 2048);
     spi::k_leg_fill<<<gx, 256, 0, st>>>(sk, xi, yi, n, si, mi, *vg, lhs, lhs_inv, status);
-    for (int k = 0; k < mi; ++k) {
+    SPI_LAUNCH_CHECK();
+    const bool one = spi::leg_gj(lhs_inv, mi, n, in_dists, piv, status, st);
+    for (int k = 0; k < mi && !one; ++k) {
       spi::k_leg_pivot<<<1, spi::LT, 0, st>>>(lhs_inv, mi, k, piv, status);
       spi::k_leg_update<<<(mi + 7) / 8, 256, 0, st>>>(lhs_inv, mi, k, status);
     }
