@@ -542,13 +542,48 @@ __device__ __forceinline__ void digits4(const uint64_t (&v)[4], uint2 (&o)[SL_D]
   }
 }
 
+// x 2^(q0 + 1075) as an integer (under 2^63), rounded; by shifts.
+__device__ __forceinline__ int64_t scaled_int(double x, int q0) {
+  const int64_t b = __double_as_longlong(x);
+  const int e = (int)((b >> 52) & 0x7ff);
+  const int64_t m = (b & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
+  const int sh = (e ? e : 1) + q0;  // x = m 2^(e - 1075)
+  const int64_t v = sh >= 0 ? m << min(sh, 63) : ((m >> min(-sh - 1, 62)) + 1) >> 1;
+  return b < 0 ? -v : v;
+}
+// (h 2^32 + l) 2^e as a double, rounded; by shifts, and by FP64 operations
+// only where it leaves the normal range.
+__device__ __forceinline__ double scaled_double(long long h, uint32_t l, int e) {
+  const bool neg = h < 0;
+  uint64_t a = (uint64_t)h;
+  uint32_t b = l;
+  if (neg) {
+    b = 0u - l;
+    a = ~a + (l == 0 ? 1 : 0);
+  }
+  if (a == 0 && b == 0) return 0.0;
+  // the top 64 bits, normalised: |value| = m 2^(32 - c)
+  const int c = a ? __clzll((long long)a) : 64 + __clz((int)b);
+  const uint64_t m = c >= 32 ? (c < 64 ? a << c : 0) | ((uint64_t)b << (c - 32))
+                             : (a << c) | ((uint64_t)b >> (32 - c));
+  const int f = 1022 + 63 + 32 - c + e;
+  if (f < 1 || f > 2044)
+    return scalbn(fma((double)h, 4294967296.0, (double)l), e);
+  const uint64_t bits = ((uint64_t)f << 52) + (m >> 11) + ((m >> 10) & 1);
+  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0)));
+}
+
 // Given right-hand sides, scaled by a power of two per point. S.nnb: its
 // exponent, or kNotFinite.
 constexpr int kNotFinite = 0x7fffffff;
+// Neighbouring lanes take four pairs of entries of a point (64 bytes of its
+// row), eight points to a warp (128 bytes of a slot's line); the scaling is
+// a shift of the significand.
 __device__ __forceinline__ void sl_gen_rows(const SlArgs& A, SlSmem& S, int m, int k16,
-                                            int64_t gc, int cell, int part, ulonglong2* slot) {
+                                            int64_t c0, int64_t C, int tid, ulonglong2* slot) {
   constexpr int PARTS = SL_WT / SL_M;
-  const double* r = A.rows.rhs + gc * m;
+  const int cell = tid / PARTS, part = tid % PARTS;
+  const double* r = A.rows.rhs + min(c0 + cell, C - 1) * m;
   int mx = 0;
   for (int j = part; j < m; j += PARTS) mx = max(mx, __double2hiint(r[j]) & 0x7fffffff);
   int* km = reinterpret_cast<int*>(&S.q[0][0]);
@@ -558,12 +593,12 @@ __device__ __forceinline__ void sl_gen_rows(const SlArgs& A, SlSmem& S, int m, i
   const bool bad = (mx >> 20) == 0x7ff;
   const int e = max((mx >> 20) - 1022, -900);
   if (part == 0) S.nnb[cell] = bad ? kNotFinite : e;
-  const double sc = bad ? 0.0 : ldexp(1.0, FX_BITS - e);
+  const int q0 = FX_BITS - e - 1075;
   for (int p = part; p < k16 * (SL_K / 2); p += PARTS) {
     ulonglong2 v{SL_BIAS, SL_BIAS};
     const int j = 2 * p;
-    if (j < m && !bad) v.x += (uint64_t)__double2ll_rn(r[j] * sc);
-    if (j + 1 < m && !bad) v.y += (uint64_t)__double2ll_rn(r[j + 1] * sc);
+    if (j < m && !bad) v.x += (uint64_t)scaled_int(r[j], q0);
+    if (j + 1 < m && !bad) v.y += (uint64_t)scaled_int(r[j + 1], q0);
     slot[(int64_t)p * SL_M + cell] = v;
   }
 }
@@ -710,7 +745,7 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
       work_sync();
     }
     if constexpr (MODE == kRows) {
-      sl_gen_rows(A, S, n, W.k16, min(c0 + cell, C - 1), cell, part, slot);
+      sl_gen_rows(A, S, n, W.k16, c0, C, tid, slot);
     } else {
       const int64_t gc = min(c0 + cell, C - 1);
       const FxGrid gr = *A.grid;
@@ -861,8 +896,7 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
             const double y =
                 ec == kNotFinite
                     ? __longlong_as_double(0x7ff8000000000000LL)
-                    : scalbn(fma((double)acc_h[q], 4294967296.0, (double)acc_l[q]),
-                             ec + row_e[b * SL_R + q] - 68);
+                    : scaled_double(acc_h[q], acc_l[q], ec + row_e[b * SL_R + q] - 68);
             if (row < A.rows.n) lam[q] = y;
             else if (row < n) A.rows.mus[(int64_t)(row - A.rows.n) * C + dg] = y;
           }
