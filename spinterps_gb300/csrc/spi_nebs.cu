@@ -65,7 +65,7 @@ __device__ __forceinline__ void sort_ints(int* a, int n) {
 constexpr int NEB_T = 128;      // threads per CTA
 constexpr int NEB_TILE = 1024;  // stations per shared-memory tile
 constexpr float NEB_REL = 1.00001f;
-constexpr float NEB_ABS = 9.5367431640625e-07f;  // 2^-20
+constexpr float NEB_ABS = 0x1p-20f;
 
 struct NebCell {
   double x, y;
@@ -111,22 +111,55 @@ __device__ __forceinline__ float4 neb_stn(const float4* tile, const double* rx, 
   return make_float4(xs, ys, fabsf(xs) + fabsf(ys), 0.0f);
 }
 
-// The k nearest by (FP64 distance, index) over the stations within u (k_neb_nrst),
-// or over every station (u < 0).
-__device__ __noinline__ void neb_nrst_exact(const NebCell& c, const float4* tile,
-                                            const double* rx, const double* ry, int n_ref, int k,
-                                            float u, int32_t* out) {
+// Candidates of one destination that its warp puts in order together.
+constexpr int NEB_CAND = 128;
+struct NebCand {
+  double d[NEB_CAND];
+  int j[NEB_CAND], key[NEB_CAND];
+};
+// lane src's destination, to every lane
+__device__ __forceinline__ NebCell neb_share(const NebCell& c, int src) {
+  NebCell o;
+  o.x = __shfl_sync(0xffffffffu, c.x, src);
+  o.y = __shfl_sync(0xffffffffu, c.y, src);
+  o.xc = __shfl_sync(0xffffffffu, c.xc, src);
+  o.yc = __shfl_sync(0xffffffffu, c.yc, src);
+  o.sc = __shfl_sync(0xffffffffu, c.sc, src);
+  return o;
+}
+// Appends the lanes' hits in lane order; n: their number so far.
+__device__ __forceinline__ void neb_append(NebCand& w, bool hit, int j, int key, int& n) {
+  const int lane = threadIdx.x % 32;
+  const unsigned m = __ballot_sync(0xffffffffu, hit);
+  const int at = n + __popc(m & ((1u << lane) - 1));
+  if (hit && at < NEB_CAND) {
+    w.j[at] = j;
+    w.key[at] = key;
+  }
+  n += __popc(m);
+}
+// The k candidates (ascending j) of the smallest place, in ascending order.
+template <typename F>
+__device__ __forceinline__ void neb_take(const NebCand& w, int n, int k, int32_t* o, F place) {
+  const int lane = threadIdx.x % 32;
+  int cnt = 0;
+  for (int e0 = 0; e0 < n; e0 += 32) {
+    const int e = e0 + lane;
+    const bool sel = e < n && place(e) < k;
+    const unsigned m = __ballot_sync(0xffffffffu, sel);
+    if (sel) o[cnt + __popc(m & ((1u << lane) - 1))] = w.j[e];
+    cnt += __popc(m);
+  }
+}
+
+// The k nearest by (FP64 distance, index) over every station.
+__device__ __noinline__ void neb_nrst_exact(const NebCell& c, const double* rx, const double* ry,
+                                            int n_ref, int k, int32_t* out) {
   double ld[NEB_MAX];
   int li[NEB_MAX];
   int len = 0;
-  for (int j = 0; j < n_ref; ++j) {
-    if (u >= 0.0f) {
-      const float4 s = neb_stn(tile, rx, ry, n_ref, j);
-      const float lim = fmaf(NEB_ABS, s.z + c.sc, u);
-      if (!(neb_d2(c, s) <= lim * lim)) continue;
-    }
+  for (int j = 0; j < n_ref; ++j)
     neb_insert(ld, li, &len, k, dist_f64(c.x, c.y, rx[j], ry[j]), j);
-  }
   sort_ints(li, len);
   for (int q = 0; q < k; ++q) out[q] = li[q];
 }
@@ -140,13 +173,16 @@ __device__ __noinline__ void neb_nrst_exact(const NebCell& c, const float4* tile
 //   U (1 + 1e-5) + 2^-20 (|x_s| + |y_s| + |x_c| + |y_c|)
 // is none of the k. The second scan writes the others out as they come, in
 // ascending index; where they are exactly k they are the answer, whatever
-// their order, else (a tie within the rounding) they are put in order by
-// their FP64 distances; where a coordinate is not finite or beyond the
-// bounds' range, every station is.
+// their order, else (a tie within the rounding) the destination's warp puts
+// them in order by their FP64 distances, a candidate to a lane; where a
+// coordinate is not finite or beyond the bounds' range, every station is, by
+// the destination's thread.
 //
-// Bound by the scans' instructions. FP64 insertion lists in local memory
-// took 13.0 ms for 13 selections of 16 of 750 stations at 62 500
-// destinations; 13 x 0.27 ms now (750 stations), 40% of the issue slots used.
+// Bound by the scans' latency (about 13 warps to an SM at 62 500
+// destinations). 16 of 750 stations there: 1.06 ms with FP64 insertion lists
+// in local memory, 0.27 with these lists and ties left to a thread, 0.076 now.
+// Four threads to a destination take longer (0.33): four lists make more
+// insertions than one.
 template <int K>
 __global__ __launch_bounds__(NEB_T) void k_neb_nrst(const double* __restrict__ dx_,
                                                     const double* __restrict__ dy_,
@@ -155,6 +191,7 @@ __global__ __launch_bounds__(NEB_T) void k_neb_nrst(const double* __restrict__ d
                                                     const double* __restrict__ ry, int n_ref,
                                                     int k, int32_t* __restrict__ out) {
   __shared__ float4 tile[NEB_TILE];
+  __shared__ NebCand cand[NEB_T / 32];
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const bool act = i < n_dst;
   const double ox = rx[0], oy = ry[0];
@@ -196,7 +233,37 @@ __global__ __launch_bounds__(NEB_T) void k_neb_nrst(const double* __restrict__ d
       }
     }
   }
-  if (act && (!ok || cnt != k)) neb_nrst_exact(c, tile, rx, ry, n_ref, k, ok ? u : -1.0f, o);
+  // (a thread alone took three times as long over its candidates as the whole
+  // scan, and held its CTA's place: half of the kernel's time)
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  NebCand& w = cand[warp];
+  for (unsigned tie = __ballot_sync(0xffffffffu, ok && cnt != k && cnt <= NEB_CAND); tie;
+       tie &= tie - 1) {
+    const int src = __ffs((int)tie) - 1;
+    const NebCell b = neb_share(c, src);
+    const float ub = __shfl_sync(0xffffffffu, u, src);
+    int n = 0;
+    for (int j0 = 0; j0 < n_ref; j0 += 32) {
+      bool hit = false;
+      if (j0 + lane < n_ref) {
+        const float4 s = neb_stn(tile, rx, ry, n_ref, j0 + lane);
+        const float lim = fmaf(NEB_ABS, s.z + b.sc, ub);
+        hit = neb_d2(b, s) <= lim * lim;
+      }
+      neb_append(w, hit, j0 + lane, 0, n);
+    }
+    n = min(n, NEB_CAND);
+    __syncwarp();
+    for (int e = lane; e < n; e += 32) w.d[e] = dist_f64(b.x, b.y, rx[w.j[e]], ry[w.j[e]]);
+    __syncwarp();
+    neb_take(w, n, k, out + (i - lane + src) * k, [&](int e) {
+      int r = 0;
+      for (int f = 0; f < n; ++f) r += neb_less(w.d[f], f, w.d[e], e);
+      return r;
+    });
+    __syncwarp();
+  }
+  if (act && (!ok || cnt > NEB_CAND)) neb_nrst_exact(c, rx, ry, n_ref, k, o);
 }
 
 // a station's pie by the reference's rules in FP64
@@ -235,27 +302,15 @@ __device__ __forceinline__ int neb_pie(const NebCell& c, float4 s, const double*
   return neb_pie_f64(c.x, c.y, rx[j], ry[j], n_pies);
 }
 
-// The rule in FP64 over the stations within their pie's limit (lims, a
-// thread's slots; k_neb_pie), or over every station (null).
-__device__ __noinline__ void neb_pie_exact(const NebCell& c, const float4* tile,
-                                           const double* rx, const double* ry, int n_ref, int k,
-                                           int n_pies, const float* lims, int stride,
-                                           int32_t* out) {
+// The rule in FP64 over every station.
+__device__ __noinline__ void neb_pie_exact(const NebCell& c, const double* rx, const double* ry,
+                                           int n_ref, int k, int n_pies, int32_t* out) {
   double pd[NEB_PIE_SLOTS];
   int pi_[NEB_PIE_SLOTS];
   int plen[16];
   for (int p = 0; p < n_pies; ++p) plen[p] = 0;
   for (int j = 0; j < n_ref; ++j) {
-    int p;
-    if (lims) {
-      const float4 s = neb_stn(tile, rx, ry, n_ref, j);
-      const float v = neb_d2(c, s);
-      p = neb_pie(c, s, rx, ry, j, n_pies, v);
-      const float lim = lims[p * stride];
-      if (!(v <= lim * lim)) continue;
-    } else {
-      p = neb_pie_f64(c.x, c.y, rx[j], ry[j], n_pies);
-    }
+    const int p = neb_pie_f64(c.x, c.y, rx[j], ry[j], n_pies);
     neb_insert(pd + p * k, pi_ + p * k, &plen[p], k, dist_f64(c.x, c.y, rx[j], ry[j]), j);
   }
   // the first k by (rank within pie, distance, index)
@@ -291,12 +346,14 @@ __device__ __noinline__ void neb_pie_exact(const NebCell& c, const float4* tile,
 // the second scan writes out the stations up to it plus the rounding's
 // bound, in ascending index. Where these are exactly k they are the answer.
 // Where they are not, or where the last rank's cut falls between two
-// distances closer than the bound, the rule is put to the stations of the
-// ranks up to the last one in FP64; to every station where the ranks kept
-// don't suffice, or the coordinates are out of the bounds' range.
+// distances closer than the bound, the destination's warp puts the rule to
+// the stations of the ranks up to the last one in FP64, a candidate to a
+// lane; the destination's thread puts it to every station where the ranks
+// kept don't suffice, or the coordinates are out of the bounds' range.
 //
-// FP64 angles and lists in local memory took 20.2 ms for 13 selections of 12
-// of 270 stations in 8 pies at 20 083 destinations, 13 x 0.33 ms now.
+// 12 of 270 stations in 8 pies at 20 083 destinations (a warp to a scheduler,
+// all latency): 1.6 ms with FP64 angles and lists in local memory, 0.33 with
+// undecided destinations left to a thread, 0.21 now.
 constexpr int NEB_LISTS = 192;  // values a thread keeps: at most 104 KB a CTA
 
 __global__ __launch_bounds__(NEB_T) void k_neb_pie(const double* __restrict__ dx_,
@@ -307,6 +364,7 @@ __global__ __launch_bounds__(NEB_T) void k_neb_pie(const double* __restrict__ dx
                                                    int k, int n_pies, int R,
                                                    int32_t* __restrict__ out) {
   __shared__ float4 tile[NEB_TILE];
+  __shared__ NebCand cand[NEB_T / 32];
   extern __shared__ float pies[];  // [n_pies][R + 1][NEB_T]
   float* near = pies + threadIdx.x;
   const int R1 = R + 1;  // (slot R: the limits)
@@ -393,18 +451,66 @@ __global__ __launch_bounds__(NEB_T) void k_neb_pie(const double* __restrict__ dx
       }
     }
   }
-  if (act && (!ok || cnt != k)) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  NebCand& w = cand[warp];
+  const bool undecided = act && (!ok || cnt != k);
+  if (undecided && in_lists)
     // the stations that may be of a rank up to r, or (whole ranks only) of one
     // below it
-    if (in_lists)
-      for (int p = 0; p < n_pies; ++p) {
-        float* l = near + p * (R1 * NEB_T);
-        const float v = l[(left > 0 ? r : max(r - 1, 0)) * NEB_T];
-        l[R * NEB_T] = v < INFINITY ? fmaf(sqrtf(v) * NEB_REL, NEB_REL, slack) : INFINITY;
+    for (int p = 0; p < n_pies; ++p) {
+      float* l = near + p * (R1 * NEB_T);
+      const float v = l[(left > 0 ? r : max(r - 1, 0)) * NEB_T];
+      l[R * NEB_T] = v < INFINITY ? fmaf(sqrtf(v) * NEB_REL, NEB_REL, slack) : INFINITY;
+    }
+  __syncwarp();
+  bool done = !undecided;
+  for (unsigned tie = __ballot_sync(0xffffffffu, undecided && in_lists); tie; tie &= tie - 1) {
+    const int src = __ffs((int)tie) - 1;
+    const NebCell b = neb_share(c, src);
+    const float* lims = near - lane + src + R * NEB_T;
+    int n = 0;
+    for (int j0 = 0; j0 < n_ref; j0 += 32) {
+      bool hit = false;
+      int p = 0;
+      if (j0 + lane < n_ref) {
+        const float4 s = neb_stn(tile, rx, ry, n_ref, j0 + lane);
+        const float v = neb_d2(b, s);
+        p = neb_pie(b, s, rx, ry, j0 + lane, n_pies, v);
+        const float lim = lims[p * (R1 * NEB_T)];
+        hit = v <= lim * lim;
       }
-    neb_pie_exact(c, tile, rx, ry, n_ref, k, n_pies, in_lists ? near + R * NEB_T : nullptr,
-                  R1 * NEB_T, o);
+      neb_append(w, hit, j0 + lane, p, n);
+    }
+    if (n > NEB_CAND) continue;
+    if (lane == src) done = true;
+    __syncwarp();
+    for (int e = lane; e < n; e += 32) w.d[e] = dist_f64(b.x, b.y, rx[w.j[e]], ry[w.j[e]]);
+    __syncwarp();
+    // the pie becomes the rank in it
+    int rank[NEB_CAND / 32];
+#pragma unroll
+    for (int q = 0; q < NEB_CAND / 32; ++q) {
+      const int e = q * 32 + lane;
+      rank[q] = 0;
+      if (e < n)
+        for (int f = 0; f < n; ++f)
+          rank[q] += w.key[f] == w.key[e] && neb_less(w.d[f], f, w.d[e], e);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NEB_CAND / 32; ++q)
+      if (q * 32 + lane < n) w.key[q * 32 + lane] = rank[q];
+    __syncwarp();
+    neb_take(w, n, k, out + (i - lane + src) * k, [&](int e) {
+      int at = 0;
+      for (int f = 0; f < n; ++f)
+        at += w.key[f] < w.key[e] ||
+              (w.key[f] == w.key[e] && neb_less(w.d[f], f, w.d[e], e));
+      return at;
+    });
+    __syncwarp();
   }
+  if (!done) neb_pie_exact(c, rx, ry, n_ref, k, n_pies, o);
 }
 
 // Rows of neighbour lists into a hash table of row indices (open addressing,
