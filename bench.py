@@ -350,10 +350,14 @@ def measured_peaks():
 # (fma_peak_tflops).
 KERNEL_BOUND = {
     "var_tc": ("tensor", "spi::k_var_tc (tcgen05 TF32 OK-variance contraction, 5 MMAs per product)"),
-    "var_df": ("fp32", "spi::k_var_df (double-float OK-variance contraction, FP32 pipe)"),
-    "cells_fp32": ("fp32", "spi::k_krige_cells<float> (FP32 tier: estimates, sum check)"),
-    "cells_fp64": ("fp64", "spi::k_krige_cells<double> (FP64 tier: ill-conditioned and "
-                           "routed systems, the plain path's kernel)"),
+    "var_df": ("tensor", "spi::k_sl_gemm (OK variance of the ill-conditioned systems: FP64 as 36 "
+                         "exact FP16 slice products, tcgen05); spi::k_var_df for variograms "
+                         "without that form"),
+    "cells_fp32": ("fp32", "spi::k_krige_cells_stream<float> (FP32 tier: estimates, sum check)"),
+    # (against the FP64 pipe's rate, which the sliced products pass: over 1)
+    "cells_fp64": ("fp64", "spi::k_sl_gemm (FP64 as 36 exact FP16 slice products, tcgen05); "
+                           "spi::k_krige_cells<double> for exact-inverse systems and "
+                           "variograms without that form"),
     "idw": ("fp32", "spi::k_idw (FP64 path) / spi::k_idw_tc (mixed path: tcgen05 masked GEMM "
                     "pair)"),
 }
@@ -395,7 +399,9 @@ def roofline_for(name, k):
     bf16, hbm, src = measured_peaks()
     bound, kernel = KERNEL_BOUND[name]
     if bound == "tensor":
-        peak, psrc = bf16, src + " (bf16 dense; the kernel runs 5 TF32 MMAs per product: a0b0 + a0b1 + a1b0 + a0b2 + a1b1)"
+        peak, psrc = bf16, src + (
+            " (bf16 dense; the kernel runs 5 TF32 MMAs per product: a0b0 + a0b1 + a1b0 + a0b2 + "
+            "a1b1)" if name == "var_tc" else " (bf16 dense; 36 FP16 products per FP64 product)")
     elif bound == "fp64":
         peak, psrc = fma_peak_tflops(True), "measured FP64 FMA rate (spi_peak_fma, bench.py)"
     else:
@@ -1079,8 +1085,10 @@ def run_legacy(args):
                        "l2": "outputs (1.6 GB per step) exceed L2"},
             "e2e": {"value": n_out / t_e2e, "unit": "points/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h},
-            "gpu_launches": 4 * args.steps,
-            "roofline": {"bound": "fp64", "kernel": "spi::k_leg_lambda (lambda = P r, FP64)",
+            # the system's five kernels, the points' nine
+            "gpu_launches": 14 * args.steps,
+            "roofline": {"bound": "fp64", "kernel": "spi::k_sl_gemm (lambda = P r as exact "
+                                                    "sliced products; over 1 of the FP64 pipe)",
                          "achieved": flop / (ms / 1e3) / 1e12, "peak": fma_peak_tflops(True),
                          "unit": "TFLOP/s",
                          "frac": flop / (ms / 1e3) / 1e12 / fma_peak_tflops(True),

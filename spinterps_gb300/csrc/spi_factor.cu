@@ -10,9 +10,10 @@
 // Lagrange / drift rows are handled by a Schur complement S = F'A^-1 F.
 //
 // GB300's FP64 pipe is narrow (about 2 DFMA per SM per clock), so these
-// kernels are FP64-issue bound, not memory bound: one CTA per system, tiles
-// staged in shared memory, and every operand read from L2 at most once per
-// 32-wide block of FMAs.
+// kernels are FP64-issue bound, not memory bound. The factor and its inverse
+// (spi_chol.cu) and the dual vectors (spi_duals.cu) spread over the GPU; the
+// assembly, the drift check, the exact inverse of small systems and the host
+// side are here.
 #include "spi_common.cuh"
 #include "spi_factor.cuh"
 #include "spi_gj.cuh"
