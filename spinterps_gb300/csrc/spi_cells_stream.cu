@@ -25,12 +25,14 @@
 // One cell to a lane and 16 warps to an SM left every second issue slot
 // empty, waiting on the chain of one entry: two cells to a lane, 32 warps
 // (the FP64 totals in shared memory, the entries without a pair form out of
-// line; what still spills at 64 registers lies outside the loop), one
-// branch for both cells' cuts and the usual passes' vectors known at
-// compile time. 8 systems of 2900 stations, 10^6 cells, 4 vectors: 203 ms
-// as double-floats, 90 with the pairs, 72.5 with 32 warps; 8 of 750
-// stations, 250 000 cells: 33, 19.4, 17.4 ms. (Three CTAs of 80 registers
-// are as fast on large grids, a sixth slower on small systems.)
+// line), one branch for both cells' cuts, which leaves the inner loop for the
+// exact form, and the usual passes' vectors known at compile time. 8 systems
+// of 2900 stations, 10^6 cells, 4 vectors: 203 ms as double-floats, 90 with
+// the pairs, 72.5 with 32 warps, 66.5 with the exact form outside the loop
+// (85% of the issue slots used before that, 109 instructions an entry, some
+// of them spills); 8 of 750 stations, 250 000 cells: 33, 19.4, 17.4, 17.0
+// ms. (Three CTAs of 80 registers take 6% longer on large grids, a fifth on
+// small systems.)
 #include <type_traits>
 
 #include "spi_cells.cuh"
@@ -60,7 +62,9 @@ inline __device__ __noinline__ df stream_general(const CellsArgs& A, const spi_v
 // two cells share the loads, and their chains overlap.
 // CODE: the single structure's model (rho_pair, in units of its sill), or -1.
 // SK's entries at or below the cut are zero, OK's / EDK's past it the whole
-// sill; entries near it take the exact form (rho_cut). NP, NV: np and nv
+// sill; entries near it take the exact form (rho_cut), for which the warp
+// leaves the inner loop: a call inside it would hold the loop's registers to
+// those a call preserves. NP, NV: np and nv
 // where they are known at compile time, or -1.
 template <int CODE, bool SK, bool TRACK, int NP, int NV>
 __device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t* vgp,
@@ -72,38 +76,9 @@ __device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t*
                                              float (&ph)[SSV][2], float (&pl)[SSV][2],
                                              NearDf (&nf)[2], int j0, float esp) {
   const float lo = ko.lo, hi = ko.hi;
-  for (int jj = warp; jj < nj; jj += SNW) {
-    const float4 sp = s_sp[jj];
-    df c[2];
-    if constexpr (CODE < 0) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const df d2 = df_dist2(cp[u], sp);
-        if constexpr (TRACK) nf[u].add(d2, j0 + jj, esp);
-        c[u] = stream_general(A, vgp, kd, SK, sh, d2, gc[u], idxc + jj);
-      }
-    } else {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const df s = dist2_pair(cp[u], sp);
-        if constexpr (TRACK) nf[u].add(s, j0 + jj, esp);
-        c[u] = rho_pair<CODE>(ko, s, tab);
-        if constexpr (SK) {
-          const bool z = c[u].h < lo;
-          c[u].h = z ? 0.f : c[u].h;
-          c[u].l = z ? 0.f : c[u].l;
-        }
-      }
-      // (one branch for both cells)
-      if (SK ? (c[0].h >= lo && c[0].h <= hi) || (c[1].h >= lo && c[1].h <= hi)
-             : fmaxf(c[0].h, c[1].h) >= hi) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-          if (SK ? c[u].h >= lo && c[u].h <= hi : c[u].h >= hi)
-            c[u] = rho_cut(A.dom, vgp, kd, ko, SK, sh, gc[u], idxc + jj, c[u]);
-      }
-    }
-    if constexpr (NV >= 0) np = NP, nv = NV;
+  if constexpr (NV >= 0) np = NP, nv = NV;
+  // an entry pair against the vectors
+  auto take = [&](const df (&c)[2], int jj) {
 #pragma unroll
     for (int v = 0; v < SSV; ++v) {
       if (v >= nv) continue;
@@ -122,6 +97,51 @@ __device__ __forceinline__ void stream_chunk(const CellsArgs& A, const spi_vg_t*
           ph[v][u] = s2.h;
           pl[v][u] += s2.l + e;
         }
+      }
+    }
+  };
+  if constexpr (CODE < 0) {
+    for (int jj = warp; jj < nj; jj += SNW) {
+      df c[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const df d2 = df_dist2(cp[u], s_sp[jj]);
+        if constexpr (TRACK) nf[u].add(d2, j0 + jj, esp);
+        c[u] = stream_general(A, vgp, kd, SK, sh, d2, gc[u], idxc + jj);
+      }
+      take(c, jj);
+    }
+  } else {
+    int jj = warp;
+    while (jj < nj) {
+      df c[2];
+      bool cut = false;
+      for (; jj < nj; jj += SNW) {
+        const float4 sp = s_sp[jj];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const df s = dist2_pair(cp[u], sp);
+          if constexpr (TRACK) nf[u].add(s, j0 + jj, esp);
+          c[u] = rho_pair<CODE>(ko, s, tab);
+          if constexpr (SK) {
+            const bool z = c[u].h < lo;
+            c[u].h = z ? 0.f : c[u].h;
+            c[u].l = z ? 0.f : c[u].l;
+          }
+        }
+        // (one branch for both cells, and out of the loop for the exact form)
+        cut = SK ? (c[0].h >= lo && c[0].h <= hi) || (c[1].h >= lo && c[1].h <= hi)
+                 : fmaxf(c[0].h, c[1].h) >= hi;
+        if (__any_sync(0xffffffffu, cut)) break;
+        take(c, jj);
+      }
+      if (jj < nj) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (SK ? c[u].h >= lo && c[u].h <= hi : c[u].h >= hi)
+            c[u] = rho_cut(A.dom, vgp, kd, ko, SK, sh, gc[u], idxc + jj, c[u]);
+        take(c, jj);
+        jj += SNW;
       }
     }
   }

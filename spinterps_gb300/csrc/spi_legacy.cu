@@ -129,7 +129,7 @@ __global__ __launch_bounds__(LT) void k_leg_system(int sk, const double* __restr
 // microseconds. The operations are those of gj_invert in its order, so the
 // inverse is the same to the last bit. The pivots sit in the distance array,
 // filled last; *status holds 0, or the failing step + 1.
-constexpr int LS_MIN_M = 96;  // below, 2 m launches outlast the one CTA (2.4 ms at 96)
+constexpr int LS_MIN_M = 96;  // below, k_leg_gj takes longer than the one CTA (0.60 and 0.53 ms a call at 64, the same at 96)
 
 __global__ void k_leg_fill(int sk, const double* __restrict__ xi, const double* __restrict__ yi,
                            int n, const double* __restrict__ si, int m, spi_vg_t vg,
