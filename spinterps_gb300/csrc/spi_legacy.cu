@@ -15,8 +15,9 @@
 //
 // Kernels: the distances, the matrix and its Gauss-Jordan inverse in place of
 // numpy.linalg.pinv (k_leg_system, one CTA, for small matrices; else k_leg_fill
-// .. k_leg_dists, every elimination step spread over the GPU); k_leg_rhs
-// (every point's right-hand side, grid-stride); lambda = P r for every point
+// .. k_leg_dists, the elimination over the GPU in one cooperative launch,
+// k_leg_gj, or step by step); every point's right-hand side (k_leg_rhs_fx in
+// integers, k_leg_rhs in FP64); lambda = P r for every point
 // as sliced tensor-core products (spi_slices.cu; without their scratch
 // k_leg_lambda, an FP64 tiled contraction); k_leg_finish (a warp per point:
 // estimate, variance, indicator).
