@@ -894,14 +894,20 @@ extern "C" int spi_vg_de(int32_t n_prob, const spi_de_problem_t* prob, const int
   if (n_prob == 0) return SPI_OK;
   if (!prob || !bin_off || !n_bins || !bin_h || !bin_g || !best_x || !best_f || !n_gen)
     return SPI_ERR_ARG;
-  if (n_prob > INT32_MAX / DE_CL) return SPI_ERR_TOO_LARGE;
   const size_t smem = sizeof(DeSmem);
   if (cudaFuncSetAttribute(k_de, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return SPI_ERR_CUDA;
-  DeArgs A{n_prob, prob, bin_off, n_bins, bin_h, bin_g, maxiter, tol, best_x, best_f, n_gen};
-  k_de<<<n_prob * DE_CL, DE_T, smem, (cudaStream_t)stream>>>(A);
-  SPI_LAUNCH_CHECK();
+  // (as many problems at a time as a grid of clusters holds)
+  constexpr int32_t kMax = INT32_MAX / DE_CL;
+  for (int32_t q0 = 0; q0 < n_prob;) {
+    const int32_t nq = n_prob - q0 < kMax ? n_prob - q0 : kMax;
+    DeArgs A{nq, prob + q0, bin_off, n_bins, bin_h, bin_g, maxiter, tol,
+             best_x + (int64_t)q0 * 4, best_f + q0, n_gen + q0};
+    k_de<<<nq * DE_CL, DE_T, smem, (cudaStream_t)stream>>>(A);
+    SPI_LAUNCH_CHECK();
+    q0 += nq;
+  }
   return SPI_OK;
 }
 
