@@ -81,10 +81,19 @@ __global__ __launch_bounds__(LT) void k_leg_system(int sk, const double* __restr
   const int m = n + a;
   for (int64_t e = tid; e < (int64_t)m * m; e += LT) {
     const int i = (int)(e / m), j = (int)(e - (int64_t)i * m);
-    const double val = leg_entry(sk, xi, yi, n, si, vg, i, j);
+    double val = 0.0;
     if (i < n && j < n) {
-      const int lo = min(i, j), hi = max(i, j);
-      dists[(int64_t)i * n + j] = i == j ? 0.0 : dist_f64(xi[lo], yi[lo], xi[hi], yi[hi]);
+      // (leg_entry with the distance kept: a second root took 40 us at m = 91)
+      double d = 0.0;
+      if (i != j) {
+        const int lo = min(i, j), hi = max(i, j);
+        d = dist_f64(xi[lo], yi[lo], xi[hi], yi[hi]);
+        const double g = leg_gamma(vg, d);
+        val = sk ? -g : g;
+      }
+      dists[(int64_t)i * n + j] = d;
+    } else {
+      val = leg_entry(sk, xi, yi, n, si, vg, i, j);
     }
     lhs[e] = val;
     inv[e] = val;

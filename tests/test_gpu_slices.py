@@ -89,12 +89,13 @@ def test_double_float_tier():
 
 @pytest.mark.parametrize("kind", ["OK", "SK", "EDK"])
 @pytest.mark.parametrize("n,C", [(63, 600), (64, 513), (95, 640), (96, 700), (127, 515), (200, 900)])
-def test_single_neighbourhood(kind, n, C):
+def test_single_neighbourhood(kind, n, C, monkeypatch):
     """The classes' weights as sliced products and their matrix inverted step
     by step over the GPU, against the oracle's restatement of the classes:
     1e-9 of each array's largest value (condition up to 1e5)."""
     import torch
     from spinterps_gb300 import legacy
+    monkeypatch.setattr(legacy, "SLICES_MIN_WORK", 0)
     rng = np.random.default_rng(n)
     xi, yi, zi = rng.uniform(0, 1e5, n), rng.uniform(0, 1e5, n), rng.gamma(1.2, 3.0, n)
     xk, yk = rng.uniform(0, 1e5, C), rng.uniform(0, 1e5, C)
@@ -116,13 +117,14 @@ def test_single_neighbourhood(kind, n, C):
                                    "0.3 Nug(0.0) + 1.2 Gau(9000)", "1.0 Lin(50000)",
                                    "0.2 Nug(0.0) + 0.5 Exp(9000) + 0.7 Sph(50000)",
                                    "0.5 Exp(1e-5)", "0.7 Hol(20000)", "1.0 Pow(1.2)", "2.0 Nug(0.0)"])
-def test_single_neighbourhood_right_hand_sides(kind, model):
+def test_single_neighbourhood_right_hand_sides(kind, model, monkeypatch):
     """Fixed-point right-hand sides (512 points on) against the FP64 formulas
     (the same points 511 at a time), coinciding pairs included, also a
     distance of an ulp. Either evaluation rounds a structure at most about 8
     times at up to 1.5 times its sill: 16 * 2^-53 of the sills, twice."""
     import torch
     from spinterps_gb300 import legacy
+    monkeypatch.setattr(legacy, "SLICES_MIN_WORK", 0)
     n, C = 97, 1500
     rng = np.random.default_rng(5)
     xi, yi, zi = 4e6 + rng.uniform(0, 1e5, n), 5e6 + rng.uniform(0, 1e5, n), rng.gamma(1.2, 3.0, n)
