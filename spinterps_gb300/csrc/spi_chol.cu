@@ -23,6 +23,8 @@
 // mirrored (upper) block, so the inverse may overwrite its factor.
 #include <cooperative_groups.h>
 
+#include <utility>
+
 #include "spi_factor.cuh"
 
 namespace cg = cooperative_groups;
@@ -452,6 +454,9 @@ __global__ __cluster_dims__(CC, 1, 1) __launch_bounds__(CTH) void k_trinv_cond(
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   __shared__ double red[CTH / 32];
   __shared__ double part[CC];
+  cg::cluster_group cl = cg::this_cluster();
+  // (CTA 0 runs before another CTA stores into its shared memory)
+  auto started = cl.barrier_arrive();
   const int nw = CC * (CTH / 32), w0 = rank * (CTH / 32) + warp;
   const double t = cond_rows<T>(X, n, s, probes, w0, nw);
   if (!probes)
@@ -459,7 +464,7 @@ __global__ __cluster_dims__(CC, 1, 1) __launch_bounds__(CTH) void k_trinv_cond(
       for (int j = i + 1 + lane; j < n; j += 32) X[(int64_t)i * n + j] = T(0);
   if (lane == 0) red[warp] = t;
   __syncthreads();
-  cg::cluster_group cl = cg::this_cluster();
+  cl.barrier_wait(std::move(started));
   if (tid == 0) {
     double f = 0.0;
     for (int w = 0; w < CTH / 32; ++w) f += red[w];
