@@ -410,7 +410,7 @@ struct SlSmem {
   FxVg vg;
   int list[SL_CAP];
   int nact;
-  uint64_t afull[SL_ST], bfull[SL_ST], empty[SL_ST], chunk, drained;
+  uint64_t afull[SL_ST], bfull[SL_ST], empty[SL_ST], chunk, drained, quit;
   uint32_t tbase;
   int fail, any_bad;
 };
@@ -623,6 +623,7 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
     }
     mbar_init(smem_u32(&S.chunk), 1);
     mbar_init(smem_u32(&S.drained), SL_W);
+    mbar_init(smem_u32(&S.quit), 1);
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   if (tid >= 64 && tid < 64 + 256) S.tab[tid - 64] = fx_exp2_entry(tid - 64);
@@ -646,6 +647,7 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
   const int sk = MODE == kKrige && A.sys.kind == SPI_KIND_SK;
   int g = 0;     // stages of the earlier items (every role counts them alike)
   int nch = 0;   // their chunks (drains)
+  int issued = 0;  // copies issued (the copying thread's)
   bool ok = true;
 
   for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
@@ -669,6 +671,7 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
             tc_bulk_load(smem_u32(ring + st * SL_STAGE + SL_A_BYTES),
                          reinterpret_cast<const float*>(src), SL_B_BYTES,
                          smem_u32(&S.bfull[st]));
+            issued = f + 1;
           }
       }
       ok = __shfl_sync(0xffffffffu, (int)ok, 0);
@@ -1022,14 +1025,16 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
   }
   __syncthreads();
   if (S.fail) {
-    if (tid == 0) {
-      atomicExch(A.err, 1);
-      // copies and MMAs that may still be in flight: one more bounded wait
-      // each, by parity, before the columns are freed
-      for (int q = 0; q < SL_ST; ++q)
-        for (uint32_t ph = 0; ph < 2; ++ph) mbar_wait_bounded(smem_u32(&S.bfull[q]), ph);
-      tc_commit(smem_u32(&S.chunk));
-      for (uint32_t ph = 0; ph < 2; ++ph) mbar_wait_bounded(smem_u32(&S.chunk), ph);
+    if (tid == 0) atomicExch(A.err, 1);
+    // what is still in flight, one more bounded wait each: every stage's last
+    // copy, and the MMAs, whose completion only a commit of the thread that
+    // issued them signals
+    if (warp == SL_W + 1 && lane == 0)
+      for (int f = max(0, issued - SL_ST); f < issued; ++f)
+        mbar_wait_bounded(smem_u32(&S.bfull[f % SL_ST]), (uint32_t)(f / SL_ST) & 1u);
+    if (warp == SL_W && lane == 0) {
+      tc_commit(smem_u32(&S.quit));
+      mbar_wait_bounded(smem_u32(&S.quit), 0);
     }
     __syncthreads();
   }
