@@ -456,13 +456,13 @@ int spi_krige_var_df(const spi_domain_t *dom, const spi_systems_t *sys,
 /* The precision-0 pass of spi_krige_cells_tiled (route_filter 0 or 2) with
  * the contractions (the OK variance, the dual columns, every step's
  * estimates) on the tensor cores as exact products of 8-bit slices: operands
- * of 55 bits, exact sums, FP64 results. Systems it covers: the Cholesky path
+ * of 63 bits, exact sums, FP64 results. Systems it covers: the Cholesky path
  * (SK also on the exact-inverse path) with Exp, Gau, Sph, Lin and Nug
  * structures; the others run as in spi_krige_cells_tiled. max_steps: the
  * most steps of a system of the batch. scratch: device memory of
  * spi_slices_scratch_bytes (want_var 0 for SK; systems beyond it go in
- * groups). err_flag (device): set to 1 when a tensor-core wait ran out, whose
- * cells are then incomplete. */
+ * groups). err_flag (device, 0 on entry): set to 1 when a tensor-core wait
+ * ran out, and the FP64 kernels then compute every system. */
 int spi_krige_cells_sliced(const spi_domain_t *dom, const spi_systems_t *sys,
                            const double *vals, const spi_krige_ws_t *ws, int32_t want_var,
                            int32_t route_filter, double cond_split, const spi_out_t *out,
@@ -470,7 +470,8 @@ int spi_krige_cells_sliced(const spi_domain_t *dom, const spi_systems_t *sys,
                            int64_t scratch_bytes, int32_t *err_flag, spi_stream_t stream);
 
 /* spi_krige_var_df's systems by the same sliced contraction (FP64 accuracy),
- * the double-float kernel for those it does not cover. Requires linv_arena
+ * the double-float kernel for those it does not cover (and, as above, for all
+ * of them after a wait that ran out). Requires linv_arena
  * besides what spi_krige_var_df requires; scratch of spi_slices_scratch_bytes
  * with want_fields 0. */
 int spi_krige_var_sliced(const spi_domain_t *dom, const spi_systems_t *sys,
@@ -845,7 +846,7 @@ int spi_legacy_points(int32_t kind, const double *xi, const double *yi, const do
                       double *lambdas, double *mus, double *zk, double *est, double *ik,
                       spi_stream_t stream);
 
-/* The same with lambda = P r as sliced tensor-core products (55-bit
+/* The same with lambda = P r as sliced tensor-core products (63-bit
  * operands, exact sums). scratch: spi_slices_one_scratch_bytes(m, m), m the
  * matrix's rows; err_flag (device, 0 on entry): set to 1 when a tensor-core
  * wait ran out, and the FP64 kernel then computes the weights. */

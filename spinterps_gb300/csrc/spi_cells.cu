@@ -474,7 +474,7 @@ __device__ __forceinline__ void cells_tile(const CellsArgs& A, int npad, int64_t
 template <typename T, int TC, typename OutT>
 __global__ __launch_bounds__(CT) void k_krige_cells(CellsArgs A, int npad) {
   const int s = blockIdx.y;
-  if (A.skip && A.skip[(int64_t)s * A.skip_stride]) return;
+  if (A.done.has(s)) return;
   // filter 1: well-conditioned Cholesky systems; filter 2: all others
   const bool fast = fp32_tier(A.ws, s, A.cond_split, A.sys.kind == SPI_KIND_SK);
   if ((A.route_filter == 1 && !fast) || (A.route_filter == 2 && fast)) return;
@@ -619,8 +619,6 @@ extern "C" int spi_krige_cells_tiled(const spi_domain_t* dom, const spi_systems_
   A.route_filter = route_filter;
   A.cond_split = cond_split;
   A.out = *out;
-  A.skip = nullptr;
-  A.skip_stride = 0;
   return launch_cells(A, precision, tile, (cudaStream_t)stream);
 }
 
@@ -665,7 +663,7 @@ extern "C" int spi_krige_cells_sliced(const spi_domain_t* dom, const spi_systems
   A.route_filter = route_filter;
   A.cond_split = cond_split;
   A.out = *out;
-  const int rc = launch_slices(c, &A.skip, &A.skip_stride, (cudaStream_t)stream);
+  const int rc = launch_slices(c, &A.done, (cudaStream_t)stream);
   if (rc) return rc;
   return launch_cells(A, 0, tile, (cudaStream_t)stream);
 }

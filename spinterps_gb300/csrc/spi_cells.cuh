@@ -1,6 +1,7 @@
 // Shared by the cell kernels (spi_cells.cu, spi_cells_stream.cu).
 #pragma once
 #include "spi_common.cuh"
+#include "spi_slices.cuh"
 
 namespace spi {
 
@@ -15,9 +16,7 @@ struct CellsArgs {
   int route_filter;
   double cond_split;
   spi_out_t out;
-  // systems already computed (spi_slices.cu): skip[s * skip_stride] != 0
-  const int32_t* skip;
-  int skip_stride;
+  SlicesDone done;  // systems already computed
 };
 
 // Exact (FP64, reference-ordered) nearest station of a cell among a

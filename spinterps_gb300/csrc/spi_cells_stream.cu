@@ -155,7 +155,7 @@ __global__ __launch_bounds__(STC * SNW, sizeof(T) == 4 ? 4 : 2) void k_krige_cel
   const int s = blockIdx.y;
   const int64_t C = A.dom.n_cells;
   const int64_t c0 = (int64_t)blockIdx.x * TC;
-  if (c0 >= C || (A.skip && A.skip[(int64_t)s * A.skip_stride])) return;
+  if (c0 >= C || A.done.has(s)) return;
   const int route = A.ws.route[s];
   {
     const bool fast = fp32_tier(A.ws, s, A.cond_split, A.sys.kind == SPI_KIND_SK);

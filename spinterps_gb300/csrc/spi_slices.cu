@@ -1088,7 +1088,7 @@ int64_t slices_scratch(int max_n, int n_sys, int max_vec, bool var, bool vec) {
   return (int64_t)(p.fixed + p.per_sys * (size_t)grp + 256);
 }
 
-int launch_slices(const SlicesCall& c, const int32_t** use, int* use_stride, cudaStream_t st) {
+int launch_slices(const SlicesCall& c, SlicesDone* done, cudaStream_t st) {
   const int sms = n_sms();
   if (sms <= 0) return SPI_ERR_CUDA;
   const SlPlan p(c.sys.max_n, c.sys.n_sys, c.max_vec, c.want_var, c.want_vec, sms);
@@ -1131,8 +1131,7 @@ int launch_slices(const SlicesCall& c, const int32_t** use, int* use_stride, cud
   A.row_e = reinterpret_cast<int32_t*>(q);
   q += al((size_t)p.rs * 4) * grp;
   A.pack = q;
-  *use = &A.rec[0].use;
-  *use_stride = (int)(sizeof(SlSys) / sizeof(int32_t));
+  *done = SlicesDone{&A.rec[0].use, (int)(sizeof(SlSys) / sizeof(int32_t)), c.err};
   if (cudaMemsetAsync(A.head->mn, 0xff, sizeof(A.head->mn), st) != cudaSuccess ||
       cudaMemsetAsync(A.head->mx, 0, sizeof(A.head->mx), st) != cudaSuccess)
     return SPI_ERR_CUDA;

@@ -6,11 +6,15 @@
 
 namespace spi {
 
-struct Yes {
-  static constexpr bool value = true;
-};
-struct No {
-  static constexpr bool value = false;
+// The systems that a sliced contraction has computed, for the kernel that
+// computes the others: all of them where one of its waits ran out (*err).
+struct SlicesDone {
+  const int32_t* use = nullptr;  // use[s * stride] != 0
+  int stride = 0;
+  const int32_t* err = nullptr;
+  __device__ __forceinline__ bool has(int s) const {
+    return use && use[(int64_t)s * stride] && !*err;
+  }
 };
 
 // Right-hand sides rhs [points, m] against the rows of inv [m, m]: the first
@@ -41,8 +45,6 @@ struct SlicesCall {
 
 int64_t slices_scratch(int max_n, int n_sys, int max_vec, bool var, bool vec);
 
-// Runs the systems that have a sliced form; (*use)[s * *stride] != 0 (on the
-// device, in stream order) marks them, the caller computes the others.
 // The other contraction: *use != 0 (on the device) where it ran, else the
 // caller computes it.
 int64_t slices_scratch_one(int n, int rows);
@@ -54,6 +56,8 @@ int launch_slices_rows(const SlRows& r, void* scratch, int64_t scratch_bytes, in
 int launch_fx_scene(const spi_domain_t& dom, void* scratch, const FxScene** scene,
                     cudaStream_t st);
 
-int launch_slices(const SlicesCall& c, const int32_t** use, int* stride, cudaStream_t st);
+// Runs the systems that have a sliced form; done marks them (on the device, in
+// stream order), the caller computes the others.
+int launch_slices(const SlicesCall& c, SlicesDone* done, cudaStream_t st);
 
 }  // namespace spi

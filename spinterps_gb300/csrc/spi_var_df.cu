@@ -31,9 +31,7 @@ struct VarDfArgs {
   spi_systems_t sys;
   spi_krige_ws_t ws;
   double cond_cap;
-  // systems already computed (spi_slices.cu): skip[s * skip_stride] != 0
-  const int32_t* skip;
-  int skip_stride;
+  SlicesDone done;  // systems already computed
 };
 
 __device__ __forceinline__ bool var_df_system(const spi_krige_ws_t& ws, int s, double cap) {
@@ -57,7 +55,7 @@ __global__ __launch_bounds__(VD_T) void k_var_df(VarDfArgs A) {
   const int64_t C = A.dom.n_cells;
   if (A.sys.kind == SPI_KIND_SK) return;
   if (!var_df_system(A.ws, s, A.cond_cap)) return;
-  if (A.skip && A.skip[(int64_t)s * A.skip_stride]) return;
+  if (A.done.has(s)) return;
   const int64_t soff = A.sys.stn_off[s];
   const int n = (int)(A.sys.stn_off[s + 1] - soff);
   const int32_t* idx = A.sys.stn_idx + soff;
@@ -193,7 +191,7 @@ extern "C" int spi_krige_var_df(const spi_domain_t* dom, const spi_systems_t* sy
   if (sys->n_sys < 0 || sys->n_sys > 65535) return SPI_ERR_TOO_LARGE;
   if (sys->n_sys == 0 || dom->n_cells == 0) return SPI_OK;
   if (int rc = check_var_df(dom, sys, ws)) return rc;
-  return launch_var_df(VarDfArgs{*dom, *sys, *ws, cond_cap, nullptr, 0}, (cudaStream_t)stream);
+  return launch_var_df(VarDfArgs{*dom, *sys, *ws, cond_cap, {}}, (cudaStream_t)stream);
 }
 
 // The same systems' |Linv c|^2 by the sliced tensor-core contraction, the
@@ -217,7 +215,7 @@ extern "C" int spi_krige_var_sliced(const spi_domain_t* dom, const spi_systems_t
   c.scratch = scratch;
   c.scratch_bytes = scratch_bytes;
   c.err = err_flag;
-  VarDfArgs A{*dom, *sys, *ws, cond_cap, nullptr, 0};
-  const int rc = launch_slices(c, &A.skip, &A.skip_stride, (cudaStream_t)stream);
+  VarDfArgs A{*dom, *sys, *ws, cond_cap, {}};
+  const int rc = launch_slices(c, &A.done, (cudaStream_t)stream);
   return rc ? rc : launch_var_df(A, (cudaStream_t)stream);
 }

@@ -1,0 +1,50 @@
+"""Where the sliced tensor-core passes (csrc/spi_slices.cu) hand systems back
+to the FP64 kernels, against those kernels alone (tensor_cores=False)."""
+import numpy as np
+import pytest
+
+pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+EXP = "0.05 Nug(0.0) + 0.95 Exp(20000)"
+
+
+def _job(n, T, C, seed=0):
+    rng = np.random.default_rng(seed)
+    box = 8e3 * np.sqrt(n)
+    sx, sy = rng.uniform(0, box, n), rng.uniform(0, box, n)
+    return sx, sy, 3.0 + rng.normal(size=(T, n)), rng.uniform(0, box, C), rng.uniform(0, box, C)
+
+
+def _plan(job, methods, vg, tensor_cores=True, **kw):
+    from spinterps_gb300 import steps
+    sx, sy, z, cx, cy = job
+    kw.setdefault("est_vars", "OK" in methods)
+    args = steps.interp_args_for(methods, est_vars=kw["est_vars"])
+    kw = dict(dict(min_vg_val=1e-4, intrp_dtype=np.float64), **kw)
+    return steps.InterpPlan(sx, sy, z, cx, cy, [vg] * len(z), args, tensor_cores=tensor_cores, **kw)
+
+
+@pytest.mark.parametrize("precision,vg", [("fp64", EXP),
+                                          ("mixed", "0.00001 Exp(1.0) + 0.9 Gau(25000)")])
+def test_after_a_wait_that_ran_out(precision, vg):
+    """With the error flag up (as a timed-out wait leaves it) every system is
+    computed by the FP64 (double-float) kernels: the same bits as without
+    tensor cores in FP64, the mixed tier's 1e-5 else (its own tensor-core
+    variance stays on)."""
+    job = _job(150, 3, 300)
+    p = _plan(job, ["OK", "SK"], vg, precision=precision)
+    p.slices_err.fill_(1)
+    p.execute()
+    got, plain = p.fields(), _plan(job, ["OK", "SK"], vg, False, precision=precision)
+    plain.execute()
+    want = plain.fields()
+    for lab in want:
+        g, w = (x[lab].cpu().numpy() if hasattr(x[lab], "cpu") else x[lab] for x in (got, want))
+        if precision == "fp64":
+            assert np.array_equal(g, w), lab
+        else:
+            assert np.isfinite(g).all()
+            assert np.abs(g - w).max() <= 1e-5 * np.abs(w).max(), lab
+    with pytest.raises(RuntimeError, match="timed out"):
+        p.collect_info()
