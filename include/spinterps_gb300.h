@@ -483,7 +483,8 @@ int spi_krige_var_sliced(const spi_domain_t *dom, const spi_systems_t *sys,
 int64_t spi_slices_one_scratch_bytes(int32_t n, int32_t rows);
 
 /* Device scratch of spi_krige_cells_sliced (want_fields 1) or
- * spi_krige_var_sliced (want_fields 0) on the current device. */
+ * spi_krige_var_sliced (want_fields 0) on the current device. n_drift: 0 for
+ * OK and SK. */
 int64_t spi_slices_scratch_bytes(int32_t max_n, int32_t n_sys, int32_t max_steps,
                                  int32_t n_drift, int32_t want_var, int32_t want_fields);
 

@@ -650,7 +650,9 @@ extern "C" int spi_krige_cells_sliced(const spi_domain_t* dom, const spi_systems
   c.want_var = want_var && sys->kind != SPI_KIND_SK;
   c.want_vec = 1;
   c.filter = route_filter;
-  c.max_vec = 1 + dom->n_drift + max_steps;
+  // (as dual_rows and spi_slices_scratch_bytes's caller count: a domain with
+  // drifts also serves OK and SK)
+  c.max_vec = (sys->kind == SPI_KIND_SK ? 1 : extra_rows(sys->kind, dom->n_drift)) + max_steps;
   c.scratch = scratch;
   c.scratch_bytes = scratch_bytes;
   c.err = err_flag;

@@ -48,3 +48,20 @@ def test_after_a_wait_that_ran_out(precision, vg):
             assert np.abs(g - w).max() <= 1e-5 * np.abs(w).max(), lab
     with pytest.raises(RuntimeError, match="timed out"):
         p.collect_info()
+
+
+@pytest.mark.parametrize("drifts", [1, 2])
+@pytest.mark.parametrize("T", [62, 63, 127])
+def test_scratch_of_ok_beside_edk(T, drifts):
+    """OK with its variance and EDK in one plan, one shared system: the OK
+    batch's scratch holds its own rows (1 + T: a whole number of blocks of 64
+    at 63 and 127), not the drifts'."""
+    job = _job(70, T, 130)
+    rng = np.random.default_rng(T)
+    kw = dict(stn_drifts=rng.uniform(0, 1, (70, drifts)), cell_drifts=rng.uniform(0, 1, (drifts, 130)))
+    a, b = (_plan(job, ["OK", "EDK"], EXP, tc, **kw) for tc in (True, False))
+    a.execute()
+    b.execute()
+    for lab, w in b.fields().items():
+        g = a.fields()[lab]
+        assert np.isfinite(g).all() and np.abs(g - w).max() <= 1e-11 * np.abs(w).max(), lab
