@@ -138,7 +138,7 @@ __global__ __launch_bounds__(LT) void k_leg_system(int sk, const double* __restr
 // m = 401, where the step-by-step launches below take 2 m launches of a few
 // microseconds. The operations are those of gj_invert in its order, so the
 // inverse is the same to the last bit. The pivots sit in the distance array,
-// filled last; *status holds 0, or the failing step + 1.
+// filled last, where it holds them; *status holds 0, or the failing step + 1.
 constexpr int LS_MIN_M = 96;  // below, k_leg_gj takes longer than the one CTA (0.60 and 0.53 ms a call at 64, the same at 96)
 
 __global__ void k_leg_fill(int sk, const double* __restrict__ xi, const double* __restrict__ yi,
@@ -717,10 +717,12 @@ extern "C" int spi_legacy_system(int32_t kind, const double* xi, const double* y
   const int64_t m = (int64_t)n + (sk ? 0 : 1 + n_drift);
   const size_t smem = (size_t)m * (2 * sizeof(double) + sizeof(int));
   if (smem > 200 * 1024) return SPI_ERR_TOO_LARGE;
-  if (m >= spi::LS_MIN_M) {
+  // (few stations with many drifts: the one CTA)
+  const bool piv_fits = m * (int64_t)sizeof(int32_t) <= (int64_t)n * n * (int64_t)sizeof(double);
+  if (m >= spi::LS_MIN_M && piv_fits) {
     cudaStream_t st = (cudaStream_t)stream;
     const int mi = (int)m;
-    int32_t* piv = reinterpret_cast<int32_t*>(in_dists);  // n^2 doubles >= m ints
+    int32_t* piv = reinterpret_cast<int32_t*>(in_dists);
     const int gx = (int)((m * m + 2047) / 2048);
     spi::k_leg_fill<<<gx, 256, 0, st>>>(sk, xi, yi, n, si, mi, *vg, lhs, lhs_inv, status);
     SPI_LAUNCH_CHECK();
