@@ -83,6 +83,7 @@ constexpr int64_t SL_BAND = 64ll << (FX_BITS - 54);  // units around the min_vg_
 // The launch's device-side header at the start of the scratch.
 struct SlHead {
   unsigned long long mn[2], mx[2];  // ordered encodings of the coordinates' range
+  unsigned long long bad;           // a coordinate is not finite
 };
 
 // What a launch contracts: the kriging systems of a batch; given right-hand
@@ -131,10 +132,15 @@ __device__ __forceinline__ double dec(unsigned long long u) {
   return __longlong_as_double((long long)((u >> 63) ? u & 0x7fffffffffffffffull : ~u));
 }
 
-// The range of all coordinates.
-__global__ __launch_bounds__(256) void k_sl_range(spi_domain_t dom, SlHead* h) {
+// The range of the coordinates of the cells and of the stations in use: those
+// of the systems (stn_off, stn_idx), else all. (A gauge without a value may
+// have any coordinates.)
+__global__ __launch_bounds__(256) void k_sl_range(spi_domain_t dom, const int64_t* stn_off,
+                                                  const int32_t* stn_idx, int n_sys, SlHead* h) {
   unsigned long long mn[2] = {~0ull, ~0ull}, mx[2] = {0, 0};
+  bool bad = false;
   auto take = [&](double x, double y) {
+    bad = bad || !isfinite(x) || !isfinite(y);
     const unsigned long long a = enc(x), b = enc(y);
     mn[0] = min(mn[0], a);
     mx[0] = max(mx[0], a);
@@ -144,8 +150,12 @@ __global__ __launch_bounds__(256) void k_sl_range(spi_domain_t dom, SlHead* h) {
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < dom.n_cells; i += step)
     take(dom.cell_x[i], dom.cell_y[i]);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < dom.n_stns; i += step)
-    take(dom.stn_x[i], dom.stn_y[i]);
+  const int64_t used = stn_idx ? stn_off[n_sys] : dom.n_stns;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < used; i += step) {
+    const int64_t st = stn_idx ? stn_idx[i] : i;
+    take(dom.stn_x[st], dom.stn_y[st]);
+  }
+  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&h->bad, 1ull);
   for (int d = 0; d < 2; ++d) {
     for (int o = 16; o > 0; o >>= 1) {
       mn[d] = min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
@@ -165,23 +175,13 @@ __device__ __forceinline__ int dual_rows(const SlArgs& A, int route) {
 
 // The common grid of the range; false where it has none.
 __device__ bool sl_grid(const SlHead* h, FxGrid& g) {
-  const double x0 = dec(h->mn[0]), x1 = dec(h->mx[0]);
-  const double y0 = dec(h->mn[1]), y1 = dec(h->mx[1]);
-  double ext = fmax(x1 - x0, y1 - y0);
-  g.ox = x0;
-  g.oy = y0;
-  const bool ok = ext >= 0.0 && ext < 1e200 && x0 > -1e250 && y0 > -1e250;
-  if (!(ext > 1e-200)) ext = 1e-200;
-  int e = 0;
-  frexp(ext, &e);
-  g.q = FX_GRID - 1 - e;
-  return ok;
+  return fx_grid(dec(h->mn[0]), dec(h->mx[0]), dec(h->mn[1]), dec(h->mx[1]), g) && !h->bad;
 }
 
 // The grid, and which systems of the launch take this path: on the Cholesky
 // path (SK: also the exact-inverse path, whose estimates contract the same
-// covariances), every structure with a fixed-point form, and in the pass by
-// its filter.
+// covariances), every structure with a fixed-point form that the grid resolves,
+// and in the pass by its filter.
 __global__ __launch_bounds__(256) void k_sl_select(SlArgs A) {
   __shared__ FxGrid g;
   __shared__ int ok;
@@ -202,7 +202,7 @@ __global__ __launch_bounds__(256) void k_sl_select(SlArgs A) {
   if (A.filter == 3) use = use && (A.ws.tier ? A.ws.tier[s] == 2 : fast);
   // (a variogram of nuggets alone has no covariances to contract)
   fx_init(r.vg, A.sys.vg[s], sk, A.dom.min_vg_val, g.q);
-  if (!r.vg.ok || r.vg.n == 0) use = 0;
+  if (!r.vg.ok || r.vg.n == 0 || !fx_resolves(A.sys.vg[s], g.q)) use = 0;
   r.use = use;
   // |y| <= sqrt(sill) for y = Linv c: y / sill in units of 2^unit, 58 bits
   // with 8 times as much room
@@ -1133,9 +1133,9 @@ int launch_slices(const SlicesCall& c, SlicesDone* done, cudaStream_t st) {
   A.pack = q;
   *done = SlicesDone{&A.rec[0].use, (int)(sizeof(SlSys) / sizeof(int32_t)), c.err};
   if (cudaMemsetAsync(A.head->mn, 0xff, sizeof(A.head->mn), st) != cudaSuccess ||
-      cudaMemsetAsync(A.head->mx, 0, sizeof(A.head->mx), st) != cudaSuccess)
+      cudaMemsetAsync(A.head->mx, 0, sizeof(SlHead) - sizeof(A.head->mn), st) != cudaSuccess)
     return SPI_ERR_CUDA;
-  k_sl_range<<<2 * sms, 256, 0, st>>>(c.dom, A.head);
+  k_sl_range<<<2 * sms, 256, 0, st>>>(c.dom, c.sys.stn_off, c.sys.stn_idx, c.sys.n_sys, A.head);
   SPI_LAUNCH_CHECK();
   auto kern = c.out.out_f64 ? k_sl_gemm<kKrige, double> : k_sl_gemm<kKrige, float>;
   if (!smem_opt_in(kern, SL_SMEM)) return SPI_ERR_CUDA;
@@ -1211,9 +1211,9 @@ int launch_fx_scene(const spi_domain_t& dom, void* scratch, const FxScene** scen
   SlHead* h = reinterpret_cast<SlHead*>(q);
   FxScene* o = reinterpret_cast<FxScene*>(q + al(sizeof(SlHead)));
   if (cudaMemsetAsync(h->mn, 0xff, sizeof(h->mn), st) != cudaSuccess ||
-      cudaMemsetAsync(h->mx, 0, sizeof(h->mx), st) != cudaSuccess)
+      cudaMemsetAsync(h->mx, 0, sizeof(SlHead) - sizeof(h->mn), st) != cudaSuccess)
     return SPI_ERR_CUDA;
-  k_sl_range<<<2 * sms, 256, 0, st>>>(dom, h);
+  k_sl_range<<<2 * sms, 256, 0, st>>>(dom, nullptr, nullptr, 0, h);
   k_fx_scene<<<1, 1, 0, st>>>(h, o);
   SPI_LAUNCH_CHECK();
   *scene = o;

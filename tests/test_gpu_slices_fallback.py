@@ -65,3 +65,69 @@ def test_scratch_of_ok_beside_edk(T, drifts):
     for lab, w in b.fields().items():
         g = a.fields()[lab]
         assert np.isfinite(g).all() and np.abs(g - w).max() <= 1e-11 * np.abs(w).max(), lab
+
+
+def _near(got, want, bar=1e-11):
+    for lab, w in want.items():
+        g = got[lab]
+        assert np.array_equal(np.isnan(g), np.isnan(w)), lab
+        if np.isfinite(w).any():
+            assert np.nanmax(np.abs(g - w)) <= bar * np.nanmax(np.abs(w)), lab
+
+
+FAR = [1e12, 1e20, 9.969209968386869e36, np.inf, np.nan]
+
+
+@pytest.mark.parametrize("far", FAR)
+@pytest.mark.parametrize("axis", [0, 1])
+def test_a_far_gauge_without_a_value(far, axis):
+    """Its coordinates (a fill value, say) are nobody's business."""
+    job = list(_job(90, 3, 200))
+    want = _plan(job, ["OK", "SK"], EXP, False)
+    want.execute()
+    job[axis] = np.append(job[axis], far)
+    job[1 - axis] = np.append(job[1 - axis], 1e5)
+    job[2] = np.column_stack([job[2], np.full(3, np.nan)])
+    p = _plan(job, ["OK", "SK"], EXP)
+    p.execute()
+    _near(p.fields(), want.fields())
+
+
+@pytest.mark.parametrize("far", FAR[:3])
+@pytest.mark.parametrize("vg", [EXP, "0.9 Sph(60000)", "0.1 Nug(0.0) + 0.9 Gau(9000)"])
+def test_a_far_gauge_in_use_and_a_far_cell(far, vg):
+    for where in (0, 3):
+        job = list(_job(90, 3, 200))
+        job[where][7] = far
+        a, b = (_plan(job, ["OK", "SK"], vg, tc) for tc in (True, False))
+        a.execute()
+        b.execute()
+        _near(a.fields(), b.fields())
+
+
+@pytest.mark.parametrize("far", FAR[3:])
+@pytest.mark.parametrize("axis", [3, 4])
+def test_a_cell_without_a_place(far, axis):
+    """A domain ten times as long in x as in y, a cell at NaN or infinity: the
+    other cells keep their values."""
+    job = list(_job(90, 3, 200))
+    job[1], job[4] = job[1] / 10, job[4] / 10
+    want = _plan(job, ["OK", "SK"], EXP, False)
+    want.execute()
+    job[axis][11] = far
+    p = _plan(job, ["OK", "SK"], EXP)
+    p.execute()
+    rest = np.arange(200) != 11
+    _near({k: v[:, rest] for k, v in p.fields().items()},
+          {k: v[:, rest] for k, v in want.fields().items()})
+
+
+def test_a_range_short_of_the_domain():
+    """Exp(12) in a domain of 76 km: stations a few metres apart."""
+    job = list(_job(90, 2, 200))
+    for a, b in ((0, 3), (1, 4)):
+        job[b][:80] = job[a][:80] + np.random.default_rng(a).uniform(-9, 9, 80)
+    a, b = (_plan(job, ["OK", "SK"], "0.9 Exp(12)", tc) for tc in (True, False))
+    a.execute()
+    b.execute()
+    _near(a.fields(), b.fields(), 1e-14)
