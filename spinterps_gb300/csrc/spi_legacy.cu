@@ -439,7 +439,8 @@ __global__ void k_leg_dists(const double* __restrict__ xi, const double* __restr
 
 // rhss[k, :] of every point k.
 // The same with the entries in fixed point (spi_fx.cuh), where the points
-// and the variogram have that form, else by the FP64 formulas. A warp takes
+// and the variogram have that form on a grid that resolves the ranges, else by
+// the FP64 formulas. A warp takes
 // 32 points at a time (their grid coordinates by one lane each), its lanes
 // the stations, whose grid coordinates lie in shared memory. A coinciding
 // pair (0 on the grid) goes to the FP64 formula, which decides whether its
@@ -464,7 +465,7 @@ __global__ __launch_bounds__(LR_T) void k_leg_rhs_fx(
   const int m = n + (sk ? 0 : 1 + n_drift);
   if (tid == 0) {
     fx_init(f, vg, sk, 0.0, gr.q);
-    if (!scene->ok) f.ok = 0;
+    if (!scene->ok || !fx_resolves(vg, gr.q)) f.ok = 0;
     double t = 0.0;
     for (int c = 0; c < vg.n_comp; ++c)
       if (vg.code[c] == SPI_VG_NUG) t += vg.sill[c];
