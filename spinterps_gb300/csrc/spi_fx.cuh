@@ -330,6 +330,11 @@ FX_HD FxDist fx_dist(int64_t cx, int64_t cy, int64_t sx, int64_t sy) {
   return {(fx_sqrh(ax) >> 2) + (fx_sqrh(ay) >> 2), L};
 }
 
+// A correlation times its structure's weight.
+FX_HD int64_t fx_weighed(int64_t v, uint64_t w) {
+  return w == ~0ull ? v : (int64_t)(fx_mulh((uint64_t)v << 1, w) >> 1);
+}
+
 // One structure's correlation, its weight included; H: fx_sqrt(S) =
 // h 2^(L - 1) (not read by Gau). No branches on data: a warp's lanes keep
 // together.
@@ -365,7 +370,7 @@ FX_HD int64_t fx_rho(int code, const FxComp& k, FxDist d, uint64_t H, const uint
     }
   }
   v = d.S == 0 ? (int64_t)1 << FX_BITS : v;
-  return k.w == ~0ull ? v : (int64_t)(fx_mulh((uint64_t)v << 1, k.w) >> 1);
+  return fx_weighed(v, k.w);
 }
 
 // N entries of one cell, before the min_vg_val cut. CODE: the model of a

@@ -442,9 +442,12 @@ __global__ void k_leg_dists(const double* __restrict__ xi, const double* __restr
 // and the variogram have that form on a grid that resolves the ranges, else by
 // the FP64 formulas. A warp takes
 // 32 points at a time (their grid coordinates by one lane each), its lanes
-// the stations, whose grid coordinates lie in shared memory. A coinciding
-// pair (0 on the grid) goes to the FP64 formula, which decides whether its
-// distance is zero.
+// the stations, whose grid coordinates lie in shared memory. The FP64 formula
+// takes a coinciding pair (0 on the grid), deciding whether its distance is
+// zero, and a spherical's or linear's semivariance under 1/32 of the sills:
+// those formulas keep their relative precision down to distance 0, which a
+// difference from the sill (some 2^-58 of it off) has only above that. A pair
+// in a thousand or less.
 //
 // Bound by integer issue, some 230 operations an entry and one FP64
 // operation (a structure's share of a nugget and a sill); the FP64 formulas
@@ -460,6 +463,7 @@ __global__ __launch_bounds__(LR_T) void k_leg_rhs_fx(
   __shared__ FxVg f;
   __shared__ uint64_t tab[256];
   __shared__ double nug;
+  __shared__ int64_t one;  // the entry at distance 0: the weights' sum
   const FxGrid gr = scene->g;
   const int tid = threadIdx.x, lane = tid & 31;
   const int m = n + (sk ? 0 : 1 + n_drift);
@@ -470,6 +474,8 @@ __global__ __launch_bounds__(LR_T) void k_leg_rhs_fx(
     for (int c = 0; c < vg.n_comp; ++c)
       if (vg.code[c] == SPI_VG_NUG) t += vg.sill[c];
     nug = t;
+    one = 0;
+    for (int c = 0; c < f.n; ++c) one += fx_weighed((int64_t)1 << FX_BITS, f.c[c].w);
   }
   if (tid < 256) tab[tid] = fx_exp2_entry(tid);
   __syncthreads();
@@ -483,6 +489,7 @@ __global__ __launch_bounds__(LR_T) void k_leg_rhs_fx(
   const int code = f.n == 1 ? f.c[0].code : -1;
   // (an OK / EDK entry: nugget + sill (1 - rho); SK's covariance: sill rho)
   const double base = sk ? 0.0 : nug, sill = f.sill;
+  const int64_t one_ = one;
   for (int64_t b = w0 * 32; b < n_out; b += nw * 32) {
     const int64_t kl = min(b + lane, n_out - 1);
     const double xl = xk[kl], yl = yk[kl];
@@ -506,14 +513,17 @@ __global__ __launch_bounds__(LR_T) void k_leg_rhs_fx(
           int64_t v[2];
           fx_entries<CODE, 2>(f, d, tab, v);
           double r[2];
+          bool near[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            // (nests may round a unit past their sills)
-            const int64_t g = sk ? v[e] : ((int64_t)1 << FX_BITS) - v[e];
+            // (nests may round a unit past their sills, whose sum in FP64 is not
+            // exact: the weights then add up to 2^-53 more or less than 1)
+            const int64_t g = sk ? v[e] : one_ - v[e];
+            near[e] = (CODE == SPI_VG_SPH || CODE < 0) && !sk && g < ((int64_t)1 << (FX_BITS - 5));
             r[e] = fma(fx_double((uint64_t)(g < 0 ? 0 : g)), sill, base);
           }
-          if (d[0].S == 0) r[0] = exact(j);
-          if (d[1].S == 0) r[1] = exact(j1);
+          if (d[0].S == 0 || near[0]) r[0] = exact(j);
+          if (d[1].S == 0 || near[1]) r[1] = exact(j1);
           out[j] = r[0];
           if (j + 32 < n) out[j + 32] = r[1];
         }

@@ -51,3 +51,19 @@ def test_ranges_short_of_the_domain(rhss, model):
     for kind in ("OK", "SK"):
         got, want = rhss(kind, xi, yi, xk, yk, model)
         assert np.abs(got - want).max() <= 8 * 2.0 ** -53 * 0.7, kind
+
+
+@pytest.mark.parametrize("model", ["0.7 Sph(60000)", "1.3 Lin(50000)",
+                                   "0.5 Sph(60000) + 0.2 Lin(30000)"])
+def test_semivariances_beside_a_station(rhss, model):
+    """Relative: the FP64 formulas of a spherical or linear lose a few
+    roundings at any distance (16 * 2^-53 bounds both evaluations)."""
+    xi, yi, xk, yk = _points(4)
+    rng = np.random.default_rng(5)
+    near = rng.integers(0, 97, 900)
+    d = np.exp(rng.uniform(np.log(1e-4), np.log(3e3), 900))
+    a = rng.uniform(0, 2 * np.pi, 900)
+    xk[:900], yk[:900] = xi[near] + d * np.cos(a), yi[near] + d * np.sin(a)
+    got, want = rhss("OK", xi, yi, xk, yk, model)
+    assert (want > 0).all()
+    assert (np.abs(got - want) / want).max() <= 16 * 2.0 ** -53
