@@ -226,8 +226,8 @@ __global__ void k_sl_select_one(SlArgs A) { A.rec[0].use = 1; }
 template <int MODE>
 __device__ __forceinline__ RowRef row_ref(const SlArgs& A, int s, int n, int nvb, int row) {
   if constexpr (MODE == kRows) {
-    if (row >= n) return {nullptr, 0};
-    return {A.rows.inv + (int64_t)row * n, n};
+    if (row >= A.rows.m) return {nullptr, 0};
+    return {A.rows.inv + (int64_t)row * A.rows.m, n};
   } else {
     const int64_t soff = A.sys.stn_off[s];
     if (row < nvb * SL_R) {
@@ -247,7 +247,7 @@ __device__ __forceinline__ RowRef row_ref(const SlArgs& A, int s, int n, int nvb
 // Entries per cell of a system.
 template <int MODE>
 __device__ __forceinline__ int n_entries(const SlArgs& A, int s) {
-  if constexpr (MODE == kRows) return A.rows.m;
+  if constexpr (MODE == kRows) return A.rows.n;
   else return (int)(A.sys.stn_off[s + 1] - A.sys.stn_off[s]);
 }
 // Rows besides the variance's.
@@ -573,19 +573,19 @@ __device__ __forceinline__ double scaled_double(long long h, uint32_t l, int e) 
   return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0)));
 }
 
-// Given right-hand sides, scaled by a power of two per point. S.nnb: its
-// exponent, or kNotFinite.
+// Given right-hand sides' stations, scaled by a power of two per point. S.nnb:
+// its exponent, or kNotFinite.
 constexpr int kNotFinite = 0x7fffffff;
 // Neighbouring lanes take four pairs of entries of a point (64 bytes of its
 // row), eight points to a warp (128 bytes of a slot's line); the scaling is
 // a shift of the significand.
-__device__ __forceinline__ void sl_gen_rows(const SlArgs& A, SlSmem& S, int m, int k16,
+__device__ __forceinline__ void sl_gen_rows(const SlArgs& A, SlSmem& S, int n, int k16,
                                             int64_t c0, int64_t C, int tid, ulonglong2* slot) {
   constexpr int PARTS = SL_WT / SL_M;
   const int cell = tid / PARTS, part = tid % PARTS;
-  const double* r = A.rows.rhs + min(c0 + cell, C - 1) * m;
+  const double* r = A.rows.rhs + min(c0 + cell, C - 1) * A.rows.m;
   int mx = 0;
-  for (int j = part; j < m; j += PARTS) mx = max(mx, __double2hiint(r[j]) & 0x7fffffff);
+  for (int j = part; j < n; j += PARTS) mx = max(mx, __double2hiint(r[j]) & 0x7fffffff);
   int* km = reinterpret_cast<int*>(&S.q[0][0]);
   km[part * SL_M + cell] = mx;
   work_sync();
@@ -597,8 +597,8 @@ __device__ __forceinline__ void sl_gen_rows(const SlArgs& A, SlSmem& S, int m, i
   for (int p = part; p < k16 * (SL_K / 2); p += PARTS) {
     ulonglong2 v{SL_BIAS, SL_BIAS};
     const int j = 2 * p;
-    if (j < m && !bad) v.x += (uint64_t)scaled_int(r[j], q0);
-    if (j + 1 < m && !bad) v.y += (uint64_t)scaled_int(r[j + 1], q0);
+    if (j < n && !bad) v.x += (uint64_t)scaled_int(r[j], q0);
+    if (j + 1 < n && !bad) v.y += (uint64_t)scaled_int(r[j + 1], q0);
     slot[(int64_t)p * SL_M + cell] = v;
   }
 }
@@ -890,20 +890,34 @@ __global__ __launch_bounds__(SL_T, 1) void k_sl_gemm(SlArgs A, int tiles) {
       if constexpr (MODE == kRows) {
         // (b + row) 0 .. of this thread's point
         const int row0 = b * SL_R + rq * SL_RT;
-        const int ec = S.nnb[dcell];
-        if (dg < C) {
-          double* lam = A.rows.lambdas + dg * A.rows.n + row0;
+        const int ec = S.nnb[dcell], m = A.rows.m;
+        if (dg < C)
 #pragma unroll
-          for (int q = 0; q < SL_RT; ++q) {
-            const int row = row0 + q;
-            const double y =
-                ec == kNotFinite
-                    ? __longlong_as_double(0x7ff8000000000000LL)
-                    : scaled_double(acc_h[q], acc_l[q], ec + row_e[b * SL_R + q] - 68);
-            if (row < A.rows.n) lam[q] = y;
-            else if (row < n) A.rows.mus[(int64_t)(row - A.rows.n) * C + dg] = y;
+          for (int h = 0; h < SL_RT; h += 4) {
+            // (four rows at a time: their loads overlap, the others' sums keep
+            // their registers)
+            double y[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              y[q] = ec == kNotFinite
+                         ? __longlong_as_double(0x7ff8000000000000LL)
+                         : scaled_double(acc_h[h + q], acc_l[h + q],
+                                         ec + row_e[b * SL_R + h + q] - 68);
+            for (int k = n; k < m; ++k) {
+              const double r = A.rows.rhs[dg * m + k];
+              const double* inv = A.rows.inv + (int64_t)(row0 + h) * m + k;
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                y[q] = fma(row0 + h + q < m ? __ldg(inv + (int64_t)q * m) : 0.0, r, y[q]);
+            }
+            double* lam = A.rows.lambdas + dg * n + row0 + h;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int row = row0 + h + q;
+              if (row < n) lam[q] = y[q];
+              else if (row < m) A.rows.mus[(int64_t)(row - n) * C + dg] = y[q];
+            }
           }
-        }
         continue;
       }
       if (b < W.nvb) {
@@ -1230,9 +1244,9 @@ int launch_slices_rows(const SlRows& r, void* scratch, int64_t scratch_bytes, in
                        const int32_t** use, cudaStream_t st) {
   const int sms = n_sms();
   if (sms <= 0) return SPI_ERR_CUDA;
-  SlPlan p(r.m, 1, r.m, false, true, sms);
+  SlPlan p(r.n, 1, r.m, false, true, sms);
   SlArgs A = {};
-  if (int rc = one_layout(A, p, r.m, scratch, scratch_bytes, sms)) return rc;
+  if (int rc = one_layout(A, p, r.n, scratch, scratch_bytes, sms)) return rc;
   A.err = err;
   A.rows = r;
   *use = &A.rec[0].use;

@@ -18,7 +18,10 @@ struct SlicesDone {
 };
 
 // Right-hand sides rhs [points, m] against the rows of inv [m, m]: the first
-// n results to lambdas [points, n], the rest to mus [m - n, points].
+// n results to lambdas [points, n], the rest to mus [m - n, points]. The first
+// n entries of each, the stations', go through the slices, the others (ones
+// and drifts, whose size has nothing to do with the variogram's) through FP64:
+// on one scale with them, semivariances of 1e-9 kept 32 bits.
 struct SlRows {
   const double* rhs;
   const double* inv;
