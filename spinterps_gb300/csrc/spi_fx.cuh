@@ -144,6 +144,21 @@ FX_HD int64_t fx_coord0(double x, int q) {
   return b < 0 ? -v : v;
 }
 
+// The place of x's last bit, x = odd 2^place: a grid of 2^-q holds x exactly
+// where it is -q or more.
+FX_HD int fx_place(double x) {
+#ifdef __CUDA_ARCH__
+  const int64_t b = __double_as_longlong(x);
+#else
+  int64_t b;
+  __builtin_memcpy(&b, &x, 8);
+#endif
+  const int e = (int)((b >> 52) & 0x7ff);
+  const int64_t m = (b & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
+  if (m == 0) return 4096;
+  return (e ? e : 1) - 1075 + 63 - fx_clz((uint64_t)(m & -m));
+}
+
 // A positive double as a 64-bit mantissa and an exponent: v = m 2^e, m with
 // its top bit set.
 FX_HD void fx_norm(double v, uint64_t& m, int& e) {
@@ -420,9 +435,27 @@ FX_HD double fx_double(uint64_t v) {
 
 // A squared distance as a monotone key: the exponent above 55 bits of the
 // normalised square (its top bit set). 0: the points coincide.
+constexpr int FX_KEY = 511;
 FX_HD uint64_t fx_key(FxDist d) {
   const int z = fx_clz(d.S | 1);
-  return d.S ? ((uint64_t)(200 - 2 * d.L - z) << 55) + ((d.S << z) >> 9) : 0ull;
+  return d.S ? ((uint64_t)(FX_KEY - 2 * d.L - z) << 55) + ((d.S << z) >> 9) : 0ull;
+}
+
+// The same form of a squared distance d2 > 0 given in FP64 (normal), on a grid
+// of 2^-q: what lies too close for the grid. Distances under 2^-191 steps
+// count as that.
+FX_HD FxDist fx_dist_f64(double d2, int q) {
+#ifdef __CUDA_ARCH__
+  const int64_t b = __double_as_longlong(d2);
+#else
+  int64_t b;
+  __builtin_memcpy(&b, &d2, 8);
+#endif
+  const int e = (int)(b >> 52) - 1022;  // d2 = f 2^e, f in [1/2, 1)
+  const int t = 128 - e - 2 * q, L = t >> 1;
+  const uint64_t m = (uint64_t)((b & 0xfffffffffffffll) | (1ll << 52));
+  if (L > 254) return {1ull << 60, 254};
+  return {m << (9 - (t & 1)), L};
 }
 
 // The inverse-square weight (h_ref / h)^2 <= 1 as a double, by its bits (no
@@ -434,7 +467,7 @@ FX_HD double fx_weight2(FxDist d, uint64_t ref) {
   const int c = fx_clz(q);
   // the top 53 bits, rounded (a carry into the exponent comes out right)
   const uint64_t m = ((q << c) >> 11) + (((q << c) >> 10) & 1);
-  const int e = 1024 - c - ((200 - 2 * d.L - z) - (int)(ref >> 55));
+  const int e = 1024 - c - ((FX_KEY - 2 * d.L - z) - (int)(ref >> 55));
   const uint64_t b = ((uint64_t)(e - 1) << 52) + m;
 #ifdef __CUDA_ARCH__
   return __longlong_as_double((long long)b);

@@ -200,8 +200,10 @@ __global__ __launch_bounds__(CT) void k_idw(IdwArgs A, int npad) {
 // ratios (d_ref / d)^2 (spi_fx.cuh; relative rms 0.5 units of 2^-53), and a
 // thread sums one (cell, step), an FMA and an addition per present station,
 // the stations split over the threads that few steps leave free. 1000
-// stations, 4 steps, 62 500 cells: 12.2 -> 1.7 ms (73 steps: 29.6 -> 16.6); 150 stations, 24 steps,
-// 40 000 cells: 1.30 -> 0.64 ms.
+// stations, 4 steps, 62 500 cells: 12.2 -> 1.8 ms (73 steps: 29.6 -> 16.6); 150
+// stations, 24 steps, 40 000 cells: 1.30 -> 0.61 ms. (Integers alone took 1.76
+// ms there, but held near pairs of a wide domain to its grid; with offsets of
+// 4e5 and 5.5e6, where most pairs count as near, 1.88.)
 constexpr int IT = 512;
 
 template <int TC, typename OutT>
@@ -212,44 +214,80 @@ __global__ __launch_bounds__(IT) void k_idw_sq(IdwArgs A) {
   __shared__ unsigned long long key[NG][TC];
   __shared__ int onst[NG][TC];
   __shared__ double2 part[NG][TC];
-  __shared__ int red[IT / 32];
+  __shared__ int red[IT / 32], redp[IT / 32];
   const int64_t C = A.dom.n_cells;
   const int N = (int)A.dom.n_stns;
   const int tid = threadIdx.x, cell = tid % TC, grp = tid / TC;
   const int64_t c0 = (int64_t)blockIdx.x * TC, gc = min(c0 + cell, C - 1);
   const double cx = A.dom.cell_x[gc], cy = A.dom.cell_y[gc];
-  // the grid: every coordinate under 2^FX_GRID of its units
-  int mx = max(__double2hiint(cx) & 0x7fffffff, __double2hiint(cy) & 0x7fffffff);
-  for (int j = tid; j < N; j += IT)
+  // the grid: every station's and this cell's coordinates under 2^FX_GRID of
+  // its units; and the finest place of their coordinates
+  int mx = 0, place = 4096;
+  for (int j = tid; j < N; j += IT) {
+    place = min(place, min(fx_place(A.dom.stn_x[j]), fx_place(A.dom.stn_y[j])));
     mx = max(mx, max(__double2hiint(A.dom.stn_x[j]) & 0x7fffffff,
                      __double2hiint(A.dom.stn_y[j]) & 0x7fffffff));
-  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((tid & 31) == 0) red[tid >> 5] = mx;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    place = min(place, __shfl_xor_sync(0xffffffffu, place, o));
+  }
+  if ((tid & 31) == 0) {
+    red[tid >> 5] = mx;
+    redp[tid >> 5] = place;
+  }
   __syncthreads();
-  for (int w = 0; w < IT / 32; ++w) mx = max(mx, red[w]);
-  const int q = FX_GRID - ((mx >> 20) - 1022);
+  for (int w = 0; w < IT / 32; ++w) {
+    mx = max(mx, red[w]);
+    place = min(place, redp[w]);
+  }
+  mx = max(mx, max(__double2hiint(cx) & 0x7fffffff, __double2hiint(cy) & 0x7fffffff));
+  // coordinates that are not finite, or of a size that the keys' exponents
+  // don't span: FP64 alone
+  const int size = (mx >> 20) - 1022;  // |x| < 2^size
+  const bool wild = size > 100 || size < -100;
+  const int q = FX_GRID - size;
   const int64_t X = fx_coord0(cx, q), Y = fx_coord0(cy, q);
-  // a station's distance; points that share their grid place but not their
-  // coordinates count as the least distance
+  const bool cell_exact = min(fx_place(cx), fx_place(cy)) >= -q;
+  const bool exact = cell_exact && place >= -q;
+  // a station's distance. Coordinates are cut off at the grid, which moves a
+  // distance by up to 1.4 steps: from 2^54 steps on (L <= 8) that is under
+  // FP64's rounding of the weight; a nearer pair with a coordinate that the
+  // grid does not hold takes the FP64 distance.
   auto dist = [&](int j, bool& on) {
     const double sx = A.dom.stn_x[j], sy = A.dom.stn_y[j];
     FxDist d = fx_dist(X, Y, fx_coord0(sx, q), fx_coord0(sy, q));
     on = false;
-    if (d.S == 0) {
-      on = cx == sx && cy == sy;
-      d = {1ull << 60, 63};
+    if (d.L > 8) {
+      if (exact || (cell_exact && min(fx_place(sx), fx_place(sy)) >= -q)) {
+        on = d.S == 0;
+      } else {
+        const double d2 = dist2_f64(cx, cy, sx, sy);
+        on = d2 == 0.0;
+        d = fx_dist_f64(d2, q);
+      }
     }
     return d;
   };
   // ---- 1. the nearest distance; the first station on the cell ----
+  // (wild: the squared distance's bits, which order as it does)
   unsigned long long best = ~0ull;
   int on1 = 0x7fffffff;
+  if (wild) {
+    best = 0x7ff0000000000000ull;
+    for (int j = grp; j < N; j += NG) {
+      const double d2 = dist2_f64(cx, cy, A.dom.stn_x[j], A.dom.stn_y[j]);
+      if (d2 == 0.0) on1 = min(on1, j);
+      else best = min(best, (unsigned long long)__double_as_longlong(d2) & 0x7fffffffffffffffull);
+    }
+  } else {
 #pragma unroll 2
-  for (int j = grp; j < N; j += NG) {
-    bool on;
-    const FxDist d = dist(j, on);
-    if (on) on1 = min(on1, j);
-    else best = min(best, (unsigned long long)fx_key(d));
+    for (int j = grp; j < N; j += NG) {
+      bool on;
+      const FxDist d = dist(j, on);
+      if (on) on1 = min(on1, j);
+      else best = min(best, (unsigned long long)fx_key(d));
+    }
   }
   key[grp][cell] = best;
   onst[grp][cell] = on1;
@@ -259,11 +297,18 @@ __global__ __launch_bounds__(IT) void k_idw_sq(IdwArgs A) {
     on1 = min(on1, onst[g][cell]);
   }
   // ---- 2. weights, 0 on a station ----
+  if (wild) {
+    for (int j = grp; j < N; j += NG) {
+      const double d2 = dist2_f64(cx, cy, A.dom.stn_x[j], A.dom.stn_y[j]);
+      W[j * TC + cell] = d2 == 0.0 ? 0.0 : __longlong_as_double((long long)best) / d2;
+    }
+  } else {
 #pragma unroll 2
-  for (int j = grp; j < N; j += NG) {
-    bool on;
-    const FxDist d = dist(j, on);
-    W[j * TC + cell] = on ? 0.0 : fx_weight2(d, best);
+    for (int j = grp; j < N; j += NG) {
+      bool on;
+      const FxDist d = dist(j, on);
+      W[j * TC + cell] = on ? 0.0 : fx_weight2(d, best);
+    }
   }
   __syncthreads();
   // ---- 3. steps ----
