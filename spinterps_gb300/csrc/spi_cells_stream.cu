@@ -53,6 +53,8 @@ inline __device__ __noinline__ df stream_general(const CellsArgs& A, const spi_v
                                                  int64_t gc, const int32_t* stp) {
   return rhs_df_d2(A.dom, vgp, kd, sk, sh, d2, gc, stp);
 }
+// The coordinates up to which squared distances stay within FP32.
+constexpr float kFar = 1e18f;
 
 // One shared-memory chunk of stations against the pass's vectors (FP32
 // tier): double-float entries times hi/lo vector pairs, the product's head
@@ -283,6 +285,7 @@ __global__ __launch_bounds__(STC * SNW, sizeof(T) == 4 ? 4 : 2) void k_krige_cel
 
   double cx = 0.0, cy = 0.0;
   float4 cp[NC];
+  __shared__ int wild;  // a cell too far for FP32's squares, or without a place
   __shared__ RhsDf kd;
   __shared__ RhsOne ko;
   // the variogram with its reciprocal ranges (FP64 right-hand sides)
@@ -299,6 +302,14 @@ __global__ __launch_bounds__(STC * SNW, sizeof(T) == 4 ? 4 : 2) void k_krige_cel
       if (kd.exact && kd.single >= 0) ko.init(kd, vg, sk, sh, A.dom.min_vg_val);
     }
     for (int e = tid; e < 256; e += STC * SNW) s_tab[e] = kExp2.v[e];
+    bool w = false;
+#pragma unroll
+    for (int u = 0; u < NC; ++u) w = w || !(fabsf(cp[u].x) + fabsf(cp[u].z) < kFar);
+    w = __syncthreads_or(w) != 0;
+    if (tid == 0) {
+      wild = w;
+      if (w) kd.exact = 0;  // (every entry in FP64)
+    }
   }
   const spi_vg_t* vgp = A.sys.vg + s;
   const float4* sp4 = reinterpret_cast<const float4*>(A.dom.stn_split);
@@ -371,7 +382,11 @@ __global__ __launch_bounds__(STC * SNW, sizeof(T) == 4 ? 4 : 2) void k_krige_cel
         const int nj = min(SCH, n - j0);
         __syncthreads();
         for (int e = tid; e < nj; e += STC * SNW) {
-          s_sp[e] = sp4[idx[j0 + e]];
+          // (a gauge beyond kFar is that far from every cell but the wild ones)
+          float4 sp = sp4[idx[j0 + e]];
+          sp.x = fminf(fmaxf(sp.x, -kFar), kFar);
+          sp.z = fminf(fmaxf(sp.z, -kFar), kFar);
+          s_sp[e] = sp;
 #pragma unroll
           for (int v = 0; v < SSV; ++v)
             if (v < nv) s_w[e][v] = make_float2(vph[v][j0 + e], vpl[v][j0 + e]);
@@ -446,7 +461,7 @@ __global__ __launch_bounds__(STC * SNW, sizeof(T) == 4 ? 4 : 2) void k_krige_cel
       // red is free again
 #pragma unroll
       for (int u = 0; u < NC; ++u) s_nf[warp * TC + u * STC + lane] = nf[u];
-      nf_ready = true;
+      nf_ready = !wild;
     }
     for (int e = tid; e < nv * TC; e += STC * SNW)
       if (v0 + e / TC < ndual) qsh[v0 + e / TC][e % TC] = vres[e / TC][e % TC];
