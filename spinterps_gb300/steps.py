@@ -243,6 +243,19 @@ def _align(x, a=32):
     return (x + a - 1) // a * a
 
 
+def slices_scratch_bytes(n, n_sys, max_steps, n_drift, want_var, mixed):
+    """Device scratch of the sliced tensor-core passes of n_sys systems of up
+    to n stations and max_steps steps: 0 for systems too small for them.
+    n_drift: 0 for OK and SK; want_var: with the OK variance."""
+    if n < SLICES_MIN_N:
+        return 0
+    lib = nat.lib()
+    need = lib.spi_slices_scratch_bytes(n, n_sys, max_steps, n_drift, int(want_var), 1)
+    if mixed and want_var:
+        need = max(need, lib.spi_slices_scratch_bytes(n, n_sys, 0, 0, 1, 0))
+    return int(need)
+
+
 class _KrigeBatch:
     """One chunk of kriging systems: device descriptors and workspaces."""
 
@@ -395,15 +408,8 @@ class _KrigeBatch:
     def slices_bytes(self, want_var):
         """Scratch of the sliced tensor-core contraction: 0 for systems too
         small for it."""
-        n = int(self.n.max())
-        if n < SLICES_MIN_N:
-            return 0
-        lib = nat.lib()
-        need = lib.spi_slices_scratch_bytes(n, len(self.ch), self.max_steps, self.n_drift,
-                                            int(want_var), 1)
-        if self.precision == 1 and want_var:
-            need = max(need, lib.spi_slices_scratch_bytes(n, len(self.ch), 0, 0, 1, 0))
-        return int(need)
+        return slices_scratch_bytes(int(self.n.max()), len(self.ch), self.max_steps,
+                                    self.n_drift, want_var, self.precision == 1)
 
     def cells_fp64(self, dom, out, want_var, filt, cond_split, tile, s):
         """The FP64 cell pass on the cells of dom: the sliced tensor-core

@@ -10,7 +10,8 @@ cell x station matrices never exist, so only the steps are cut: a wave
 holds as many steps as its fields (cells x labels x the output type) and
 its factor arenas ((n + 8)^2 doubles per system, twice with the OK
 variance's inverse factor, plus the tensor-core variance's n_cells doubles
-per OK system of the mixed path) leave within the budget. Every step's
+per OK system of the mixed path) and the scratch of the sliced passes, one
+per wave, leave within the budget. Every step's
 system is its own (its station set and variogram), so cutting the steps
 changes no result: a wave's fields equal the same rows of a one-shot run.
 
@@ -32,7 +33,7 @@ import numpy as np
 import torch
 
 from . import _native as nat
-from .steps import InterpPlan, _require_cuda
+from .steps import InterpPlan, _require_cuda, slices_scratch_bytes
 
 
 def step_bytes(n_present, n_cells, n_labels, out_itemsize, krige_kinds, ok_var, mixed):
@@ -56,36 +57,49 @@ def step_bytes(n_present, n_cells, n_labels, out_itemsize, krige_kinds, ok_var, 
     return int(b)
 
 
+def scratch_bytes(n_present, n_steps, krige_kinds, ok_var, mixed, n_drift=0):
+    """Device bytes of a wave's one scratch, which its kriging kinds share
+    (the sliced tensor-core passes): an upper bound, every step a system of
+    n_present stations or all of them steps of one."""
+    return max((slices_scratch_bytes(int(n_present), n_steps, n_steps,
+                                     n_drift if kind == "EDK" else 0, ok_var and kind == "OK",
+                                     mixed) for kind in krige_kinds), default=0)
+
+
 def nebs_fixed_bytes(n_cells, k):
     """Device bytes a wave of the neighbour methods holds besides its
     fields: one step group's neighbour lists ([n_cells, k] int32, selected
-    and mapped), their grouping (int64 inverse and order, int32 copies)
-    and the kriging scratch of spi_local_groups (at most
+    and mapped), their grouping (int64 inverse and order, int32 copies; the
+    hash table's 9 int32 a cell) and the kriging scratch of spi_local_groups (at most
     nebs.GRP_SCRATCH_BYTES)."""
     from .nebs import GRP_SCRATCH_BYTES
-    return int(GRP_SCRATCH_BYTES + n_cells * (3 * 4 * max(int(k), 1) + 4 * 8))
+    return int(GRP_SCRATCH_BYTES + n_cells * (3 * 4 * max(int(k), 1) + 4 * 8 + 9 * 4))
 
 
 def plan_waves(data, n_cells, interp_args, *, budget, out_itemsize=4, est_vars=False,
-               precision="fp64", neighbours=False):
+               precision="fp64", neighbours=False, n_drift=0, tensor_cores=True):
     """Cut the steps of ``data`` [T, N] (NaN = missing) into consecutive
-    waves whose step_bytes add up to at most ``budget``; a step that alone
-    exceeds it is a wave of its own. With ``neighbours`` (the neighbour
+    waves whose step_bytes and scratch_bytes add up to at most ``budget``; a
+    step that alone exceeds it is a wave of its own. With ``neighbours`` (the neighbour
     methods) a step costs its fields only. Returns [(first, end), ...]."""
     types = [a[0] for a in interp_args]
     kinds = [t for t in ("OK", "SK", "EDK") if t in types]
     n_labels = len(interp_args)
     n_av = np.isfinite(np.asarray(data)).sum(1)
-    waves, t0, acc = [], 0, 0
+    waves, t0, acc, n_max = [], 0, 0, 0
     for t in range(n_av.size):
         if neighbours:
             b = n_cells * n_labels * out_itemsize
         else:
             b = step_bytes(int(n_av[t]), n_cells, n_labels, out_itemsize, kinds, est_vars,
                            precision == "mixed")
-        if t > t0 and acc + b > budget:
+        n_max = max(n_max, int(n_av[t]))
+        fixed = 0
+        if tensor_cores and not neighbours:
+            fixed = scratch_bytes(n_max, t + 1 - t0, kinds, est_vars, precision == "mixed", n_drift)
+        if t > t0 and acc + b + fixed > budget:
             waves.append((t0, t))
-            t0, acc = t, 0
+            t0, acc, n_max = t, 0, int(n_av[t])
         acc += b
     if n_av.size:
         waves.append((t0, n_av.size))
@@ -137,8 +151,12 @@ def interp_steps_waves(stn_x, stn_y, data, cell_x, cell_y, vgs, interp_args, *, 
                     prblm.append(t)
             info.append({"steps": [int(a), int(b)], "call_s": time.perf_counter() - t0})
         return prblm, info
+    n_drift = 0
+    if stn_drifts is not None:
+        n_drift = np.asarray(stn_drifts).reshape(np.asarray(stn_x).size, -1).shape[1]
     waves = plan_waves(data, C, interp_args, budget=budget, out_itemsize=itemsize,
-                       est_vars=est_vars, precision=precision)
+                       est_vars=est_vars, precision=precision, n_drift=n_drift,
+                       tensor_cores=plan_kw.get("tensor_cores", True))
 
     def build(w):
         a, b = w
