@@ -229,8 +229,8 @@ __global__ __launch_bounds__(256) void k_leg_update(double* __restrict__ A, int 
 // operations as k_leg_pivot and k_leg_update, which take a launch each per
 // step and pass the matrix through L2 (both stay for matrices whose rows
 // don't fit, m > ~1850). A step is bound by latency, the barrier's and L2's
-// in a chain: m = 401 5.9 ms before, 3.4 now; 201 2.4, 1.2; 801 15.7, 10.5;
-// 1501 41.8, 23.7. (Half as many CTAs: 3.0, 1.2, 11.4.)
+// in a chain: m = 401 5.9 ms by launches, 3.0 so; 201 2.4, 1.2; 801 15.7, 10.5;
+// 1501 41.8, 23.7.
 //
 // The barrier's wait is bounded: on expiry the CTA stores a status (the
 // caller then takes its pseudo-inverse path from lhs) and leaves, and so do
@@ -684,6 +684,15 @@ static int leg_check(int32_t kind, const double* xi, const double* yi, int32_t n
 }
 
 namespace spi {
+// Fewer CTAs make the barrier shorter and the updates longer. A whole
+// spi_legacy_system call with an eighth as many CTAs as rows, and with a
+// quarter: 2.40 and 2.25 ms at 301 rows, 3.24 and 3.65 at 401, 4.19 and 4.73 at
+// 501, 5.84 and 5.78 at 601, 12.0 and 11.2 at 801.
+static int leg_gj_ctas(int m, int sms) {
+  const int b = m >= 350 && m <= 560 ? m / 8 : m / 4;
+  return b < sms ? b : sms;
+}
+
 // k_leg_gj where its rows fit in shared memory (a quarter as many CTAs as
 // rows at most, so that two published rows of each fit in the n^2 doubles of
 // the workspace); false: not launched.
@@ -693,7 +702,7 @@ static bool leg_gj(double* A, int m, int n, double* ws, int32_t* piv, int32_t* s
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
-  const int B = m / 4 < sms ? m / 4 : sms;
+  const int B = leg_gj_ctas(m, sms);
   int rp = (m + B - 1) / B;
   const size_t smem = ((size_t)rp * m + m + rp) * sizeof(double) + rp * sizeof(int);
   // piv (m ints), the counter, the candidates, the rows
