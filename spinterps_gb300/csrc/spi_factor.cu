@@ -101,8 +101,10 @@ __global__ __launch_bounds__(256) void k_build_sys(spi_domain_t dom, spi_systems
       // (i, j) and its mirror from the same distance: dists[lo, hi]
       const int si = v.idx[i], sj = v.idx[j];
       const double d = dist_f64(dom.stn_x[sj], dom.stn_y[sj], dom.stn_x[si], dom.stn_y[si]);
-      const double g = mid ? pre.fill(d, sk, dom.min_vg_val)
-                           : vg_fill_f64(vg, d, sk, dom.min_vg_val);
+      // (a product by a reciprocal takes an infinite distance, or one of 2^497 on
+      // whose cube is, for no number)
+      const double g = mid && __double2hiint(d) < 0x5f000000 ? pre.fill(d, sk, dom.min_vg_val)
+                                                             : vg_fill_f64(vg, d, sk, dom.min_vg_val);
       x = sk ? g : __dsub_rn(sh, g);
     }
     A[e] = x;
