@@ -83,6 +83,20 @@ LOCAL_KIND = {"OK": 0, "SK": 1, "EDK": 2, "IDW": 3, "NNB": 4}
 GRP_SCRATCH_BYTES = 2 << 30
 
 
+def grp_scratch_bytes(kind, k, n_drift, n_grps, n_steps, n_stns):
+    """Scratch of a spi_local_groups call: all of its steps', at most
+    GRP_SCRATCH_BYTES, at least one step's. Room for the table of all
+    stations' pairs, which the call makes where the groups hold more entries
+    than it, as far as that allows."""
+    need, one = (nat.lib().spi_local_groups_scratch_bytes(kind, k, n_drift, n_grps, n)
+                 for n in (n_steps, 1))
+    tab = n_stns * n_stns * 8
+    if n_stns * n_stns <= n_grps * k * k and one + tab <= GRP_SCRATCH_BYTES:
+        need += n_steps * tab
+        one += tab
+    return max(one, min(need, GRP_SCRATCH_BYTES))
+
+
 def device_groups(nb):
     """Cells with identical neighbour lists, on the device: (grp_nebs [G, k],
     cell_grp [C], cell_order [C]) as int32, cell_order listing each group's
@@ -167,6 +181,7 @@ def interp_steps_nebs(stn_x, stn_y, data, cell_x, cell_y, vgs, interp_args, neb_
     inv = np.asarray(inv).ravel()
     s = _stream()
     held = []  # device arrays in use by queued launches
+    scratch = None  # one for all of them, in stream order
     for gi in np.argsort(first):
         rows = np.where(inv == gi)[0]
         stn_idxs = np.where(avail[rows[0]])[0]
@@ -181,7 +196,7 @@ def interp_steps_nebs(stn_x, stn_y, data, cell_x, cell_y, vgs, interp_args, neb_
         d_vg = vgt[d_rows.long()].contiguous() if krig else None
         d_nug = nug[d_rows.long()].contiguous() if krig else None
         d_pr = torch.zeros(rows.size, dtype=torch.int32, device=dev)
-        grp = scratch = None
+        grp = None
         held.append((d_stn, d_nb, d_rows, d_vg, d_nug, d_pr))
         for a in interp_args:
             if a[0] == "EST_VARS_OK":  # written by the OK launch
@@ -195,17 +210,9 @@ def interp_steps_nebs(stn_x, stn_y, data, cell_x, cell_y, vgs, interp_args, neb_
                     grp = device_groups(d_nb)
                     G = grp[0].shape[0]
                     held.append(grp)
-                need = nat.lib().spi_local_groups_scratch_bytes(kind, k, n_drift, G, rows.size)
-                one = nat.lib().spi_local_groups_scratch_bytes(kind, k, n_drift, G, 1)
-                # room for the table of all stations' pairs, which the call
-                # makes where the groups hold more entries than it
-                if sx.size ** 2 <= G * k * k:
-                    need += rows.size * sx.size ** 2 * 8
-                    one += sx.size ** 2 * 8
-                nbytes = max(one, min(need, GRP_SCRATCH_BYTES))
+                nbytes = grp_scratch_bytes(kind, k, n_drift, G, rows.size, sx.size)
                 if scratch is None or scratch.numel() < nbytes:
                     scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-                    held.append(scratch)
                 nat.call("spi_local_groups", ctypes.byref(dom.st), kind, k, _ptr(grp[0]), G,
                          _ptr(grp[1]), _ptr(grp[2]), rows.size, _ptr(d_rows), _ptr(d_rows),
                          _ptr(d_data), data.shape[1], _ptr(d_vg), _ptr(d_nug),
