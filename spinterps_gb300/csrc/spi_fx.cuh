@@ -24,7 +24,7 @@
 namespace spi {
 
 constexpr int FX_BITS = 62;                    // an entry of the structures' sills is 2^62
-constexpr int FX_GRID = 61;                    // coordinates: |X| <= 2^61
+constexpr int FX_GRID = 61;                    // coordinates without an origin: |X| <= 2^61
 
 #define FX_HD __host__ __device__ __forceinline__
 
@@ -76,6 +76,7 @@ FX_HD float fx_rcpf(float x) {
 struct FxGrid {
   double ox, oy;
   int q;
+  int exact;  // it holds every point exactly
 };
 
 // It, and whether the points have one (finite, not past FP64's middle range).
@@ -84,10 +85,26 @@ struct FxScene {
   int ok;
 };
 
+// The place of x's last bit, x = odd 2^place: a grid of 2^-q holds x exactly
+// where it is -q or more.
+FX_HD int fx_place(double x) {
+#ifdef __CUDA_ARCH__
+  const int64_t b = __double_as_longlong(x);
+#else
+  int64_t b;
+  __builtin_memcpy(&b, &x, 8);
+#endif
+  const int e = (int)((b >> 52) & 0x7ff);
+  const int64_t m = (b & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
+  if (m == 0) return 4096;
+  return (e ? e : 1) - 1075 + 63 - fx_clz((uint64_t)(m & -m));
+}
+
 // The grid of points between (x0, y0) and (x1, y1): its origin in
-// their middle, so that |X| <= 2^61 with a step of 2^-62 to 2^-61 of the larger
-// side. False where it has none.
-FX_HD bool fx_grid(double x0, double x1, double y0, double y1, FxGrid& g) {
+// their middle, so that |X| <= 2^62 (a difference stays under 2^63) with a step
+// of 2^-63 to 2^-62 of the larger side. False where it has none. place: the
+// finest place of the points' coordinates (fx_place), or less.
+FX_HD bool fx_grid(double x0, double x1, double y0, double y1, int place, FxGrid& g) {
   const double dx = x1 - x0, dy = y1 - y0;
   double ext = fmax(dx, dy);
   g.ox = x0 + 0.5 * dx;
@@ -96,20 +113,25 @@ FX_HD bool fx_grid(double x0, double x1, double y0, double y1, FxGrid& g) {
   if (!(ext > 1e-200)) ext = 1e-200;
   int e = 0;
   frexp(ext, &e);
-  g.q = FX_GRID + 1 - e;
+  g.q = FX_GRID + 2 - e;
+  const int po = fx_place(g.ox) < fx_place(g.oy) ? fx_place(g.ox) : fx_place(g.oy);
+  g.exact = (place < po ? place : po) >= -g.q;
   return ok;
 }
 
-// Whether the grid is fine enough for a variogram. Its rounding moves a
+// Whether the grid is fine enough for a variogram. It is where it holds the
+// points exactly (coordinates of some size of their own, as projected ones:
+// their last place is that of 2^-52 of it). Else its rounding moves a
 // distance by 0.41 steps (rms: four coordinates, a third of them each way), so
-// an entry by 0.41 steps times the structures' slopes at their steepest. Half
-// of the 2^-54 of the sills that an FP64 evaluation is off by bounds it; a
-// structure of little sill counts little. Measured against 113-bit arithmetic
-// (Exp, pairs within the range, where few coordinates are exact on the grid;
-// rms in units of 2^-54 of the sill, FP64 1.05): extent / range 42 (the limit
-// lies between 43 and 85 by the extent's binary place) 0.03, 128 0.08, 500
-// 0.55, 2100 3.6, 8500 14.
-FX_HD bool fx_resolves(const spi_vg_t& vg, int q) {
+// an entry by 0.41 steps times the structures' slopes at their steepest, if no
+// coordinate is exact on it (in practice most are). The 2^-54 of the
+// sills that an FP64 evaluation is off by (rms) bounds that; a structure of
+// little sill counts little. Measured against 113-bit arithmetic (Exp, pairs
+// within the range, coordinates near 0; rms in units of 2^-54 of the sill, FP64
+// 1.05): extent / range 128 0.03, 200 (the limit lies between 170 and 340 by
+// the extent's binary place) 0.05, 500 0.20, 2100 1.7, 8500 7.
+FX_HD bool fx_resolves(const spi_vg_t& vg, const FxGrid& g) {
+  if (g.exact) return true;
   double tot = 0.0, slope = 0.0;
   for (int c = 0; c < vg.n_comp; ++c) {
     if (vg.code[c] == SPI_VG_NUG) continue;
@@ -117,7 +139,7 @@ FX_HD bool fx_resolves(const spi_vg_t& vg, int q) {
     tot += vg.sill[c];
     slope += k * vg.sill[c] / vg.range[c];
   }
-  return slope <= tot * ldexp(1.0, q - 54);
+  return slope <= tot * ldexp(1.0, g.q - 53);
 }
 
 // x - o on the grid, the difference's rounding error included.
@@ -142,21 +164,6 @@ FX_HD int64_t fx_coord0(double x, int q) {
   const int sh = (e ? e : 1) - 1075 + q;  // x = m 2^(e - 1075)
   const int64_t v = sh >= 0 ? m << (sh < 63 ? sh : 63) : m >> (-sh < 63 ? -sh : 63);
   return b < 0 ? -v : v;
-}
-
-// The place of x's last bit, x = odd 2^place: a grid of 2^-q holds x exactly
-// where it is -q or more.
-FX_HD int fx_place(double x) {
-#ifdef __CUDA_ARCH__
-  const int64_t b = __double_as_longlong(x);
-#else
-  int64_t b;
-  __builtin_memcpy(&b, &x, 8);
-#endif
-  const int e = (int)((b >> 52) & 0x7ff);
-  const int64_t m = (b & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
-  if (m == 0) return 4096;
-  return (e ? e : 1) - 1075 + 63 - fx_clz((uint64_t)(m & -m));
 }
 
 // A positive double as a 64-bit mantissa and an exponent: v = m 2^e, m with

@@ -469,7 +469,7 @@ __global__ __launch_bounds__(LR_T) void k_leg_rhs_fx(
   const int m = n + (sk ? 0 : 1 + n_drift);
   if (tid == 0) {
     fx_init(f, vg, sk, 0.0, gr.q);
-    if (!scene->ok || !fx_resolves(vg, gr.q)) f.ok = 0;
+    if (!scene->ok || !fx_resolves(vg, gr)) f.ok = 0;
     double t = 0.0;
     for (int c = 0; c < vg.n_comp; ++c)
       if (vg.code[c] == SPI_VG_NUG) t += vg.sill[c];

@@ -33,18 +33,18 @@
 //      digits in shared memory, one thread copies the packed row digits (16
 //      KB by a bulk copy, packed once per system) and issues 12 MMAs: digit
 //      i of the cells against digits 0..7-i of the rows, stacked along N,
-//      lands on levels i..7 at once. A ring of 5 stages; while a chunk's last
-//      MMAs run, the next stages' digits are made.
-//   3. The accumulators are drained (lane = cell) into 128 registers a
-//      thread, which is why the CTA has 256 threads; a block's values are
-//      squared and summed in 128-bit integers (variance) or scaled to FP64
-//      (duals, estimates), and the cells' sum check, variance and fields are
-//      finished from registers.
+//      lands on levels i..7 at once. A ring of SL_ST stages; while a chunk's
+//      last MMAs run, the next stages' digits are made.
+//   3. The accumulators are drained (lane = cell) into 96-bit sums, SL_RT rows
+//      of a cell to a thread (16 working warps, 96 registers a thread); a
+//      block's values are squared and summed in 128-bit integers (variance)
+//      or scaled to FP64 (duals, estimates), and the cells' sum check,
+//      variance and fields are finished from registers.
 //
 // Measured (GB300, the cell pass alone): 750 stations on 62 500 cells, OK
 // with variance 42 -> 2.6 ms, SK 6.8 -> 1.1 ms; EDK, 400 stations, 200 steps
 // on 250 000 cells 44.8 -> 3.9 ms; 150 stations, 24 steps on 40 000 cells 2.5
-// -> 0.34 ms. The tensor pipe is busy a quarter of the time: the digits'
+// -> 0.34 ms. The tensor pipe is busy 31% of the time: the digits'
 // making, the drains (which hold the MMAs up, the accumulators filling tensor
 // memory) and the generation share the rest. Two CTAs per SM with blocks of
 // 32 rows measured 12% slower on the variance (twice the digits to make).
@@ -84,6 +84,7 @@ constexpr int64_t SL_BAND = 64ll << (FX_BITS - 54);  // units around the min_vg_
 struct SlHead {
   unsigned long long mn[2], mx[2];  // ordered encodings of the coordinates' range
   unsigned long long bad;           // a coordinate is not finite
+  long long place;                  // 4096 minus the finest place of the coordinates
 };
 
 // What a launch contracts: the kriging systems of a batch; given right-hand
@@ -110,7 +111,6 @@ struct SlArgs {
   int filter;        // 0: every system, 2: not in an FP32 tier, 3: tier 2 (or all candidates)
   int s0, ns;        // the launch's systems
   int rs;            // row records per system
-  int nvb_max;       // variance blocks of the largest system
   long pc;           // packed chunks per system
   SlHead* head;
   FxGrid* grid;
@@ -139,8 +139,10 @@ __global__ __launch_bounds__(256) void k_sl_range(spi_domain_t dom, const int64_
                                                   const int32_t* stn_idx, int n_sys, SlHead* h) {
   unsigned long long mn[2] = {~0ull, ~0ull}, mx[2] = {0, 0};
   bool bad = false;
+  int place = 4096;
   auto take = [&](double x, double y) {
     bad = bad || !isfinite(x) || !isfinite(y);
+    place = min(place, min(fx_place(x), fx_place(y)));
     const unsigned long long a = enc(x), b = enc(y);
     mn[0] = min(mn[0], a);
     mx[0] = max(mx[0], a);
@@ -155,7 +157,9 @@ __global__ __launch_bounds__(256) void k_sl_range(spi_domain_t dom, const int64_
     const int64_t st = stn_idx ? stn_idx[i] : i;
     take(dom.stn_x[st], dom.stn_y[st]);
   }
+  for (int o = 16; o > 0; o >>= 1) place = min(place, __shfl_xor_sync(0xffffffffu, place, o));
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&h->bad, 1ull);
+  if ((threadIdx.x & 31) == 0) atomicMax(&h->place, 4096ll - place);
   for (int d = 0; d < 2; ++d) {
     for (int o = 16; o > 0; o >>= 1) {
       mn[d] = min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
@@ -175,7 +179,8 @@ __device__ __forceinline__ int dual_rows(const SlArgs& A, int route) {
 
 // The common grid of the range; false where it has none.
 __device__ bool sl_grid(const SlHead* h, FxGrid& g) {
-  return fx_grid(dec(h->mn[0]), dec(h->mx[0]), dec(h->mn[1]), dec(h->mx[1]), g) && !h->bad;
+  const int place = 4096 - (int)h->place;
+  return fx_grid(dec(h->mn[0]), dec(h->mx[0]), dec(h->mn[1]), dec(h->mx[1]), place, g) && !h->bad;
 }
 
 // The grid, and which systems of the launch take this path: on the Cholesky
@@ -202,7 +207,7 @@ __global__ __launch_bounds__(256) void k_sl_select(SlArgs A) {
   if (A.filter == 3) use = use && (A.ws.tier ? A.ws.tier[s] == 2 : fast);
   // (a variogram of nuggets alone has no covariances to contract)
   fx_init(r.vg, A.sys.vg[s], sk, A.dom.min_vg_val, g.q);
-  if (!r.vg.ok || r.vg.n == 0 || !fx_resolves(A.sys.vg[s], g.q)) use = 0;
+  if (!r.vg.ok || r.vg.n == 0 || !fx_resolves(A.sys.vg[s], g)) use = 0;
   r.use = use;
   // |y| <= sqrt(sill) for y = Linv c: y / sill in units of 2^unit, 58 bits
   // with 8 times as much room
@@ -1127,7 +1132,6 @@ int launch_slices(const SlicesCall& c, SlicesDone* done, cudaStream_t st) {
   A.want_vec = c.want_vec;
   A.filter = c.filter;
   A.rs = p.rs;
-  A.nvb_max = p.nvb;
   A.pc = p.pc;
   A.sgs = p.sgs;
   A.slot_bytes = (long)p.slot;

@@ -2,7 +2,7 @@
 fx_grid and fx_resolves compiled for the host, against decimals of 50 digits.
 Where fx_resolves says yes, the entries' rms error over pairs within a range is
 no larger than that of the FP64 formula on the same pairs; a far coordinate or
-a short range makes it say no."""
+a short range makes it say no, unless the grid holds the coordinates exactly."""
 import math
 import random
 import shutil
@@ -22,14 +22,16 @@ int main() {
   uint64_t tab[256];
   for (int j = 0; j < 256; ++j) tab[j] = fx_exp2_entry(j);
   double b[4], x[4];
-  int n;
-  while (scanf("%la %la %la %la %d", &b[0], &b[1], &b[2], &b[3], &n) == 5) {
+  int n, rule;  // rule: the points count as not exact
+  while (scanf("%d %la %la %la %la %d", &rule, &b[0], &b[1], &b[2], &b[3], &n) == 6) {
     spi_vg_t vg = {};
     vg.n_comp = n;
     for (int c = 0; c < n; ++c) scanf("%d %la %la", &vg.code[c], &vg.sill[c], &vg.range[c]);
     for (int i = 0; i < 4; ++i) scanf("%la", &x[i]);
     FxGrid g;
-    const int ok = fx_grid(b[0], b[1], b[2], b[3], g) && fx_resolves(vg, g.q);
+    int place = 4096;
+    for (int i = 0; i < 4; ++i) place = place < fx_place(x[i]) ? place : fx_place(x[i]);
+    const int ok = fx_grid(b[0], b[1], b[2], b[3], rule ? -4096 : place, g) && fx_resolves(vg, g);
     FxVg f;
     fx_init(f, vg, 0, 0.0, g.q);
     const int64_t v = ok ? fx_entry(f, fx_coord(x[0], g.ox, g.q), fx_coord(x[1], g.oy, g.q),
@@ -53,10 +55,10 @@ def fx(tmp_path_factory):
                     "-I", str(ROOT / "spinterps_gb300" / "csrc"), "-I", str(cuda),
                     str(d / "main.cpp"), "-o", str(d / "fx")], check=True)
 
-    def run(cases):
+    def run(cases, rule=1):
         txt = []
         for box, vg, x in cases:
-            head = [float(v).hex() for v in box] + [len(vg)]
+            head = [rule] + [float(v).hex() for v in box] + [len(vg)]
             for name, s, r in vg:
                 head += [CODES[name], float(s).hex(), float(r).hex()]
             txt.append(" ".join(map(str, head + [float(v).hex() for v in x])))
@@ -79,21 +81,24 @@ def _rho(name, t, exp=math.exp):
 
 
 @pytest.mark.parametrize("name", ["Exp", "Gau", "Sph", "Lin"])
-@pytest.mark.parametrize("at", ["corner", "anywhere"])
+@pytest.mark.parametrize("at", ["corner", "anywhere", "exact"])
 def test_no_larger_error_than_fp64(fx, name, at):
     getcontext().prec = 50
     rng = random.Random(name + at)
     cases = []
     for _ in range(3000):
         side = math.exp(rng.uniform(0, 30))
-        r = side / math.exp(rng.uniform(1, 6))
+        r = side / math.exp(rng.uniform(1, 6 if at != "exact" else 16))
         span = 2 * r if at == "corner" else side
         lim = lambda v: min(max(v, 0.0), side)  # noqa: E731
         cx, cy = span * rng.random(), span * rng.random()
         x = (cx, cy, lim(cx + 2 * r * (rng.random() - 0.5)), lim(cy + 2 * r * (rng.random() - 0.5)))
-        cases.append(((0.0, side, 0.0, side * rng.random()), [(name, 0.01 + rng.random(), r)], x))
+        if at == "exact":   # coordinates of 53 bits of the side
+            side, u = 2.0 ** math.frexp(side)[1], 2.0 ** (math.frexp(side)[1] - 53)
+            x = tuple(round(v / u) * u for v in x)
+        cases.append(((0.0, side, 0.0, side), [(name, 0.01 + rng.random(), r)], x))
     e_fx, e_64, n = Decimal(0), Decimal(0), 0
-    for (_, vg, x), (ok, v) in zip(cases, fx(cases)):
+    for (_, vg, x), (ok, v) in zip(cases, fx(cases, int(at != "exact"))):
         if not ok:
             continue
         (_, s, r), n = vg[0], n + 1
@@ -103,7 +108,7 @@ def test_no_larger_error_than_fp64(fx, name, at):
         got = s - s * (1.0 - _rho(name, h / r))
         e_fx += (Decimal(v) / 2 ** 62 - want) ** 2
         e_64 += (Decimal(got) / Decimal(s) - want) ** 2
-    assert n > 1000
+    assert n > 1000 if at != "exact" else n == len(cases)
     assert e_fx <= e_64
 
 
@@ -126,5 +131,8 @@ def test_what_is_refused(fx):
     for far in (1e7, 1e12, 1e20, 9.969209968386869e36, 1e300, inf, nan):
         assert not ok((0, far, 0, 1e5), exp), far
         assert not ok((0, 1e5, -far, 1e5), exp), far
+    # coordinates that the grid holds exactly: any range
+    assert fx([((0, 2.5e5, 0, 1e5), [("Exp", 0.9, 1.0)], x)], rule=0)[0][0]
+    assert not fx([((0, 2.5e5, 0, 1e5), [("Exp", 0.9, 1.0)], (1e-9, *x[1:]))], rule=0)[0][0]
     # all points in one place
     assert ok((5.0, 5.0, 7.0, 7.0), exp)

@@ -122,9 +122,11 @@ def test_a_cell_without_a_place(far, axis):
           {k: v[:, rest] for k, v in want.fields().items()})
 
 
-def test_a_range_short_of_the_domain():
-    """Exp(12) in a domain of 76 km: stations a few metres apart."""
-    job = list(_job(90, 2, 200))
+@pytest.mark.parametrize("off", [0.0, 4e5])
+def test_a_range_short_of_the_domain(off):
+    """Exp(12) in a domain of 76 km: stations a few metres apart; also with
+    offsets, whose coordinates the grid holds exactly."""
+    job = [a if k == 2 else a + off for k, a in enumerate(_job(90, 2, 200))]
     for a, b in ((0, 3), (1, 4)):
         job[b][:80] = job[a][:80] + np.random.default_rng(a).uniform(-9, 9, 80)
     a, b = (_plan(job, ["OK", "SK"], "0.9 Exp(12)", tc) for tc in (True, False))
