@@ -34,8 +34,7 @@ struct Gate {
 };
 
 // Lower Cholesky factor of every system in place (spi_chol.cu); status[s]
-// receives 0 or the 1-based failing pivot. a00 (optional): A's first
-// diagonal entry as L_00^2, kept for the condition estimate.
+// receives 0 or the 1-based failing pivot.
 template <typename T>
 int launch_chol(const spi_systems_t& sys, T* arena, int32_t* status, Gate g, cudaStream_t st);
 

@@ -446,7 +446,8 @@ static int launch_idw_sq(const IdwArgs& A, cudaStream_t st) {
 template <typename T, typename OutT>
 static int dispatch_idw(const IdwArgs& A, cudaStream_t st) {
   if (sizeof(T) == 8 && A.p == 2.0) {
-    // 32 cells while two CTAs of them share an SM, 16 up to its memory
+    // 32 cells while two CTAs of them share an SM (to 395 stations), 16 up to its
+    // memory
     if (A.dom.n_stns <= 400) return launch_idw_sq<32, OutT>(A, st);
     if (A.dom.n_stns <= 1600) return launch_idw_sq<16, OutT>(A, st);
   }

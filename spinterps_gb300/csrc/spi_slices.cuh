@@ -48,8 +48,8 @@ struct SlicesCall {
 
 int64_t slices_scratch(int max_n, int n_sys, int max_vec, bool var, bool vec);
 
-// The other contraction: *use != 0 (on the device) where it ran, else the
-// caller computes it.
+// The other contraction's scratch, and its launch: *use != 0 (on the device)
+// where it ran, else the caller computes it.
 int64_t slices_scratch_one(int n, int rows);
 int launch_slices_rows(const SlRows& r, void* scratch, int64_t scratch_bytes, int32_t* err,
                        const int32_t** use, cudaStream_t st);

@@ -135,7 +135,7 @@ def interp_steps_nebs(stn_x, stn_y, data, cell_x, cell_y, vgs, interp_args, neb_
       of cells with identical neighbour lists: spi_local_groups inverts
       each group's system once per step and applies it to the group's
       cells;
-    - IDW and NNB run per cell (spi_local_cells, one warp per (cell, step)).
+    - IDW and NNB run per cell (spi_local_cells, one thread per (cell, step)).
     FP64 in either precision; the other keywords of steps.interp_steps do
     not apply. Returns (fields, problem steps) like steps.interp_steps."""
     import torch

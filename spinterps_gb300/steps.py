@@ -294,8 +294,8 @@ class _KrigeBatch:
         n_sys = len(ch)
         self.L = torch.empty(self.arena, dtype=torch.float64, device=dev)
         # Linv only where the OK variance (or leave-one-out) reads it; other
-        # systems get their duals and condition estimate from L by
-        # triangular solves (spi_krige_factor / spi_krige_duals)
+        # systems keep their inverse factor over L, and their duals come
+        # from it (spi_krige_factor / spi_krige_duals)
         if need_linv is None:
             need_linv = bool(want_var and kind == "OK")
         self.X = torch.empty(self.arena, dtype=torch.float64, device=dev) if need_linv else None
@@ -968,7 +968,7 @@ class InterpPlan:
         as _KrigeBatch.run makes them: row fills; per batch the build,
         Cholesky, inverse (or condition estimate), Gauss-Jordan and the pinv
         check of the exact-inverse systems, the duals
-        (plus two triangular-solve kernels without the inverse), the FP32
+        (two more launches without an arena for the inverse), the FP32
         splits, the probe (tensor-core and double-float variances, both
         tiers' cell kernels, the tier pick), the main variance kernels and
         one cell kernel per tier; per IDW / NNB field its fill, split (mixed
