@@ -179,7 +179,10 @@ __global__ __launch_bounds__(DT) void k_duals(spi_domain_t dom, spi_systems_t sy
   // every early return below is the same for the whole cluster
   if (route == 2) return;
   const bool linv = ws.linv_arena != nullptr;
-  if (phase == kAll ? (route == 0 && !linv) : route != 0) return;
+  // (in the fallback pass kSolve also takes what has left the Cholesky path)
+  if (phase == kAll ? (route == 0 && !linv)
+                    : route != 0 && !(fallback && phase == kSolve && route == 1))
+    return;
   if (fallback && ws.ir[s] != 2) return;
   const SysView v = sys_view(sys, s);
   const int n = v.n, tid = threadIdx.x;
@@ -192,7 +195,8 @@ __global__ __launch_bounds__(DT) void k_duals(spi_domain_t dom, spi_systems_t sy
   const int beside = with_f ? max(1, nk - a) : nk;
   // (kSolve: one cluster per system takes the first steps; kSteps: the rest)
   const int first = phase == kSteps ? max(1, nk - a) : 0;
-  const int todo = phase == kSolve ? min(nsteps, beside) : max(0, nsteps - first);
+  const int todo =
+      phase == kSolve && route == 0 ? min(nsteps, beside) : max(0, nsteps - first);
   const int per = max(beside, (todo + ngrp - 1) / ngrp);
   const int q0 = min(todo, gi * per) + first, q1 = min(todo, (gi + 1) * per) + first;
   if (gi > 0 ? q0 >= q1 : (!with_f && q0 >= q1)) return;
@@ -518,7 +522,11 @@ __global__ __launch_bounds__(DT) void k_duals(spi_domain_t dom, spi_systems_t sy
 }
 
 // Systems whose refinement did not converge fall back to the FP64 factor
-// (ir = 2): they are then factored and solved again.
+// (ir = 2): they are then factored, given their route and solved again. (An
+// FP32 factor of a singular matrix, of two gauges in one place for instance,
+// has a small pivot of rounding where the FP64 one fails or is far too ill
+// conditioned for the Cholesky path.)
+constexpr double kFallbackCondMax = 1e13;  // the callers' usual cond_max
 __global__ void k_ir_fail_gate(spi_systems_t sys, spi_krige_ws_t ws) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= sys.n_sys) return;
@@ -571,6 +579,7 @@ int launch_duals(const spi_domain_t& dom, const spi_systems_t& sys, const spi_kr
         if (rc) return rc;
         if ((rc = launch_trinv<double>(sys, ws.l_arena, ws.l_arena, ws.status, ws.cond, 1, g, st)))
           return rc;
+        if ((rc = launch_routes(dom, sys, ws, kFallbackCondMax, g, st))) return rc;
       }
       if (e == cudaSuccess) e = launch(kSolve, pass, 1);
       if (e == cudaSuccess) e = launch(kSteps, pass, gx);

@@ -129,9 +129,10 @@ __global__ __launch_bounds__(FT) void k_gj(spi_domain_t dom, spi_systems_t sys,
                                           const int32_t* __restrict__ status,
                                           double* __restrict__ cond,
                                           int32_t* __restrict__ route, double cond_max,
-                                          int pinv_on) {
+                                          int pinv_on, Gate g) {
   const int s = blockIdx.x;
   const int tid = threadIdx.x;
+  if (g.skips(s)) return;
   if (status[s] == 0 && cond[s] <= cond_max) {
     if (tid == 0) route[s] = 0;
     return;
@@ -286,6 +287,22 @@ __global__ __launch_bounds__(FT) void k_loo(spi_domain_t dom, spi_systems_t sys,
   }
 }
 
+static size_t gj_smem(int max_n) {
+  return (size_t)(max_n + GA) * (2 * sizeof(double) + sizeof(int));
+}
+
+int launch_routes(const spi_domain_t& dom, const spi_systems_t& sys, const spi_krige_ws_t& ws,
+                  double cond_max, Gate g, cudaStream_t st) {
+  const size_t gsm = gj_smem(sys.max_n);
+  if (gsm > 200 * 1024) return SPI_ERR_TOO_LARGE;
+  if (!smem_opt_in(k_gj, gsm)) return SPI_ERR_CUDA;
+  const int pinv_on = ws.pinv_scratch != nullptr;
+  k_gj<<<sys.n_sys, FT, gsm, st>>>(dom, sys, ws.l_arena, ws.status, ws.cond, ws.route, cond_max,
+                                   pinv_on, g);
+  SPI_LAUNCH_CHECK();
+  return pinv_on ? launch_pinv(dom, sys, ws, st) : SPI_OK;
+}
+
 }  // namespace spi
 
 using namespace spi;
@@ -350,19 +367,9 @@ extern "C" int spi_krige_factor(const spi_domain_t* dom, const spi_systems_t* sy
   if ((rc = launch_trinv<double>(sy, ws->l_arena, x, ws->status, ws->cond,
                                  ws->linv_arena ? 0 : 1, g, st)))
     return rc;
-  size_t gsm = (size_t)(sys->max_n + GA) * (2 * sizeof(double) + sizeof(int));
-  if (gsm > 200 * 1024) return SPI_ERR_TOO_LARGE;
-  if (!smem_opt_in(k_gj, gsm)) return SPI_ERR_CUDA;
+  if (gj_smem(sys->max_n) > 200 * 1024) return SPI_ERR_TOO_LARGE;
   if (sys->kind == SPI_KIND_EDK) {
     k_drift_check<<<sys->n_sys, FT, 0, st>>>(d, sy, ws->status);
-    SPI_LAUNCH_CHECK();
-  }
-  const int pinv_on = ws->pinv_scratch != nullptr;
-  if (ws->gj_scratch) {
-    if ((rc = launch_gj_multi(d, sy, *ws, cond_max, pinv_on, st))) return rc;
-  } else {
-    k_gj<<<sys->n_sys, FT, gsm, st>>>(d, sy, ws->l_arena, ws->status, ws->cond, ws->route,
-                                      cond_max, pinv_on);
     SPI_LAUNCH_CHECK();
   }
   if (ws->pinv_used) {
@@ -370,6 +377,9 @@ extern "C" int spi_krige_factor(const spi_domain_t* dom, const spi_systems_t* sy
         cudaSuccess)
       return SPI_ERR_CUDA;
   }
+  if (!ws->gj_scratch) return launch_routes(d, sy, *ws, cond_max, every, st);
+  const int pinv_on = ws->pinv_scratch != nullptr;
+  if ((rc = launch_gj_multi(d, sy, *ws, cond_max, pinv_on, st))) return rc;
   if (pinv_on) return launch_pinv(d, sy, *ws, st);
   return SPI_OK;
 }

@@ -46,6 +46,12 @@ template <typename T>
 int launch_trinv(const spi_systems_t& sys, const T* l, T* x, const int32_t* status, double* cond,
                  int probes, Gate g, cudaStream_t st);
 
+// The route of every gated system from its factor's status and condition, the
+// exact inverse (k_gj, one CTA each, and the pinv check) where that is off the
+// Cholesky path (spi_factor.cu).
+int launch_routes(const spi_domain_t& dom, const spi_systems_t& sys, const spi_krige_ws_t& ws,
+                  double cond_max, Gate g, cudaStream_t st);
+
 // G, S^-1, 1'G and the steps' dual weights of every system (spi_duals.cu).
 int launch_duals(const spi_domain_t& dom, const spi_systems_t& sys, const spi_krige_ws_t& ws,
                  const double* vals, cudaStream_t st);

@@ -570,7 +570,9 @@ class _KrigeBatch:
             return 0
         panels = (n + 31) // 32 - 1
         levels = panels.bit_length()
-        return (2 * panels + 2 * levels + 1) * (3 if self.l32 is not None else 1)
+        n = (2 * panels + 2 * levels + 1) * (3 if self.l32 is not None else 1)
+        # the refinement's fallback pass: the routes (and their pinv check)
+        return n + (1 + (self.pinv is not None) if self.l32 is not None else 0)
 
     def slices_launches(self, fields):
         """Kernels of a sliced contraction beside the FP64 kernel's own: the
