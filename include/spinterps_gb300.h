@@ -268,8 +268,9 @@ typedef struct {
                             factored in FP64 as without it */
     int32_t *ir;         /* [n_sys] with l32: 1 where the FP32 factor is
                             kept, 2 where its refinement did not converge
-                            and the system was factored and solved again in
-                            FP64, 0 where it was factored in FP64 from the
+                            and the system was factored again in FP64, given
+                            its route (the exact inverse beyond a condition
+                            estimate of 1e13) and solved again, 0 where it was factored in FP64 from the
                             start */
     int32_t *ir_iters;   /* [n_sys] with l32: refinement corrections the
                             duals took (the largest over their right-hand
